@@ -1,26 +1,30 @@
 // Parallel-beam backprojection with TMA-staged projection rows (sm_100a).
 //
-// Arithmetic of MultiProjectionBPparallel::BackProject (MultiProjBPparallel.cpp:39-170),
-// every float operation in the reference's order with explicitly rounded intrinsics, so the
-// volume is bit-identical to the plain kernel and to the reference (no-tilt branch):
+// Arithmetic of MultiProjectionBPparallel::BackProject (MultiProjBPparallel.cpp:39-170), with and
+// without tilt correction, and of the factory's serial and nearest-neighbour backprojectors, every
+// float operation in the reference's order and rounded on its own, so the volume is bit-identical
+// to the plain kernel and to the reference; without tilt
 //   u = (startu_i + cos_i y) - sin_i x,  n = (int)u in [0, nu-2],  f = |u - n|,
 //   vol[y-1][x-1][z] += (P[z][n] (1 - f) + P[z][n+1] f)          (P pre-multiplied by weight_i)
 //
-// Tiling: a CTA owns 32 (x) x 8 (y) voxel columns x 32 slices; a thread keeps its 32 slices
-// in registers over all projections. In this geometry the detector column of a voxel does
-// not depend on its slice, so one projection's footprint on the tile is at most ~34 columns
-// by the tile's 32 detector rows: a producer warp projects the 4 tile corners with the voxel
-// formula (affine in x and y, so the corners bound every voxel exactly; the per-projection
-// sin/cos/startu are copied into shared memory with cp.async three batches ahead and the
-// corners use those copies, as the voxels do), and one TMA tile
-// load (cp.async.bulk.tensor.3d, no multicast) brings a 48 x 32 box per projection into
-// shared memory, batches of 8 projections on two stages with bounded mbarrier waits. The
-// box pitch is a compile-time constant, so the slice loop addresses its two samples with
-// immediate offsets; the two interpolation products are one f32x2 mul (an f32x2 mul feeding
-// scalar adds is not contracted). Rows beyond the detector are zero-filled by the TMA unit
-// and never read (only z < 4*(nv/4) is updated). A footprint that does not fit the box falls
-// back to guarded global loads for that tile and projection (same arithmetic). The volume
-// (z fastest) is read and written as float4 runs.
+// Tiling: a CTA owns 32 (x) x 2 NW (y) voxel columns x TZ slices; a thread keeps the TZ slices of
+// two neighbouring rows' columns in registers over all projections. In this geometry the detector
+// column of a voxel does not depend on its slice, so one projection's footprint on the tile is at
+// most ~37 columns by the tile's TZ detector rows: a producer warp projects the 4 tile corners with
+// the voxel formula (affine in x and y, and float rounding is monotone, so the corners bound every
+// voxel exactly; the per-projection sin/cos/startu are copied into shared memory with cp.async three
+// batches ahead and the corners use those copies, as the voxels do), and one TMA tile load
+// (cp.async.bulk.tensor.3d, no multicast) brings a 48 x TZ box per projection into shared memory,
+// batches of NB projections on two stages with bounded mbarrier waits. Rows beyond the detector are
+// zero-filled by the TMA unit (slices from 4*(nv/4) on are computed and never stored). A footprint
+// that does not fit the box falls back to guarded global loads for that tile and projection (same
+// arithmetic). The volume (z fastest) is read and written as float4 runs.
+//
+// Bound: shared-memory load wavefronts (78 % of the LSU's peak) and instruction issue (64 %). One
+// row per thread needs two samples per update, 2.2 wavefronts and 6.9 warp instructions with the
+// set-up; two rows share three samples, and slices go in pairs through the paired FP32 pipe: 1.7
+// wavefronts and 5.6 instructions. 2048^2 x 64 slices from 1125 projections: 60.8 -> 47.4 ms;
+// 1001^2 x 60 with tilt from 625 projections: 30.1 (direct-load kernel) -> 7.8 ms.
 #include "mr_common.cuh"
 #include "mr_tma.cuh"
 
@@ -45,14 +49,27 @@ int bp_device_status_take()
 
 namespace bp2 {
 
-constexpr int TX = 32, TY = 8, TZ = 32, THREADS = TX * TY, NB = 8, G = 4, BW = 48;
-constexpr int CTAS_PER_SM = 2;
-constexpr int BOXBYTES = BW * TZ * 4;
-constexpr int GEO = 8; // sin, cos, startu, weight, slab (as int bits), pad
+constexpr int TX = 32, G = 4, BW = 48;
+constexpr float kMagic = 12582912.0f; // 1.5 * 2^23
+constexpr int kMagicBits = 0x4B400000;
+constexpr int GEO = 4; // sin, cos, startu, slab (as int bits)
+
+// What a voxel adds per projection (MultiProjBPparallel.cpp:39-170 and the factory's other two):
+//   kLinear      acc += pa (1 - f) + pb f, f = |u - n|
+//   kNearest     acc += pa (NNMultiProjBP.cpp:84-90)
+//   kTilt        u shifted by the centre offset before the x term; f of slice group g is
+//                |(u - n) - g inc - g inc|, the first shift a running subtraction (:86-105)
+//   kTiltSerial  u shifted after the x term, f = |(u - n) - g inc| (MultiProjBP.cpp:61-84)
+//   kTiltNearest u shifted after the x term, the sample at n (NNMultiProjBP.cpp:61-90)
+enum Mode { kLinear, kNearest, kTilt, kTiltSerial, kTiltNearest };
+
+// How a tile reads one projection: its footprint does not fit the box (guarded global loads), no
+// voxel of the tile lies on the detector, staged, staged with every voxel of the tile on the detector
+// and cos away from +-1 (n of neighbouring rows is then the same or one apart).
+enum Footprint { kUnfit, kNothing, kStaged, kClean };
 
 struct Params {
     const float *proj;
-    const float *weight;
     const int32_t *index;
     const float *sinv, *cosv, *startu;
     const uint32_t *mask;
@@ -60,9 +77,14 @@ struct Params {
     int nproj, nu, nv, nz4;
     int wait_limit; // tries of each per-batch wait
     int ybegin, yend; // volume rows y1 - 1 in [ybegin, yend)
+    int pitch;        // floats between detector rows
+    float toff, tinc; // tilt: centre offset and its step per group of 4 slices
+    float neg_zero;   // -0 (see blend_add)
 };
 
+template <int TZ, int NB>
 struct Smem {
+    static constexpr int BOXBYTES = BW * TZ * 4;
     float *box;      // [2][NB][TZ][BW]
     float *geo;      // [3][NB][GEO]
     int4 *meta;      // [2][NB]: x0, mode
@@ -82,75 +104,121 @@ struct Smem {
 };
 
 // Detector position of voxel (x1, y1) (1-based) for list entry i, reference order.
-__device__ __forceinline__ float posu(float sn, float cs, float su, float fx, float fy)
+template <int MODE>
+__device__ __forceinline__ float posu(float sn, float cs, float su, float fx, float fy, float toff)
 {
-    return __fsub_rn(__fadd_rn(su, __fmul_rn(cs, fy)), __fmul_rn(sn, fx));
+    float local = __fadd_rn(su, __fmul_rn(cs, fy));
+    if constexpr (MODE == kTilt) local = __fsub_rn(local, toff);
+    const float u = __fsub_rn(local, __fmul_rn(sn, fx));
+    if constexpr (MODE == kTiltSerial || MODE == kTiltNearest) return __fsub_rn(u, toff);
+    return u;
 }
 
-// Slices of one voxel column for one staged projection: p points at the sample pair of slice 0
-// (row pitch BW). FULL: all TZ slices exist.
-template <bool HASW, bool FULL>
-__device__ __forceinline__ void staged_column(float (&acc)[TZ], const float *p, float wa, float wb, float w, int zmax)
+// Two slices of acc += pa * wa + pb * wb in the reference's order, every product and sum rounded on
+// its own. ptxas contracts a paired multiply that feeds a paired add even when both carry .rn, so the
+// products are paired fmas with an addend of -0 that it cannot see (`nz`, a kernel argument): p + -0 is
+// p bit for bit, signed zeros included, and the sum that follows stays an add.
+__device__ __forceinline__ void blend_add(float2 &acc, float2 pa, float2 pb, float2 wa, float2 wb, float2 nz)
 {
-    const float2 wab = make_float2(wa, wb);
+    acc = __fadd2_rn(acc, __fadd2_rn(__ffma2_rn(pa, wa, nz), __ffma2_rn(pb, wb, nz)));
+}
+
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// Interpolation weight of slice group g (float) of a voxel whose u - n is d; kTilt also steps d.
+template <int MODE>
+__device__ __forceinline__ float group_weight(float &d, float g, float tinc)
+{
+    if constexpr (MODE != kTilt && MODE != kTiltSerial) return fabsf(d);
+    const float f = fabsf(__fsub_rn(d, __fmul_rn(g, tinc)));
+    if constexpr (MODE == kTilt) d = __fsub_rn(d, tinc);
+    return f;
+}
+
+// One voxel column's slices for one staged projection: p points at the sample pair of slice 0 (row
+// pitch BW), d is u - n.
+template <int MODE, int TZ>
+__device__ __forceinline__ void staged_column(float2 (&acc)[TZ / 2], const float *p, float d, float g0, float tinc, float2 nz)
+{
 #pragma unroll
-    for (int q = 0; q < TZ; ++q) {
-        if (!FULL && q >= zmax) break;
-        float pa = p[q * BW], pb = p[q * BW + 1];
-        if (HASW) {
-            pa = __fmul_rn(pa, w);
-            pb = __fmul_rn(pb, w);
+    for (int q4 = 0; q4 < TZ; q4 += 4) {
+        const float wb = group_weight<MODE>(d, g0 + static_cast<float>(q4 / 4), tinc), wa = __fsub_rn(1.0f, wb);
+#pragma unroll
+        for (int q = q4; q < q4 + 4; q += 2) {
+            const float2 pa = make_float2(p[q * BW], p[(q + 1) * BW]);
+            if constexpr (MODE == kNearest || MODE == kTiltNearest) acc[q / 2] = __fadd2_rn(acc[q / 2], pa);
+            else blend_add(acc[q / 2], pa, make_float2(p[q * BW + 1], p[(q + 1) * BW + 1]), both(wa), both(wb), nz);
         }
-        const float2 prod = __fmul2_rn(make_float2(pa, pb), wab);
-        acc[q] = __fadd_rn(acc[q], __fadd_rn(prod.x, prod.y));
     }
 }
 
-// NearestNeighborBP's column (NNMultiProjBP.cpp:84-90): the sample at the truncated position.
-template <bool HASW, bool FULL>
-__device__ __forceinline__ void staged_column_nn(float (&acc)[TZ], const float *p, float w, int zmax)
+// The slices of two voxels of neighbouring rows for one staged projection. u changes by cos between
+// them, so the second voxel's pair of samples is the first one's (step false) or the next (step
+// true): three samples serve both, where each alone loads two. lo is the voxel with the smaller n.
+template <int MODE, int TZ>
+__device__ __forceinline__ void staged_pair(float2 (&lo)[TZ / 2], float2 (&hi)[TZ / 2], const float *p, bool step, float dlo,
+                                            float dhi, float g0, float tinc, float2 nz)
 {
 #pragma unroll
-    for (int q = 0; q < TZ; ++q) {
-        if (!FULL && q >= zmax) break;
-        float pa = p[q * BW];
-        if (HASW) pa = __fmul_rn(pa, w);
-        acc[q] = __fadd_rn(acc[q], pa);
+    for (int q4 = 0; q4 < TZ; q4 += 4) {
+        const float g = g0 + static_cast<float>(q4 / 4);
+        const float wbl = group_weight<MODE>(dlo, g, tinc), wal = __fsub_rn(1.0f, wbl);
+        const float wbh = group_weight<MODE>(dhi, g, tinc), wah = __fsub_rn(1.0f, wbh);
+#pragma unroll
+        for (int q = q4; q < q4 + 4; q += 2) {
+            const float2 s0 = make_float2(p[q * BW], p[(q + 1) * BW]);
+            const float2 s1 = make_float2(p[q * BW + 1], p[(q + 1) * BW + 1]);
+            const float2 s2 = make_float2(p[q * BW + 2], p[(q + 1) * BW + 2]);
+            blend_add(lo[q / 2], s0, s1, both(wal), both(wbl), nz);
+            blend_add(hi[q / 2], make_float2(step ? s1.x : s0.x, step ? s1.y : s0.y),
+                      make_float2(step ? s2.x : s1.x, step ? s2.y : s1.y), both(wah), both(wbh), nz);
+        }
     }
 }
 
-// NN selects NearestNeighborBP (NNMultiProjBP.cpp:36-121, no tilt): same positions, the one
-// sample at n instead of the interpolation.
-template <bool HASW, bool NN>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_bp_par_staged(const __grid_constant__ CUtensorMap tmap, const Params P)
+// A CTA of NW warps owns 32 (x) x 2 NW (y) voxel columns x TZ slices; a thread keeps the TZ slices
+// of two neighbouring rows' columns in registers over all projections.
+template <int MODE, int TZ, int NW, int NB, int CTAS>
+__global__ void __launch_bounds__(32 * NW, CTAS) k_bp_par_staged(const __grid_constant__ CUtensorMap tmap, const Params P)
 {
+    constexpr int THREADS = 32 * NW, TY = 2 * NW;
+    constexpr bool kOneSample = MODE == kNearest || MODE == kTiltNearest;
+    constexpr int BOXBYTES = Smem<TZ, NB>::BOXBYTES;
     extern __shared__ __align__(1024) unsigned char smem[];
-    Smem S(smem);
+    Smem<TZ, NB> S(smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int i0 = blockIdx.x * TX, j0 = P.ybegin + blockIdx.y * TY, z0 = blockIdx.z * TZ;
-    const int x1 = i0 + lane + 1, y1 = j0 + warp + 1;
+    const int x1 = i0 + lane + 1, y1 = j0 + 2 * warp + 1; // rows y1 and y1 + 1
     const int zmax = min(TZ, P.nz4 - z0);
-    const bool valid = x1 <= P.nu && y1 <= P.yend;
-    const bool inside = valid && static_cast<uint32_t>(x1) > P.mask[2 * (y1 - 1)] &&
-                        static_cast<uint32_t>(x1) <= P.mask[2 * (y1 - 1) + 1];
-    float *col = P.vol + (static_cast<size_t>(valid ? y1 - 1 : 0) * P.nu + (valid ? x1 - 1 : 0)) * P.nv + z0;
+    bool inside[2];
+    float *col[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const bool valid = x1 <= P.nu && y1 + r <= P.yend;
+        inside[r] = valid && static_cast<uint32_t>(x1) > P.mask[2 * (y1 + r - 1)] &&
+                    static_cast<uint32_t>(x1) <= P.mask[2 * (y1 + r - 1) + 1];
+        col[r] = P.vol + (static_cast<size_t>(valid ? y1 + r - 1 : 0) * P.nu + (valid ? x1 - 1 : 0)) * P.nv + z0;
+    }
     const bool vec = (P.nv & 3) == 0 && zmax == TZ;
 
-    float acc[TZ];
+    float2 acc0[TZ / 2], acc1[TZ / 2];
+    auto load = [&](float2 (&acc)[TZ / 2], const float *c, bool in) {
 #pragma unroll
-    for (int q = 0; q < TZ; q += 4) {
-        if (inside && vec) {
-            const float4 v = *reinterpret_cast<const float4 *>(col + q);
-            acc[q] = v.x;
-            acc[q + 1] = v.y;
-            acc[q + 2] = v.z;
-            acc[q + 3] = v.w;
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[q + e] = (inside && q + e < zmax) ? col[q + e] : 0.0f;
+        for (int q = 0; q < TZ; q += 4) {
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (in && vec) {
+                v = *reinterpret_cast<const float4 *>(c + q);
+            } else if (in && q < zmax) {
+                v = make_float4(c[q], c[q + 1], c[q + 2], c[q + 3]);
+            }
+            acc[q / 2] = make_float2(v.x, v.y);
+            acc[q / 2 + 1] = make_float2(v.z, v.w);
         }
-    }
-    if (!__syncthreads_or(inside)) return;
+    };
+    load(acc0, col[0], inside[0]);
+    load(acc1, col[1], inside[1]);
+    const bool any_inside = inside[0] || inside[1];
+    if (!__syncthreads_or(any_inside)) return;
 
     if (threadIdx.x == 0) {
         tma::mbar_init(&S.bars[0], 1);
@@ -163,13 +231,12 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_bp_par_staged(const __
     const int nbatch = (P.nproj + NB - 1) / NB;
 
     // Geometry of batch s into geometry buffer gb (cp.async by all threads, three batches
-    // ahead; the weight only with HASW, the slab only with an index list).
+    // ahead; the slab only with an index list).
     auto stage_geometry = [&](int s, int gb) {
         for (int idx = threadIdx.x; idx < NB * GEO; idx += THREADS) {
             const int b = idx / GEO, e = idx % GEO, i = s * NB + b;
-            const float *src = e == 0 ? P.sinv : e == 1 ? P.cosv : e == 2 ? P.startu : e == 3 ? P.weight
-                                                                                              : reinterpret_cast<const float *>(P.index);
-            const bool ok = i < P.nproj && (e < 3 || (e == 3 && HASW) || (e == 4 && P.index));
+            const float *src = e == 0 ? P.sinv : e == 1 ? P.cosv : e == 2 ? P.startu : reinterpret_cast<const float *>(P.index);
+            const bool ok = i < P.nproj && (e < 3 || P.index);
             tma::copy4_zfill(S.geo + gb * NB * GEO + idx, ok ? src + i : P.sinv, ok);
         }
     };
@@ -177,42 +244,51 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_bp_par_staged(const __
     // staged geometry (4 corner lanes per projection) and issues the TMA copies.
     auto issue_batch = [&](int s, int st, int gb) {
         if (warp != 0) return;
-        const int b = lane >> 2, corner = lane & 3;
-        const int i = s * NB + b;
-        const float *g = S.geo + (gb * NB + b) * GEO;
-        int nmin = 0, nmax = 0;
-        bool ok = i < P.nproj;
-        if (ok) {
-            const float u = posu(g[0], g[1], g[2], static_cast<float>((corner & 1) ? xb : xa),
-                                 static_cast<float>((corner & 2) ? yb : ya));
-            ok = fabsf(u) < 1.0e9f;
-            nmin = nmax = ok ? __float2int_rz(u) : 0;
-        }
-#pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-            nmin = min(nmin, __shfl_xor_sync(0xffffffffu, nmin, o));
-            nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
-            ok = __shfl_xor_sync(0xffffffffu, static_cast<int>(ok), o) && ok;
-        }
-        // 0: global fallback, 1: staged, 2: no voxel of the tile has n in [0, nu-2]
-        int mode = 0, x0 = 0;
-        if (i < P.nproj && ok) {
-            if (nmax < 0 || nmin > P.nu - 2) {
-                mode = 2;
-            } else {
-                x0 = nmin >= 0 ? (nmin & ~3) : -(((-nmin) + 3) & ~3);
-                if (nmax + 1 < x0 + BW) mode = 1;
+#pragma unroll 1
+        for (int r = 0; r < NB; r += 8) {
+            const int b = r + (lane >> 2), corner = lane & 3;
+            const int i = s * NB + b;
+            const float *g = S.geo + (gb * NB + (b < NB ? b : 0)) * GEO;
+            int nmin = 0, nmax = 0;
+            bool ok = b < NB && i < P.nproj, positive = true;
+            if (ok) {
+                const float u = posu<MODE>(g[0], g[1], g[2], static_cast<float>((corner & 1) ? xb : xa),
+                                           static_cast<float>((corner & 2) ? yb : ya), P.toff);
+                ok = fabsf(u) < 1.0e9f;
+                nmin = nmax = ok ? __float2int_rz(u) : 0;
+                positive = u >= 0.0f;
             }
-        }
-        const unsigned staged = __ballot_sync(0xffffffffu, corner == 0 && mode == 1);
-        if (lane == 0) tma::mbar_expect_tx(&S.bars[st], static_cast<uint32_t>(__popc(staged)) * BOXBYTES);
-        __syncwarp();
-        if (corner == 0 && i < P.nproj) {
-            S.meta[st * NB + b] = make_int4(x0, mode, 0, 0);
-            if (mode == 1) {
-                const int slab = P.index ? __float_as_int(g[4]) : i;
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tma::load_3d(S.box + (st * NB + b) * (BW * TZ), &tmap, x0, z0, slab, &S.bars[st]);
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                nmin = min(nmin, __shfl_xor_sync(0xffffffffu, nmin, o));
+                nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
+                ok = __shfl_xor_sync(0xffffffffu, static_cast<int>(ok), o) && ok;
+                positive = __shfl_xor_sync(0xffffffffu, static_cast<int>(positive), o) && positive;
+            }
+            int mode = kUnfit, x0 = 0;
+            if (ok) {
+                if (nmax < 0 || nmin > P.nu - 2) {
+                    mode = kNothing;
+                } else {
+                    x0 = nmin >= 0 ? (nmin & ~3) : -(((-nmin) + 3) & ~3);
+                    if (nmax + 1 < x0 + BW) mode = positive && nmax <= P.nu - 2 && fabsf(g[1]) < 0.999f ? kClean : kStaged;
+                }
+            }
+            const unsigned staged = __ballot_sync(0xffffffffu, corner == 0 && mode >= kStaged);
+            if (lane == 0) {
+                // the phase completes on the last round's arrival; earlier rounds only add their bytes
+                const uint32_t bytes = static_cast<uint32_t>(__popc(staged)) * BOXBYTES;
+                if (r + 8 < NB) tma::mbar_add_tx(&S.bars[st], bytes);
+                else tma::mbar_expect_tx(&S.bars[st], bytes);
+            }
+            __syncwarp();
+            if (corner == 0 && b < NB && i < P.nproj) {
+                S.meta[st * NB + b] = make_int4(x0, mode, 0, 0);
+                if (mode >= kStaged) {
+                    const int slab = P.index ? __float_as_int(g[3]) : i;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    tma::load_3d(S.box + (st * NB + b) * (BW * TZ), &tmap, x0, z0, slab, &S.bars[st]);
+                }
             }
         }
     };
@@ -225,8 +301,14 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_bp_par_staged(const __
 
     uint32_t phase0 = 0, phase1 = 0;
     bool failed = false;
-    const float fx = static_cast<float>(x1), fy = static_cast<float>(y1);
+    // a thread past the volume follows the last column or row (its sums are never stored), so every
+    // position of the tile lies between the corners'
+    const float fx = static_cast<float>(min(x1, P.nu)), fy0 = static_cast<float>(min(y1, P.yend)),
+                fy1 = static_cast<float>(min(y1 + 1, P.yend));
     const int um2 = P.nu - 2;
+    const int group0 = z0 / 4;
+    const float g0 = static_cast<float>(group0);
+    const float2 nz = both(P.neg_zero);
     int s = 0;
     for (int gb = 0; s < nbatch; ++s, gb = gb == 2 ? 0 : gb + 1) {
         const int st = s & 1; // stage buffer; geometry buffer gb = s % 3
@@ -239,89 +321,99 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_bp_par_staged(const __
             failed = true;
             if (lane == 0) atomicExch(&g_bp_error, 1);
         }
-        if (got && inside) {
-            // per-projection set-up of this voxel column: 0 nothing to add, 1 staged, 2 guarded
-            // global loads; n the detector column, off the sample offset in the stage
-            auto setup = [&](int b, int &n, uint32_t &off, float &wa, float &wb) -> int {
-                const int i = s * NB + b;
-                n = 0;
-                off = 0;
-                wa = wb = 0.0f;
-                if (i >= P.nproj) return 0;
-                const int4 m = S.meta[st * NB + b];
-                const float *g = S.geo + (gb * NB + b) * GEO;
-                const float u = posu(g[0], g[1], g[2], fx, fy);
-                n = __float2int_rz(u);
-                if (m.y == 2 || n < 0 || n > um2) return 0;
-                off = static_cast<uint32_t>((st * NB + b) * (BW * TZ) + (n - m.x));
-                wb = fabsf(__fsub_rn(u, static_cast<float>(n)));
-                wa = __fsub_rn(1.0f, wb);
-                return m.y == 1 ? 1 : 2;
+        if (got && any_inside) {
+            // kTilt: the running shift of the slice groups below this tile
+            auto skip_groups = [&](float &d) {
+                if constexpr (MODE == kTilt)
+                    for (int g = 0; g < group0; ++g) d = __fsub_rn(d, P.tinc);
+            };
+            // One row's column from any footprint (fallback and edges: positions formed here).
+            auto row = [&](float2 (&acc)[TZ / 2], int b, float4 g, int4 m, float fy) {
+                const float u = posu<MODE>(g.x, g.y, g.z, fx, fy, P.toff);
+                const int n = __float2int_rz(u);
+                if (n < 0 || n > um2) return;
+                float d = __fsub_rn(u, static_cast<float>(n));
+                skip_groups(d);
+                if (m.y != kUnfit) {
+                    // the box holds all TZ rows (zeros beyond the detector); slices from zmax on are not stored
+                    const uint32_t off = static_cast<uint32_t>((st * NB + b) * (BW * TZ) + (n - m.x));
+                    if (MR_IN_BOUNDS(off + (TZ - 1) * BW + 1, 2 * NB * BW * TZ, kSiteBpStaged))
+                        staged_column<MODE, TZ>(acc, S.box + off, d, g0, P.tinc, nz);
+                    return;
+                }
+                const int slab = P.index ? __float_as_int(g.w) : s * NB + b;
+                const float *img = P.proj + (static_cast<size_t>(slab) * P.nv + z0) * P.pitch + n;
+#pragma unroll
+                for (int q4 = 0; q4 < TZ; q4 += 4) {
+                    if (q4 >= zmax) break;
+                    const float wb = group_weight<MODE>(d, g0 + static_cast<float>(q4 / 4), P.tinc);
+                    const float wa = __fsub_rn(1.0f, wb);
+#pragma unroll
+                    for (int q = q4; q < q4 + 4; q += 2) {
+                        const float *r0 = img + static_cast<size_t>(q) * P.pitch, *r1 = r0 + P.pitch;
+                        const float2 pa = make_float2(__ldg(r0), __ldg(r1));
+                        if constexpr (kOneSample) acc[q / 2] = __fadd2_rn(acc[q / 2], pa);
+                        else blend_add(acc[q / 2], pa, make_float2(__ldg(r0 + 1), __ldg(r1 + 1)), both(wa), both(wb), nz);
+                    }
+                }
             };
 #pragma unroll 1
-            for (int b0 = 0; b0 < NB; b0 += G) {
-                // the set-up of a group is formed first so its latency overlaps, then the
-                // group's slice loops run in projection order (the reference's summation order)
-                int q_mode[G], q_n[G];
-                uint32_t q_off[G];
-                float q_wa[G], q_wb[G];
+            for (int b0 = 0; b0 < NB && s * NB + b0 < P.nproj; b0 += G) {
+                // the set-up of a group's clean footprints is formed first so its latency overlaps,
+                // then the group's slice loops run in projection order (the reference's summation
+                // order), one copy of them in the instruction cache: the set-up moves down a register
+                // per projection. n is the floor of u >= 0, from the bits of u + 1.5 * 2^23 added
+                // rounding down. The smaller n's offset, twice, plus the step to the other row's.
+                uint32_t q_at[G];
+                float q_d0[G], q_d1[G];
 #pragma unroll
-                for (int e = 0; e < G; ++e) q_mode[e] = setup(b0 + e, q_n[e], q_off[e], q_wa[e], q_wb[e]);
-                // a footprint that did not fit its box (rare; uniform over the CTA) sends the
-                // whole group through the in-order path with guarded global loads
-                bool fallback = false;
+                for (int e = 0; e < G; ++e) {
+                    const float4 g = reinterpret_cast<const float4 *>(S.geo)[gb * NB + b0 + e];
+                    const float u0 = posu<MODE>(g.x, g.y, g.z, fx, fy0, P.toff), u1 = posu<MODE>(g.x, g.y, g.z, fx, fy1, P.toff);
+                    const float k0 = __fadd_rd(u0, kMagic), k1 = __fadd_rd(u1, kMagic);
+                    q_d0[e] = __fsub_rn(u0, __fsub_rn(k0, kMagic));
+                    q_d1[e] = __fsub_rn(u1, __fsub_rn(k1, kMagic));
+                    const int n0 = __float_as_int(k0), n1 = __float_as_int(k1); // biased by kMagicBits
+                    const int lo = g.y >= 0.0f ? n0 : n1;
+                    q_at[e] = static_cast<uint32_t>(2 * (lo + ((st * NB + b0 + e) * (BW * TZ) - kMagicBits - S.meta[st * NB + b0 + e].x)) +
+                                                    (n0 != n1));
+                }
+                if constexpr (MODE == kTilt) {
+                    for (int g = 0; g < group0; ++g) {
 #pragma unroll
-                for (int e = 0; e < G; ++e)
-                    fallback |= s * NB + b0 + e < P.nproj && S.meta[st * NB + b0 + e].y == 0;
-                if (!fallback) {
-#pragma unroll
-                    for (int e = 0; e < G; ++e) {
-                        if (q_mode[e] != 1) continue;
-                        if (!MR_IN_BOUNDS(q_off[e] + (zmax - 1) * BW + 1, 2 * NB * BW * TZ, kSiteBpStaged)) continue;
-                        const float w = HASW ? S.geo[(gb * NB + b0 + e) * GEO + 3] : 1.0f;
-                        if (NN) {
-                            if (zmax == TZ) staged_column_nn<HASW, true>(acc, S.box + q_off[e], w, zmax);
-                            else staged_column_nn<HASW, false>(acc, S.box + q_off[e], w, zmax);
-                        } else if (zmax == TZ) {
-                            staged_column<HASW, true>(acc, S.box + q_off[e], q_wa[e], q_wb[e], w, zmax);
-                        } else {
-                            staged_column<HASW, false>(acc, S.box + q_off[e], q_wa[e], q_wb[e], w, zmax);
+                        for (int e = 0; e < G; ++e) {
+                            q_d0[e] = __fsub_rn(q_d0[e], P.tinc);
+                            q_d1[e] = __fsub_rn(q_d1[e], P.tinc);
                         }
                     }
-                    continue;
                 }
 #pragma unroll 1
-                for (int e = 0; e < G; ++e) {
+                for (int e = 0; e < G && s * NB + b0 + e < P.nproj; ++e) {
                     const int b = b0 + e;
-                    int n;
-                    uint32_t off;
-                    float wa, wb;
-                    const int mode = setup(b, n, off, wa, wb); // formed again: no indexed arrays
-                    const float w = HASW ? S.geo[(gb * NB + b) * GEO + 3] : 1.0f;
-                    if (mode == 1 && !MR_IN_BOUNDS(off + (zmax - 1) * BW + 1, 2 * NB * BW * TZ, kSiteBpStaged)) continue;
-                    if (mode == 1) {
-                        if (NN) staged_column_nn<HASW, false>(acc, S.box + off, w, zmax);
-                        else staged_column<HASW, false>(acc, S.box + off, wa, wb, w, zmax);
-                    } else if (mode == 2) {
-                        const int i = s * NB + b;
-                        const int slab = P.index ? __float_as_int(S.geo[(gb * NB + b) * GEO + 4]) : i;
-                        const float *img = P.proj + (static_cast<size_t>(slab) * P.nv + z0) * P.nu + n;
-#pragma unroll
-                        for (int q = 0; q < TZ; ++q) {
-                            if (q >= zmax) break;
-                            if (NN) {
-                                float pa = __ldg(img + static_cast<size_t>(q) * P.nu);
-                                if (HASW) pa = __fmul_rn(pa, w);
-                                acc[q] = __fadd_rn(acc[q], pa);
-                                continue;
-                            }
-                            float pa = __ldg(img + static_cast<size_t>(q) * P.nu), pb = __ldg(img + static_cast<size_t>(q) * P.nu + 1);
-                            if (HASW) {
-                                pa = __fmul_rn(pa, w);
-                                pb = __fmul_rn(pb, w);
-                            }
-                            acc[q] = __fadd_rn(acc[q], __fadd_rn(__fmul_rn(pa, wa), __fmul_rn(pb, wb)));
+                    const int4 m = S.meta[st * NB + b];
+                    const float4 g = reinterpret_cast<const float4 *>(S.geo)[gb * NB + b];
+                    if (m.y == kClean) {
+                        const bool step = q_at[0] & 1;
+                        const uint32_t at = q_at[0] >> 1;
+                        if (!MR_IN_BOUNDS(at + (TZ - 1) * BW + 1 + step, 2 * NB * BW * TZ, kSiteBpStaged)) {
+                        } else if constexpr (kOneSample) {
+                            const uint32_t a0 = at + (step && g.y < 0.0f), a1 = at + (step && g.y >= 0.0f);
+                            staged_column<MODE, TZ>(acc0, S.box + a0, q_d0[0], g0, P.tinc, nz);
+                            staged_column<MODE, TZ>(acc1, S.box + a1, q_d1[0], g0, P.tinc, nz);
+                        } else if (g.y >= 0.0f) { // uniform
+                            staged_pair<MODE, TZ>(acc0, acc1, S.box + at, step, q_d0[0], q_d1[0], g0, P.tinc, nz);
+                        } else {
+                            staged_pair<MODE, TZ>(acc1, acc0, S.box + at, step, q_d1[0], q_d0[0], g0, P.tinc, nz);
                         }
+                    } else if (m.y != kNothing) {
+                        if (inside[0]) row(acc0, b, g, m, fy0);
+                        if (inside[1]) row(acc1, b, g, m, fy1);
+                    }
+#pragma unroll
+                    for (int k = 0; k + 1 < G; ++k) {
+                        q_at[k] = q_at[k + 1];
+                        q_d0[k] = q_d0[k + 1];
+                        q_d1[k] = q_d1[k + 1];
                     }
                 }
             }
@@ -339,68 +431,158 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_bp_par_staged(const __
         tma::mbar_wait(&S.bars[st], st ? phase1 : phase0);
         if (s + 1 < nbatch) tma::mbar_wait(&S.bars[st ^ 1], st ? phase0 : phase1);
     }
-    if (inside) {
+    auto store = [&](const float2 (&acc)[TZ / 2], float *c, bool in) {
+        if (!in) return;
 #pragma unroll
         for (int q = 0; q < TZ; q += 4) {
             if (vec) {
-                *reinterpret_cast<float4 *>(col + q) = make_float4(acc[q], acc[q + 1], acc[q + 2], acc[q + 3]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (q + e < zmax) col[q + e] = acc[q + e];
+                *reinterpret_cast<float4 *>(c + q) = make_float4(acc[q / 2].x, acc[q / 2].y, acc[q / 2 + 1].x, acc[q / 2 + 1].y);
+            } else if (q < zmax) {
+                c[q] = acc[q / 2].x;
+                c[q + 1] = acc[q / 2].y;
+                c[q + 2] = acc[q / 2 + 1].x;
+                c[q + 3] = acc[q / 2 + 1].y;
             }
         }
+    };
+    store(acc0, col[0], inside[0]);
+    store(acc1, col[1], inside[1]);
+}
+
+// Projections of a list (all, or through an index) copied to rows of `pitch` floats, multiplied by
+// their weights: what the TMA unit needs (16-byte row pitch and base) when the caller's rows are not.
+__global__ void __launch_bounds__(256) k_repitch(const float *__restrict__ proj, const int32_t *__restrict__ index,
+                                                 const float *__restrict__ weight, int nu, int nv, int pitch,
+                                                 float *__restrict__ out)
+{
+    const int b = blockIdx.y;
+    const size_t slab = index ? index[b] : b;
+    const float *src = proj + slab * nv * static_cast<size_t>(nu);
+    float *dst = out + static_cast<size_t>(b) * nv * pitch;
+    for (int y = blockIdx.x; y < nv; y += gridDim.x)
+        for (int x = threadIdx.x; x < nu; x += blockDim.x) {
+            const float v = __ldg(src + static_cast<size_t>(y) * nu + x);
+            dst[static_cast<size_t>(y) * pitch + x] = weight ? __fmul_rn(v, weight[b]) : v;
+        }
+}
+
+template <int MODE, int TZ, int NW, int NB, int CTAS>
+static mr_status launch_tile(PFN_cuTensorMapEncodeTiled enc, const Params &P, size_t nslabs, cudaStream_t s)
+{
+    CUtensorMap map;
+    cuuint64_t dims[3] = {static_cast<cuuint64_t>(P.nu), static_cast<cuuint64_t>(P.nv), nslabs};
+    cuuint64_t strides[2] = {static_cast<cuuint64_t>(P.pitch) * 4, static_cast<cuuint64_t>(P.pitch) * P.nv * 4};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(BW), static_cast<cuuint32_t>(TZ), 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(P.proj), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
+    const size_t smem = Smem<TZ, NB>::bytes();
+    dim3 grid(div_up(static_cast<size_t>(P.nu), TX), div_up(static_cast<size_t>(P.yend - P.ybegin), 2 * NW),
+              div_up(static_cast<size_t>(P.nz4), TZ));
+    const auto kernel = k_bp_par_staged<MODE, TZ, NW, NB, CTAS>;
+    MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kernel<<<grid, 32 * NW, smem, s>>>(map, P);
+    return check_launch("k_bp_par_staged");
+}
+
+// The tile by size. A thread's set-up per projection is shared by its TZ slices, so a slice costs
+// 1 : 1.2 : 1.5 on 32-, 16- and 8-slice tiles (47.4, 56.9, 73.1 ms on 2048^2 x 64 slices from 1125
+// projections), and the slices a tile holds beyond the volume's cost the same: 40 slices at 500^2
+// from 500 projections take 1.49, 1.33 and 1.46 ms, 12 slices at 700^2 from 400 1.18, 0.69 and 0.92.
+// A volume with fewer 16-slice tiles than SMs is bound by the latency of one tile's projection loop:
+// 96^2 x 16 from 200 projections takes 136, 81 and 66 us.
+template <int MODE>
+static mr_status launch_mode(PFN_cuTensorMapEncodeTiled enc, const Params &P, size_t nslabs, cudaStream_t s)
+{
+    const auto padded = [&](int tz) { return (P.nz4 + tz - 1) / tz * tz; };
+    const int cost32 = 10 * padded(32), cost16 = 12 * padded(16), cost8 = 15 * padded(8);
+    const size_t tiles16 = static_cast<size_t>(div_up(static_cast<size_t>(P.nu), TX)) *
+                           div_up(static_cast<size_t>(P.yend - P.ybegin), 8) * div_up(static_cast<size_t>(P.nz4), 16);
+    if (tiles16 < 148 || (cost8 < cost16 && cost8 < cost32)) return launch_tile<MODE, 8, 4, 16, 4>(enc, P, nslabs, s);
+    if (cost16 < cost32) return launch_tile<MODE, 16, 4, 8, 4>(enc, P, nslabs, s);
+    return launch_tile<MODE, 32, 8, 8, 2>(enc, P, nslabs, s);
+}
+
+static mr_status launch(int mode, const Params &P, size_t nslabs, cudaStream_t s)
+{
+    PFN_cuTensorMapEncodeTiled enc = tma::encode_fn();
+    if (!enc) return MR_ERR_UNSUPPORTED;
+    switch (mode) {
+    case kLinear: return launch_mode<kLinear>(enc, P, nslabs, s);
+    case kNearest: return launch_mode<kNearest>(enc, P, nslabs, s);
+    case kTilt: return launch_mode<kTilt>(enc, P, nslabs, s);
+    case kTiltSerial: return launch_mode<kTiltSerial>(enc, P, nslabs, s);
+    default: return launch_mode<kTiltNearest>(enc, P, nslabs, s);
     }
 }
 
 } // namespace bp2
 
+// Scratch of the re-pitched projections: projections go through in runs of about this many bytes.
+constexpr size_t kRepitchBytes = size_t(1) << 30;
+
 // Returns MR_ERR_UNSUPPORTED when staging does not apply (the caller uses the plain kernel).
-mr_status bp_parallel_staged_launch(const float *proj_d, size_t nslabs, const float *weight_d, const int32_t *index_d,
-                                    const float *sin_d, const float *cos_d, const float *startu_d, size_t nproj,
-                                    size_t nu, size_t nv, const uint32_t *mask_d, size_t y_begin, size_t y_end,
-                                    bool nn, float *vol_d, cudaStream_t s)
+mr_status bp_parallel_staged_launch(int variant, const float *proj_d, size_t nslabs, const float *weight_d,
+                                    const int32_t *index_d, const float *sin_d, const float *cos_d,
+                                    const float *startu_d, size_t nproj, size_t nu, size_t nv, const uint32_t *mask_d,
+                                    int tilt, float toff, float tinc, size_t y_begin, size_t y_end, float *vol_d,
+                                    cudaStream_t s)
 {
     using namespace bp2;
-    if ((nu * 4) % 16 != 0 || (reinterpret_cast<uintptr_t>(proj_d) % 16) != 0 || nv < 4 || nslabs == 0 ||
-        nu < static_cast<size_t>(BW))
-        return MR_ERR_UNSUPPORTED;
-    PFN_cuTensorMapEncodeTiled enc = tma::encode_fn();
-    if (!enc) return MR_ERR_UNSUPPORTED;
-    CUtensorMap map;
-    cuuint64_t dims[3] = {nu, nv, nslabs};
-    cuuint64_t strides[2] = {nu * 4, nu * nv * 4};
-    cuuint32_t box[3] = {static_cast<cuuint32_t>(BW), static_cast<cuuint32_t>(TZ), 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(proj_d), dims, strides, box, estr,
-                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
+    if (nv < 4 || nslabs == 0 || nu < static_cast<size_t>(BW)) return MR_ERR_UNSUPPORTED;
+    const int mode = variant == MR_BP_NEAREST           ? (tilt ? kTiltNearest : kNearest)
+                     : !tilt                            ? kLinear
+                     : variant == MR_BP_MULTIPROJ_SERIAL ? kTiltSerial
+                                                         : kTilt;
     Params P;
-    P.proj = proj_d;
-    P.weight = weight_d;
-    P.index = index_d;
-    P.sinv = sin_d;
-    P.cosv = cos_d;
-    P.startu = startu_d;
     P.mask = mask_d;
     P.vol = vol_d;
-    P.nproj = static_cast<int>(nproj);
     P.nu = static_cast<int>(nu);
     P.nv = static_cast<int>(nv);
     P.nz4 = static_cast<int>((nv / 4) * 4);
     P.wait_limit = tma::g_batch_wait_limit.load();
     P.ybegin = static_cast<int>(y_begin);
     P.yend = static_cast<int>(y_end);
-    const size_t smem = Smem::bytes();
-    dim3 grid(div_up(nu, TX), div_up(y_end - y_begin, TY), div_up(static_cast<size_t>(P.nz4), TZ));
-    auto launch = [&](auto kernel) -> mr_status {
-        MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kernel<<<grid, THREADS, smem, s>>>(map, P);
-        return check_launch("k_bp_par_staged");
-    };
-    if (nn) return weight_d ? launch(k_bp_par_staged<true, true>) : launch(k_bp_par_staged<false, true>);
-    return weight_d ? launch(k_bp_par_staged<true, false>) : launch(k_bp_par_staged<false, false>);
+    P.toff = toff;
+    P.tinc = tinc;
+    P.neg_zero = -0.0f;
+    if (!weight_d && nu % 4 == 0 && reinterpret_cast<uintptr_t>(proj_d) % 16 == 0) {
+        P.proj = proj_d;
+        P.index = index_d;
+        P.sinv = sin_d;
+        P.cosv = cos_d;
+        P.startu = startu_d;
+        P.nproj = static_cast<int>(nproj);
+        P.pitch = P.nu;
+        return launch(mode, P, nslabs, s);
+    }
+    // rows the TMA unit cannot address: re-pitched (and weighted) copies, a run of projections at a
+    // time; the volume carries the sums from one run to the next, in projection order
+    const size_t pitch = (nu + 3) / 4 * 4, per = pitch * nv * sizeof(float);
+    const size_t run = std::min(nproj, std::max<size_t>(32, kRepitchBytes / per / 32 * 32));
+    float *scratch = nullptr;
+    if (run > 65535 || device_alloc(&scratch, run * per, s, "mr_bp_parallel: re-pitched projections") != MR_OK)
+        return MR_ERR_UNSUPPORTED; // no room: the direct-load kernel needs none
+    mr_status st = MR_OK;
+    for (size_t a = 0; a < nproj && st == MR_OK; a += run) {
+        const size_t n = std::min(run, nproj - a);
+        k_repitch<<<dim3(static_cast<unsigned>(std::min<size_t>(nv, 64)), static_cast<unsigned>(n)), 256, 0, s>>>(
+            index_d ? proj_d : proj_d + a * nu * nv, index_d ? index_d + a : nullptr, weight_d ? weight_d + a : nullptr,
+            P.nu, P.nv, static_cast<int>(pitch), scratch);
+        st = check_launch("k_repitch");
+        P.proj = scratch;
+        P.index = nullptr;
+        P.sinv = sin_d + a;
+        P.cosv = cos_d + a;
+        P.startu = startu_d + a;
+        P.nproj = static_cast<int>(n);
+        P.pitch = static_cast<int>(pitch);
+        if (st == MR_OK) st = launch(mode, P, n, s);
+    }
+    cudaFreeAsync(scratch, s);
+    return st;
 }
 
 // mr_backproject.cu: the direct-load kernel for a range of volume rows
@@ -431,12 +613,13 @@ extern "C" mr_status mr_bp_parallel_variant(int variant, const void *proj_d, siz
     // unless the tilt is corrected or the slice count is not a multiple of 4 (its second
     // interpolation sample is then read from another place of its projection buffer)
     if (variant == MR_BP_MULTIPROJ_SERIAL && !correcttilt && (nv & 3) == 0) variant = MR_BP_MULTIPROJ_PARALLEL;
-    if (variant != MR_BP_MULTIPROJ_SERIAL && dtype == MR_F32 && !correcttilt && nproj > 0 && nproj <= 0x7fffffff &&
-        nu >= 2 && nu <= 65536 && nv <= 65536 && y_begin < y_end) {
+    const bool other_column = variant == MR_BP_MULTIPROJ_SERIAL && (nv & 3) != 0;
+    if (!other_column && dtype == MR_F32 && nproj > 0 && nproj <= 0x7fffffff && nu >= 2 && nu <= 65536 &&
+        nv <= 65536 && y_begin < y_end) {
         if (!index_d && nslabs < nproj) return fail(MR_ERR_ARGUMENT, "mr_bp_parallel_variant: nslabs below nproj");
-        mr_status st = bp_parallel_staged_launch(static_cast<const float *>(proj_d), nslabs, weight_d, index_d, sin_d,
-                                                 cos_d, startu_d, nproj, nu, nv, mask_d, y_begin, y_end,
-                                                 variant == MR_BP_NEAREST, vol_d, as_stream(stream));
+        mr_status st = bp_parallel_staged_launch(variant, static_cast<const float *>(proj_d), nslabs, weight_d, index_d,
+                                                 sin_d, cos_d, startu_d, nproj, nu, nv, mask_d, correcttilt, tiltoffset,
+                                                 tiltinc, y_begin, y_end, vol_d, as_stream(stream));
         if (st != MR_ERR_UNSUPPORTED) return st;
     }
     return bp_parallel_rows(proj_d, dtype, scale_d, weight_d, index_d, sin_d, cos_d, startu_d, nproj, nu, nv, mask_d,
