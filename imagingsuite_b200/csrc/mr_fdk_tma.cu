@@ -65,7 +65,8 @@ constexpr int CTAS_PER_SM = 2;
 constexpr float kMagic = 12582912.0f; // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
 // per-projection geometry staged in shared memory (floats)
-constexpr int GEO_EXACT = TK + 3 * TI + 3 * TJ + 4; // zip1[TK], xip[TI][3], yip[TJ][3], Z0, Z2
+constexpr int GX = 3 * TK, GY = GX + 3 * TI, G0 = GY + 3 * TJ; // zip[TK][3], xip[TI][3], yip[TJ][3], zip[0][3]
+constexpr int GEO_EXACT = G0 + 4;
 constexpr int GEO_FAST = 32;                        // FP64 map[12] (24 words), scale, pad
 // per-projection tile geometry of the fast kernel (floats, formed from the FP64 map)
 constexpr int TGEO = 16;
@@ -79,13 +80,16 @@ struct Params {
     const uint32_t *mask;
     float *vol;
     int nu, nv, nproj;
+    int pitch;        // elements between detector rows
     int bw, bh;       // TMA box (elements)
     int boxbytes;     // per-projection shared buffer, 128-byte multiple
     int rowbytes;     // bw * element size
     int accumulate;
     int kbegin, kend; // cbct slices backprojected: [kbegin, kend)
+    int geo16;        // geometry rows are copied 16 bytes at a time (exact kernel)
     int xalign;       // x coordinate alignment of a TMA load (elements)
     int wait_limit;   // tries of each per-batch wait
+    float neg_zero;   // -0 (see exact_column)
 };
 
 using tma::mbar_expect_tx;
@@ -181,20 +185,18 @@ __device__ __forceinline__ void fast_coord(const TG &t, float di, float dj, floa
 // Slices of one voxel column for one staged projection (exact arithmetic). a1: the 32
 // per-slice sums zip1 + yip1 of this warp. FULL: all TK slices exist.
 //
-// Two slices per step on the paired FP32 pipe: (a1 + x1) and dw * (...) as f32x2 add and mul,
-// + 0.5 as two scalar adds, the magic-number floor as one f32x2 add rounded down, and
-// dw2 * v as one f32x2 mul followed by two scalar adds into the accumulators. Every operation
-// is IEEE-rounded on its own, so each slice gets exactly the reference's float sequence; an
-// f32x2 mul is never followed directly by an f32x2 add, because ptxas contracts that pair into
-// an f32x2 fma even with explicit rounding.
+// Two slices per step on the paired FP32 pipe, every operation IEEE-rounded on its own, so each
+// slice gets exactly the reference's float sequence: the two products are fmas with an addend of
+// -0 (`nz`, a kernel argument; p + -0 is p bit for bit), because ptxas contracts an f32x2 mul that
+// feeds an f32x2 add into one fma even with explicit rounding.
 template <bool FULL>
 __device__ __forceinline__ void exact_column(float2 (&acc)[TK / 2], const unsigned char *smem, uint32_t base,
                                              uint32_t rowbytes, const float *a1, float x1f, float dw, float dw2,
-                                             int kmax, uint32_t stage_bytes)
+                                             int kmax, float2 nz, uint32_t stage_bytes)
 {
     (void)stage_bytes; // the stage buffers' size, for the bounds-checked build
     const float2 x1 = make_float2(x1f, x1f), dwp = make_float2(dw, dw), dw2p = make_float2(dw2, dw2);
-    const float2 mg = make_float2(kMagic, kMagic);
+    const float2 mg = make_float2(kMagic, kMagic), half = make_float2(0.5f, 0.5f);
 #pragma unroll
     for (int q4 = 0; q4 < TK / 4; ++q4) {
         const float4 a4 = reinterpret_cast<const float4 *>(a1)[q4];
@@ -203,16 +205,16 @@ __device__ __forceinline__ void exact_column(float2 (&acc)[TK / 2], const unsign
             const int q = 4 * q4 + 2 * h; // slices q and q + 1 -> acc[q / 2]
             if (!FULL && q >= kmax) break;
             const bool two = FULL || q + 1 < kmax;
-            const float2 m = __fmul2_rn(dwp, __fadd2_rn(h ? make_float2(a4.z, a4.w) : make_float2(a4.x, a4.y), x1));
-            const float2 b = __fadd2_rd(make_float2(__fadd_rn(m.x, 0.5f), __fadd_rn(m.y, 0.5f)), mg);
+            const float2 m = __ffma2_rn(dwp, __fadd2_rn(h ? make_float2(a4.z, a4.w) : make_float2(a4.x, a4.y), x1), nz);
+            const float2 b = __fadd2_rd(__fadd2_rn(m, half), mg);
             const uint32_t o0 = __float_as_uint(b.x) * rowbytes + base, o1 = __float_as_uint(b.y) * rowbytes + base;
             const float v0 = MR_IN_BOUNDS(o0, stage_bytes, kSiteFdkStaged) ? *reinterpret_cast<const float *>(smem + o0) : 0.0f;
             const float v1 = two && MR_IN_BOUNDS(o1, stage_bytes, kSiteFdkStaged)
                                  ? *reinterpret_cast<const float *>(smem + o1)
                                  : 0.0f;
-            const float2 p = __fmul2_rn(dw2p, make_float2(v0, v1));
-            acc[q >> 1].x = __fadd_rn(acc[q >> 1].x, p.x);
-            if (two) acc[q >> 1].y = __fadd_rn(acc[q >> 1].y, p.y);
+            const float2 p = __ffma2_rn(dw2p, make_float2(v0, v1), nz);
+            if (two) acc[q >> 1] = __fadd2_rn(acc[q >> 1], p);
+            else acc[q >> 1].x = __fadd_rn(acc[q >> 1].x, p.x);
         }
     }
 }
@@ -271,27 +273,25 @@ struct Smem {
     }
 };
 
-// Sources of the exact kernel's geometry elements of a batch, fixed for the tile: element idx
-// (projection b = idx / GEO_EXACT of the batch) is array[offset + p * stride], p the projection;
-// bits 0-25 the offset, 26-27 the array (0 zip, 1 xip, 2 yip, 3 none: zero), 28-31 b.
+// Sources of the exact kernel's geometry of a batch, fixed for the tile: element (or, with geo16,
+// run of four elements) idx of projection b = idx / (elements per projection) is array[offset + p *
+// stride], p the projection; bits 0-25 the offset, 26-27 the array (0 zip, 1 xip, 2 yip, 3 none:
+// zero), 28-31 b.
 template <int NB>
-__device__ __forceinline__ void geometry_sources(const Params &P, uint32_t *gdesc, int i0, int j0, int k0, int kmax)
+__device__ __forceinline__ void geometry_sources(const Params &P, uint32_t *gdesc, int i0, int j0, int k0)
 {
-    for (int idx = threadIdx.x; idx < NB * GEO_EXACT; idx += THREADS) {
-        const int b = idx / GEO_EXACT, e = idx % GEO_EXACT;
+    const int run = P.geo16 ? 4 : 1, per = GEO_EXACT / run;
+    for (int idx = threadIdx.x; idx < NB * per; idx += THREADS) {
+        const int b = idx / per, e = idx % per * run;
         uint32_t arr = 3, off = 0;
-        if (e < TK) {
-            if (e < kmax) arr = 0, off = static_cast<uint32_t>((k0 + e) * 3 + 1);
-        } else if (e < TK + 3 * TI) {
-            const int ii = i0 + (e - TK) / 3;
-            if (ii < P.nu) arr = 1, off = static_cast<uint32_t>(ii * 3 + (e - TK) % 3);
-        } else if (e < TK + 3 * TI + 3 * TJ) {
-            const int jj = j0 + (e - TK - 3 * TI) / 3;
-            if (jj < P.nu) arr = 2, off = static_cast<uint32_t>(jj * 3 + (e - TK - 3 * TI) % 3);
-        } else if (e == TK + 3 * TI + 3 * TJ) {
-            arr = 0, off = 0;
-        } else if (e == TK + 3 * TI + 3 * TJ + 1) {
-            arr = 0, off = 2;
+        if (e < GX) {
+            if (k0 + e / 3 < P.nv) arr = 0, off = static_cast<uint32_t>(k0 * 3 + e);
+        } else if (e < GY) {
+            if (i0 + (e - GX) / 3 < P.nu) arr = 1, off = static_cast<uint32_t>(i0 * 3 + e - GX);
+        } else if (e < G0) {
+            if (j0 + (e - GY) / 3 < P.nu) arr = 2, off = static_cast<uint32_t>(j0 * 3 + e - GY);
+        } else if (e < G0 + 3) {
+            arr = 0, off = static_cast<uint32_t>(e - G0);
         }
         gdesc[idx] = off | arr << 26 | static_cast<uint32_t>(b) << 28;
     }
@@ -300,19 +300,20 @@ __device__ __forceinline__ void geometry_sources(const Params &P, uint32_t *gdes
 // Starts the asynchronous copy of batch s's per-projection geometry into geometry buffer gb
 // (all threads; zero where a projection, column, row or slice does not exist).
 template <bool EXACT, int NB>
-__device__ __forceinline__ void stage_geometry(const Params &P, float *geo, int s, int i0, int j0, int k0, int kmax,
-                                               const uint32_t *gdesc)
+__device__ __forceinline__ void stage_geometry(const Params &P, float *geo, int s, const uint32_t *gdesc)
 {
     if constexpr (EXACT) {
-        const size_t zstride = static_cast<size_t>(P.nv) * 3, xstride = static_cast<size_t>(P.nu) * 3;
-        for (int idx = threadIdx.x; idx < NB * GEO_EXACT; idx += THREADS) {
+        const uint32_t zstride = static_cast<uint32_t>(P.nv) * 3, xstride = static_cast<uint32_t>(P.nu) * 3;
+        const int count = P.geo16 ? NB * GEO_EXACT / 4 : NB * GEO_EXACT;
+        for (int idx = threadIdx.x; idx < count; idx += THREADS) {
             const uint32_t d = gdesc[idx];
             const uint32_t arr = (d >> 26) & 3;
             const int p = s * NB + static_cast<int>(d >> 28);
             const bool ok = arr != 3 && p < P.nproj;
             const float *base = arr == 0 ? P.zip : arr == 1 ? P.xip : P.yip;
             const float *src = base + (d & 0x3FFFFFFu) + static_cast<size_t>(p) * (arr == 0 ? zstride : xstride);
-            copy4_zfill(geo + idx, ok ? src : P.zip, ok);
+            if (P.geo16) tma::copy16_zfill(geo + 4 * idx, ok ? src : P.zip, ok);
+            else copy4_zfill(geo + idx, ok ? src : P.zip, ok);
         }
     } else {
         const float *maps = reinterpret_cast<const float *>(P.maps); // 24 words per projection
@@ -345,9 +346,9 @@ __device__ __forceinline__ void issue_batch(const Params &P, const CUtensorMap *
         float r, c;
         if constexpr (EXACT) {
             const float *g = geo + b * GEO_EXACT;
-            const float *X = g + TK + 3 * (ci - i0), *Y = g + TK + 3 * TI + 3 * (cj - j0);
-            const float Z0 = g[TK + 3 * TI + 3 * TJ], Z2 = g[TK + 3 * TI + 3 * TJ + 1];
-            const float a1 = __fadd_rn(g[(corner & 4) ? kmax - 1 : 0], Y[1]);
+            const float *X = g + GX + 3 * (ci - i0), *Y = g + GY + 3 * (cj - j0);
+            const float Z0 = g[G0], Z2 = g[G0 + 2];
+            const float a1 = __fadd_rn(g[(corner & 4) ? 3 * (kmax - 1) + 1 : 1], Y[1]);
             const float dw = __frcp_rn(__fadd_rn(__fadd_rn(Z2, Y[2]), X[2]));
             r = __fadd_rn(__fmul_rn(dw, __fadd_rn(a1, X[1])), 0.5f);
             c = __fadd_rn(__fmul_rn(dw, __fadd_rn(__fadd_rn(Z0, Y[0]), X[0])), 0.5f);
@@ -485,11 +486,11 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
 
     // geometry of batches 0-2, footprints and copies of batches 0-1
     if constexpr (EXACT) {
-        geometry_sources<NB>(P, S.gdesc, i0, j0, k0, kmax);
+        geometry_sources<NB>(P, S.gdesc, i0, j0, k0);
         __syncthreads();
     }
     for (int s = 0; s < 3 && s < nbatch; ++s)
-        stage_geometry<EXACT, NB>(P, S.geo + s * NB * GEO, s, i0, j0, k0, kmax, S.gdesc);
+        stage_geometry<EXACT, NB>(P, S.geo + s * NB * GEO, s, S.gdesc);
     copy_wait_all();
     __syncthreads();
     for (int s = 0; s < 2 && s < nbatch; ++s)
@@ -502,6 +503,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
     const float fdi = static_cast<float>(lane), fdj = static_cast<float>(warp); // voxel offset in the tile
     const uint32_t rowbytes = static_cast<uint32_t>(P.rowbytes);
     const bool warp_inside = __any_sync(0xffffffffu, inside);
+    const float2 nz = make_float2(P.neg_zero, P.neg_zero);
     int s = 0;
     for (int gb = 0; s < nbatch; ++s, gb = gb == 2 ? 0 : gb + 1) {
         const int st = s & 1;  // stage buffer
@@ -522,12 +524,12 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
             if (got && warp_inside) {
                 for (int idx = lane; idx < NB * TK; idx += 32) {
                     const float *g = geo + (idx / TK) * GEO_EXACT;
-                    S.a1[warp * NB * TK + idx] = __fadd_rn(g[idx % TK], g[TK + 3 * TI + 3 * warp + 1]);
+                    S.a1[warp * NB * TK + idx] = __fadd_rn(g[3 * (idx % TK) + 1], g[GY + 3 * warp + 1]);
                 }
                 if (lane < NB) { // the warp-uniform first sums of the set-up: (Z0 + y0), (Z2 + y2)
                     const float *g = geo + lane * GEO_EXACT;
-                    S.zy[warp * NB + lane] = make_float2(__fadd_rn(g[TK + 3 * TI + 3 * TJ], g[TK + 3 * TI + 3 * warp]),
-                                                         __fadd_rn(g[TK + 3 * TI + 3 * TJ + 1], g[TK + 3 * TI + 3 * warp + 2]));
+                    S.zy[warp * NB + lane] = make_float2(__fadd_rn(g[G0], g[GY + 3 * warp]),
+                                                         __fadd_rn(g[G0 + 2], g[GY + 3 * warp + 2]));
                 }
                 __syncwarp();
             }
@@ -547,7 +549,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
                 if (p >= P.nproj || m.z != 1) return false;
                 if constexpr (EXACT) {
                     const float *g = geo + b * GEO;
-                    const float x0f = g[TK + 3 * lane], x1f = g[TK + 3 * lane + 1], x2f = g[TK + 3 * lane + 2];
+                    const float x0f = g[GX + 3 * lane], x1f = g[GX + 3 * lane + 1], x2f = g[GX + 3 * lane + 2];
                     const float2 zy = S.zy[warp * NB + b];
                     const float dw = __frcp_rn(__fadd_rn(zy.y, x2f));
                     const float c = __fadd_rn(__fmul_rn(dw, __fadd_rn(zy.x, x0f)), 0.5f);
@@ -601,10 +603,10 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
                             const float *a1 = S.a1 + (warp * NB + b0 + e) * TK;
                             if (kmax == TK)
                                 exact_column<true>(acc, smem, q_base[e], rowbytes, a1, q_c[e], q_a[e], q_b[e], kmax,
-                                                   stage_bytes);
+                                                   nz, stage_bytes);
                             else
                                 exact_column<false>(acc, smem, q_base[e], rowbytes, a1, q_c[e], q_a[e], q_b[e], kmax,
-                                                    stage_bytes);
+                                                    nz, stage_bytes);
                         } else {
                             const unsigned short wt = static_cast<unsigned short>(__float_as_uint(q_c[e]));
                             if (kmax == TK)
@@ -624,31 +626,31 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
                     if (setup(b, qa, qb, qc, qbase)) { // set-up formed again: no indexed arrays
                         if constexpr (EXACT)
                             exact_column<false>(acc, smem, qbase, rowbytes, S.a1 + (warp * NB + b) * TK, qc, qa, qb, kmax,
-                                                stage_bytes);
+                                                nz, stage_bytes);
                         else
                             fast_column_staged<DT, false>(acc, smem, qbase, rowbytes, qa, qb,
-                                                          static_cast<unsigned short>(__float_as_uint(qc)), kmax);
+                                                               static_cast<unsigned short>(__float_as_uint(qc)), kmax);
                         continue;
                     }
                     if (p >= P.nproj || S.meta[st * NB + b].z != 0) continue;
                     const float *g = geo + b * GEO;
                     if constexpr (EXACT) {
-                        const float x0f = g[TK + 3 * lane], x1f = g[TK + 3 * lane + 1], x2f = g[TK + 3 * lane + 2];
-                        const float y0f = g[TK + 3 * TI + 3 * warp], y2f = g[TK + 3 * TI + 3 * warp + 2];
-                        const float Z0 = g[TK + 3 * TI + 3 * TJ], Z2 = g[TK + 3 * TI + 3 * TJ + 1];
+                        const float x0f = g[GX + 3 * lane], x1f = g[GX + 3 * lane + 1], x2f = g[GX + 3 * lane + 2];
+                        const float y0f = g[GY + 3 * warp], y2f = g[GY + 3 * warp + 2];
+                        const float Z0 = g[G0], Z2 = g[G0 + 2];
                         const float dw = __frcp_rn(__fadd_rn(__fadd_rn(Z2, y2f), x2f));
                         const float c = __fadd_rn(__fmul_rn(dw, __fadd_rn(__fadd_rn(Z0, y0f), x0f)), 0.5f);
                         if (c < 0.0f || c >= fw) continue;
                         const float dw2 = __fmul_rn(dw, dw);
                         const float *a1 = S.a1 + (warp * NB + b) * TK;
-                        const float *img = static_cast<const float *>(P.proj) + static_cast<size_t>(p) * P.nu * P.nv +
+                        const float *img = static_cast<const float *>(P.proj) + static_cast<size_t>(p) * P.pitch * P.nv +
                                            static_cast<int>(c);
 #pragma unroll
                         for (int q = 0; q < TK; ++q) {
                             if (q >= kmax) break;
                             const float r = __fadd_rn(__fmul_rn(dw, __fadd_rn(a1[q], x1f)), 0.5f);
                             if (r < 0.0f || r >= fh) continue;
-                            const float v = __ldg(img + static_cast<size_t>(static_cast<int>(r)) * P.nu);
+                            const float v = __ldg(img + static_cast<size_t>(static_cast<int>(r)) * P.pitch);
                             float &a = (q & 1) ? acc[q >> 1].y : acc[q >> 1].x;
                             a = __fadd_rn(a, __fmul_rn(dw2, v));
                         }
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
                         const int col = __float_as_int(t[TG_C0]) + __float2int_rd(tc);
                         if (col < 0 || col >= P.nu) continue;
                         const unsigned short wt = to_storage<DT>(dw * dw * (t[TG_SCALE] * ginv));
-                        const T *img = static_cast<const T *>(P.proj) + static_cast<size_t>(p) * P.nu * P.nv + col;
+                        const T *img = static_cast<const T *>(P.proj) + static_cast<size_t>(p) * P.pitch * P.nv + col;
                         const float wf = from_storage<DT>(wt);
                         const int r0 = __float_as_int(t[TG_R0]);
                         float2 rr = make_float2(tr0, __fadd_rn(tr0, dr));
@@ -671,7 +673,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
                             const int row = r0 + __float2int_rd((q & 1) ? rr.y : rr.x);
                             if (q & 1) rr = __fadd2_rn(rr, step);
                             if (row < 0 || row >= P.nv) continue;
-                            const unsigned short v = reinterpret_cast<const unsigned short *>(img)[static_cast<size_t>(row) * P.nu];
+                            const unsigned short v = reinterpret_cast<const unsigned short *>(img)[static_cast<size_t>(row) * P.pitch];
                             float &a = (q & 1) ? acc[q >> 1].y : acc[q >> 1].x;
                             a = fmaf(from_storage<DT>(v), wf, a);
                         }
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
             const int g2 = gb == 0 ? 2 : gb - 1;
             issue_batch<DT, EXACT, NB>(P, &tmap, S, S.geo + g2 * NB * GEO, s + 2, st, i0, j0, k0, i_hi, j_hi, kmax);
         }
-        if (s + 3 < nbatch) stage_geometry<EXACT, NB>(P, S.geo + gb * NB * GEO, s + 3, i0, j0, k0, kmax, S.gdesc);
+        if (s + 3 < nbatch) stage_geometry<EXACT, NB>(P, S.geo + gb * NB * GEO, s + 3, S.gdesc);
     }
     if (failed) {
         // copies still in flight: batch s (its wait expired) and batch s+1 when it was issued;
@@ -814,12 +816,30 @@ static void box_guess(size_t nu, size_t nv, size_t nproj, int xalign, int &bw, i
     bh = std::min(bh, 256);
 }
 
+// Filtered projections copied to float rows of `pitch` (16-bit samples times their projection's scale,
+// as the direct-load kernel reads them): what the TMA unit and the exact kernel need when the caller's
+// rows are not a multiple of 16 bytes or hold 16-bit samples.
+template <int DT>
+__global__ void __launch_bounds__(256) k_fdk_repitch(const void *__restrict__ proj, const float *__restrict__ scale, int nu,
+                                                     int nv, int pitch, float *__restrict__ out)
+{
+    const int p = blockIdx.y;
+    const auto *src = static_cast<const typename Sample<DT>::T *>(proj) + static_cast<size_t>(p) * nu * nv;
+    float *dst = out + static_cast<size_t>(p) * nv * pitch;
+    const float sc = DT == MR_F32 ? 1.0f : scale[p];
+    for (int y = blockIdx.x; y < nv; y += gridDim.x)
+        for (int x = threadIdx.x; x < nu; x += blockDim.x) {
+            const float v = Sample<DT>::load(src, static_cast<size_t>(y) * nu + x);
+            dst[static_cast<size_t>(y) * pitch + x] = DT == MR_F32 ? v : __fmul_rn(v, sc);
+        }
+}
+
 } // namespace fdk2
 
-// Launches a staged FDK kernel; returns MR_ERR_UNSUPPORTED when the layout does not allow
+// Launches a staged FDK kernel on rows of `pitch` elements; returns MR_ERR_UNSUPPORTED when the layout does not allow
 // TMA or the box does not fit shared memory (the caller then uses the plain kernel).
-static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const float *scale_d, size_t nu, size_t nv,
-                               size_t nproj, const float *xip_d, const float *yip_d, const float *zip_d,
+static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const float *scale_d, size_t nu, size_t pitch,
+                               size_t nv, size_t nproj, const float *xip_d, const float *yip_d, const float *zip_d,
                                const double *maps_d, const uint32_t *mask_d, int accumulate, int kbegin, int kend,
                                float *vol_d, int bw,
                                int bh, cudaStream_t s)
@@ -827,14 +847,14 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
     using namespace fdk2;
     const size_t es = dtype == MR_F32 ? 4 : 2;
     const int xalign = static_cast<int>(16 / es);
-    if ((nu * es) % 16 != 0 || (reinterpret_cast<uintptr_t>(proj_d) % 16) != 0) return MR_ERR_UNSUPPORTED;
+    if ((pitch * es) % 16 != 0 || (reinterpret_cast<uintptr_t>(proj_d) % 16) != 0) return MR_ERR_UNSUPPORTED;
     if (bw <= 0 || bh <= 0 || bw > 256 || bh > 256 || bw % xalign) return MR_ERR_UNSUPPORTED;
     PFN_cuTensorMapEncodeTiled enc = tma::encode_fn();
     if (!enc) return fail(MR_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
     constexpr size_t kMaxSmem = (227 * 1024) / CTAS_PER_SM - 1024; // CTAS_PER_SM CTAs per SM
     CUtensorMap map;
     cuuint64_t dims[3] = {nu, nv, nproj};
-    cuuint64_t strides[2] = {nu * es, nu * nv * es};
+    cuuint64_t strides[2] = {pitch * es, pitch * nv * es};
     cuuint32_t box[3] = {static_cast<cuuint32_t>(bw), static_cast<cuuint32_t>(bh), 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUtensorMapDataType t = dtype == MR_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
@@ -853,6 +873,7 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
     P.mask = mask_d;
     P.vol = vol_d;
     P.nu = static_cast<int>(nu);
+    P.pitch = static_cast<int>(pitch);
     P.nv = static_cast<int>(nv);
     P.nproj = static_cast<int>(nproj);
     P.bw = bw;
@@ -864,6 +885,7 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
     P.kend = kend;
     P.xalign = xalign;
     P.wait_limit = tma::g_batch_wait_limit.load();
+    P.neg_zero = -0.0f;
     dim3 grid(div_up(nu, TI), div_up(nu, TJ), div_up(static_cast<size_t>(kend - kbegin), TK));
     auto go = [&](auto kernel, size_t smem) -> mr_status {
         MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem)));
@@ -872,6 +894,8 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
     };
     if (exact) {
         if (dtype != MR_F32) return MR_ERR_UNSUPPORTED;
+        P.geo16 = nu % 4 == 0 && nv % 4 == 0 && kbegin % 4 == 0 &&
+                  ((reinterpret_cast<uintptr_t>(xip_d) | reinterpret_cast<uintptr_t>(yip_d) | reinterpret_cast<uintptr_t>(zip_d)) % 16) == 0;
         const size_t s8 = Smem<8, GEO_EXACT, true>::bytes(P.boxbytes), s4 = Smem<4, GEO_EXACT, true>::bytes(P.boxbytes);
         if (s8 <= kMaxSmem) return go(k_fdk_staged<MR_F32, true, 8>, s8);
         if (s4 <= kMaxSmem) return go(k_fdk_staged<MR_F32, true, 4>, s4);
@@ -888,12 +912,40 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
     return MR_ERR_UNSUPPORTED;
 }
 
+// The exact kernel on any layout. FP32 rows that are a multiple of 16 bytes are read where they are;
+// other widths, and 16-bit projections, go through re-pitched FP32 copies, a run of projections (about
+// 1 GiB of scratch) at a time, each run continuing the volume's sums in projection order. Without room
+// for a run the caller's direct-load kernel does the work.
 mr_status fdk_tma_launch(const void *proj_d, int dtype, const float *scale_d, size_t nu, size_t nv, size_t nproj,
                          const float *xip_d, const float *yip_d, const float *zip_d, const uint32_t *mask_d,
                          int accumulate, int kbegin, int kend, float *vol_d, int bw, int bh, cudaStream_t s)
 {
-    return staged_launch(true, proj_d, dtype, scale_d, nu, nv, nproj, xip_d, yip_d, zip_d, nullptr, mask_d, accumulate,
-                         kbegin, kend, vol_d, bw, bh, s);
+    if (dtype == MR_F32 && nu % 4 == 0 && reinterpret_cast<uintptr_t>(proj_d) % 16 == 0)
+        return staged_launch(true, proj_d, dtype, scale_d, nu, nu, nv, nproj, xip_d, yip_d, zip_d, nullptr, mask_d,
+                             accumulate, kbegin, kend, vol_d, bw, bh, s);
+    constexpr size_t kScratch = size_t(1) << 30;
+    const size_t pitch = (nu + 3) / 4 * 4, per = pitch * nv * sizeof(float);
+    const size_t run = std::min({nproj, std::max<size_t>(16, kScratch / per), size_t(65535)});
+    float *scratch = nullptr;
+    if (device_alloc(&scratch, run * per, s, "mr_fdk_backproject: re-pitched projections") != MR_OK)
+        return MR_ERR_UNSUPPORTED;
+    mr_status st = MR_OK;
+    for (size_t a = 0; a < nproj && st == MR_OK; a += run) {
+        const size_t n = std::min(run, nproj - a);
+        const dim3 grid(static_cast<unsigned>(std::min<size_t>(nv, 64)), static_cast<unsigned>(n));
+        const int inu = static_cast<int>(nu), inv = static_cast<int>(nv), ip = static_cast<int>(pitch);
+        const char *src = static_cast<const char *>(proj_d) + a * nu * nv * (dtype == MR_F32 ? 4 : 2);
+        if (dtype == MR_F32) fdk2::k_fdk_repitch<MR_F32><<<grid, 256, 0, s>>>(src, nullptr, inu, inv, ip, scratch);
+        else if (dtype == MR_BF16) fdk2::k_fdk_repitch<MR_BF16><<<grid, 256, 0, s>>>(src, scale_d + a, inu, inv, ip, scratch);
+        else fdk2::k_fdk_repitch<MR_F16><<<grid, 256, 0, s>>>(src, scale_d + a, inu, inv, ip, scratch);
+        st = check_launch("k_fdk_repitch");
+        if (st == MR_OK)
+            st = staged_launch(true, scratch, MR_F32, nullptr, nu, pitch, nv, n, xip_d + a * nu * 3, yip_d + a * nu * 3,
+                               zip_d + a * nv * 3, nullptr, mask_d, accumulate || a > 0, kbegin, kend, vol_d, bw, bh, s);
+        if (st == MR_ERR_UNSUPPORTED) break; // the box does not fit: found on the first run
+    }
+    cudaFreeAsync(scratch, s);
+    return st;
 }
 
 mr_status fdk_box_for(const float *xip_h, const float *yip_h, const float *zip_h, size_t nu, size_t nv, size_t nproj,
@@ -956,7 +1008,7 @@ mr_status mr_fdk_backproject_fast(const void *proj_d, int dtype, const float *sc
     if (nu == 0 || nv == 0 || nu > 65536 || nv > 65536)
         return fail(MR_ERR_ARGUMENT, "mr_fdk_backproject_fast: unsupported size");
     if (nproj == 0 || nproj > 0x7fffffff) return fail(MR_ERR_ARGUMENT, "mr_fdk_backproject_fast: projection count");
-    mr_status st = staged_launch(false, proj_d, dtype, scale_d, nu, nv, nproj, nullptr, nullptr, nullptr, maps_d,
+    mr_status st = staged_launch(false, proj_d, dtype, scale_d, nu, nu, nv, nproj, nullptr, nullptr, nullptr, maps_d,
                                  mask_d, accumulate, 0, static_cast<int>(nv), vol_d, box_w, box_h, as_stream(stream));
     if (st == MR_ERR_UNSUPPORTED)
         return fail(MR_ERR_UNSUPPORTED,

@@ -76,6 +76,13 @@ __device__ __forceinline__ void copy4_zfill(float *dst, const float *src, bool v
                  : "memory");
 }
 
+// The same for 16 bytes; dst and src 16-byte aligned.
+__device__ __forceinline__ void copy16_zfill(float *dst, const float *src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
 // Completes this thread's outstanding cp.async copies (a barrier then publishes them).
 __device__ __forceinline__ void copy_wait_all()
 {

@@ -1104,15 +1104,16 @@ class FDKbp_single(_BackProjectorBase):
             xip, yip, zip_, s2, sc, uni = self.partials(angles)
             bw, bh = ctypes.c_int(0), ctypes.c_int(0)
             maps = None
-            if uni and dtype != L.MR_F32:
+            if uni and dtype != L.MR_F32 and nu % 8 == 0:
                 # precision form: FP64 detector maps (the kernel forms each tile origin in FP64)
                 m64 = self.maps64(angles)
                 check(L.lib().mr_fdk_box_maps(m64.ctypes.data_as(L.P_double), nu, nv, nproj, dtype, ctypes.byref(bw),
                                               ctypes.byref(bh)))
                 maps = torch.from_numpy(m64).to(dev)
             elif uni:
+                # FP32 arithmetic (16-bit rows that TMA cannot address are staged as FP32)
                 check(L.lib().mr_fdk_box(xip.ctypes.data_as(L.P_float), yip.ctypes.data_as(L.P_float),
-                                         zip_.ctypes.data_as(L.P_float), nu, nv, nproj, dtype,
+                                         zip_.ctypes.data_as(L.P_float), nu, nv, nproj, L.MR_F32,
                                          ctypes.byref(bw), ctypes.byref(bh)))
             self._geo = (torch.from_numpy(weights).to(dev), *(torch.from_numpy(a).to(dev) for a in (xip, yip, zip_)),
                          s2, sc, uni, (bw.value, bh.value), maps)
