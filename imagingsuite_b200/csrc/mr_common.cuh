@@ -115,6 +115,10 @@ void keep_pool_memory();
 // allocation-failure hook (mr_debug_fail_allocation) takes this allocation.
 mr_status device_alloc(void **p, size_t bytes, cudaStream_t s, const char *what);
 mr_status device_alloc_sync(void **p, size_t bytes, const char *what);
+// Bytes of scratch a call that could use `want` may take: all of it where the stream-ordered pool already
+// holds that much free (a repeated call), else a quarter of the device's free memory, at least 1 GiB.
+// (Asking the driver for the free memory takes 0.1 to 100 ms and is left out where it can be.)
+size_t scratch_budget(size_t want);
 template <class T>
 inline mr_status device_alloc(T **p, size_t bytes, cudaStream_t s, const char *what)
 {

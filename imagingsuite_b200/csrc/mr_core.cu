@@ -60,6 +60,25 @@ mr_status device_alloc(void **p, size_t bytes, cudaStream_t s, const char *what)
     return MR_OK;
 }
 
+size_t scratch_budget(size_t want)
+{
+    int dev = 0;
+    cudaMemPool_t pool;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+        uint64_t reserved = 0, used = 0;
+        if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved >= used &&
+            reserved - used >= want)
+            return want;
+    }
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        free_b = size_t(1) << 30;
+    }
+    return std::max<size_t>(size_t(1) << 30, free_b / 4);
+}
+
 mr_status device_alloc_sync(void **p, size_t bytes, const char *what)
 {
     *p = nullptr;

@@ -16,8 +16,11 @@
 // marker value (morphgeo.h:213-214); after that scan the reference computes the exact
 // reconstruction of the scanned marker. The scanned marker differs from the initial one
 // only on the border and on pixels with a border pixel among their backward neighbours
-// (every other value stays the marker's interior minimum), so one thread per image replays
-// the scan over that band in raster order, and the exact reconstruction follows.
+// (every other value stays the marker's interior minimum), so the scan
+// is replayed over that band (k_peaks_band_smem), and the exact reconstruction follows.
+//
+// Few images are reconstructed by merging basins over the whole GPU (k_descend and following), many
+// (kFloodUnits) by sweeps and a worklist, one CTA per image:
 //
 // Each reconstruction runs in two kernels, one CTA per image in both. The sweep kernel
 // alternates downward and upward row sweeps for a few rounds (it stops early when a round
@@ -31,6 +34,7 @@
 // changes; the completion kernel finishes from there with a worklist (k_complete).
 #include "mr_common.cuh"
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -57,16 +61,13 @@ namespace msc {
 constexpr int kMargin = 5;
 constexpr int kSweepRounds = 3; // dense sweep rounds before the worklist completion (2-6 measured: 3 is fastest)
 constexpr int kMaxEdge = 63;
-
-struct Clamp {
-    float lo, hi;
-};
-
-// g2 after g1 (apply g1 first).
-__device__ __forceinline__ Clamp compose(const Clamp g1, const Clamp g2)
-{
-    return Clamp{fminf(fmaxf(g1.lo, g2.lo), g2.hi), fminf(fmaxf(g1.hi, g2.lo), g2.hi)};
-}
+// From this many reconstructions on, one CTA each fills the SMs and the sweeps' throughput (34 ps per
+// pixel of a reconstruction) beats the basins' (90 ps); below it a sweep CTA's latency counts, 25 to 50 ns
+// per pixel of one image: 64 images of 1000 x 700 (holes) 17 to 27 against 5 ms, 16 of 1024 x 1024 (both)
+// 34 to 39 against 3.7 ms, 4 of 2000 x 2000 (holes) 76 to 108 against 2.2 ms, 250 of 500 x 300 (both) 8.1
+// to 8.5 against 6.8 to 7.4 ms, but 700 of 1500 x 64 (both) 8 against 14 ms.
+constexpr size_t kFloodUnits = 148 * 4;
+constexpr size_t kBandSmem = 200 * 1024; // shared memory of k_peaks_band_smem
 
 // ---- preparation
 
@@ -87,17 +88,37 @@ __global__ void k_finite_max(const float *__restrict__ img, size_t per, float *_
     }
 }
 
-// Padded image (MorphSpotClean::PadEdges :264-281) after replaceInfNaN (:514-536) and
-// LimitDynamics (core/kipl/kipl/include/segmentation/thresholds.h:60-85).
-__global__ void k_pad(const float *__restrict__ img, int w, int h, const float *__restrict__ finite_max, int clamp,
-                      float lo, float hi, float *__restrict__ pad)
+// Order-preserving integer keys of floats (atomics compare them as ints).
+__device__ __forceinline__ int fkey(float f)
 {
+    const int i = __float_as_int(f);
+    return i >= 0 ? i : i ^ 0x7FFFFFFF;
+}
+
+__device__ __forceinline__ float funkey(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7FFFFFFF); }
+
+// Starting values of the per-image minimum and maximum keys.
+__global__ void k_range_init(int n, int *__restrict__ mn, int *__restrict__ mx)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    mn[i] = fkey(FLT_MAX);
+    mx[i] = fkey(-FLT_MAX);
+}
+
+// Padded image (MorphSpotClean::PadEdges :264-281) after replaceInfNaN (:514-536) and
+// LimitDynamics (core/kipl/kipl/include/segmentation/thresholds.h:60-85), and the image's range as
+// keys (NaN ignored; mn null: not asked for). The edge medians that follow change rows 0 and ph - 1 only, within the range of
+// those rows' samples, which rows 9 and ph - 10 hold too, so the range is theirs as well.
+__global__ void __launch_bounds__(256) k_pad(const float *__restrict__ img, int w, int h, const float *__restrict__ finite_max, int clamp,
+                      float lo, float hi, float *__restrict__ pad, int *__restrict__ mn, int *__restrict__ mx)
+{
+    float a = FLT_MAX, z = -FLT_MAX;
     const int pw = w + 2 * kMargin, ph = h + 2 * kMargin;
     const size_t n = static_cast<size_t>(pw) * ph;
     const int b = blockIdx.y;
     const float *src = img + static_cast<size_t>(b) * w * h;
     float *dst = pad + b * n;
-    (void)n;
     for (int y = blockIdx.x; y < ph; y += gridDim.x) {
         int sy = y - kMargin;
         if (sy < 0) sy = -1 - sy;              // padded row m-1-i <- image row i
@@ -113,7 +134,26 @@ __global__ void k_pad(const float *__restrict__ img, int w, int h, const float *
                 if (clamp) v = v < lo ? lo : (v > hi ? hi : v);
             }
             drow[xp] = v;
+            a = fminf(a, v);
+            z = fmaxf(z, v);
         }
+    }
+    if (!mn) return; // uniform
+    __shared__ int ra[8], rz[8];
+    const int ka = __reduce_min_sync(0xffffffffu, fkey(a)), kz = __reduce_max_sync(0xffffffffu, fkey(z));
+    if ((threadIdx.x & 31) == 0) {
+        ra[threadIdx.x >> 5] = ka;
+        rz[threadIdx.x >> 5] = kz;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int lowest = ra[0], highest = rz[0];
+        for (int k = 1; k < 8; ++k) {
+            lowest = min(lowest, ra[k]);
+            highest = max(highest, rz[k]);
+        }
+        atomicMin(mn + b, lowest);
+        atomicMax(mx + b, highest);
     }
 }
 
@@ -195,48 +235,15 @@ __global__ void k_edge_median(float *__restrict__ pad, int pw, int ph, int edge)
     for (int i = lane; i < pw; i += 32) row[i] = srow[i];
 }
 
-__global__ void k_minmax(const float *__restrict__ pad, size_t n, float *__restrict__ mn, float *__restrict__ mx)
-{
-    const float *p = pad + blockIdx.x * n;
-    float a = FLT_MAX, b = -FLT_MAX;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-        a = fminf(a, p[i]);
-        b = fmaxf(b, p[i]);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
-        b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    __shared__ float sa[32], sb[32];
-    if ((threadIdx.x & 31) == 0) {
-        sa[threadIdx.x >> 5] = a;
-        sb[threadIdx.x >> 5] = b;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const int nw = (blockDim.x + 31) / 32;
-        a = threadIdx.x < nw ? sa[threadIdx.x] : FLT_MAX;
-        b = threadIdx.x < nw ? sb[threadIdx.x] : -FLT_MAX;
-        for (int o = 16; o > 0; o >>= 1) {
-            a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
-            b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
-        }
-        if (threadIdx.x == 0) {
-            mn[blockIdx.x] = a;
-            mx[blockIdx.x] = b;
-        }
-    }
-}
-
 // Marker of FillHole (interior = image maximum) or FillPeaks (interior = minimum), the image
 // on its border (morphextrema.h:268-283, 299-314). sign -1 builds the marker of the negated
 // image (FillHole of -padded in the 'both' mode).
-__global__ void k_marker(const float *__restrict__ pad, int pw, int ph, const float *__restrict__ interior,
+__global__ void k_marker(const float *__restrict__ pad, int pw, int ph, const int *__restrict__ interior,
                          float sign, float *__restrict__ v)
 {
     const size_t n = static_cast<size_t>(pw) * ph;
     const int b = blockIdx.y;
-    const float in = sign * interior[b]; // max(-P) = -min(P) for the negated image
+    const float in = sign * funkey(interior[b]); // max(-P) = -min(P) for the negated image
     for (int y = blockIdx.x; y < ph; y += gridDim.x) {
         const size_t ro = b * n + static_cast<size_t>(y) * pw;
         for (int x = threadIdx.x; x < pw; x += blockDim.x) {
@@ -245,6 +252,19 @@ __global__ void k_marker(const float *__restrict__ pad, int pw, int ph, const fl
         }
     }
 }
+
+// Offset of a pixel in the band of a marker (rows 0, 1, ph - 1 of pw values, then columns 0, 1, pw - 2,
+// pw - 1 of ph values); -1 outside it.
+__device__ __forceinline__ int band_at(int x, int y, int pw, int ph)
+{
+    if (y <= 1) return y * pw + x;
+    if (y == ph - 1) return 2 * pw + x;
+    if (x <= 1) return 3 * pw + x * ph + y;
+    if (x >= pw - 2) return 3 * pw + (x - pw + 4) * ph + y;
+    return -1;
+}
+
+__host__ __device__ inline size_t band_size(int pw, int ph) { return 3 * static_cast<size_t>(pw) + 4 * static_cast<size_t>(ph); }
 
 __device__ __forceinline__ bool is_border(int x, int y, int pw, int ph)
 {
@@ -255,14 +275,14 @@ __device__ __forceinline__ bool is_border(int x, int y, int pw, int ph)
 // change: the border and every pixel with a border pixel among its backward neighbours.
 // One thread per image, raster order. v holds the marker on entry.
 __global__ void k_peaks_forward_band(const float *__restrict__ pad, int pw, int ph, int nimg, int conn8,
-                                     const float *__restrict__ minval, float *__restrict__ v)
+                                     const int *__restrict__ minval, float *__restrict__ v)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nimg) return;
     const size_t n = static_cast<size_t>(pw) * ph;
     const float *g = pad + b * n;
     float *t = v + b * n;
-    const float mnv = minval[b];
+    const float mnv = funkey(minval[b]);
     const int bx[4] = {-1, 0, -1, 1}, by[4] = {0, -1, -1, -1};
     const int nb = conn8 ? 4 : 2;
     auto visit = [&](int x, int y) {
@@ -288,6 +308,604 @@ __global__ void k_peaks_forward_band(const float *__restrict__ pad, int pw, int 
     }
 }
 
+// The same replay for images whose border columns fit in shared memory, one CTA per image. Only the
+// columns and the last row are chains: row 0 keeps the image (its backward neighbours are border pixels,
+// whose marker is the image, and v <= g everywhere); a pixel of row 1 past x = 1 takes marker values of
+// row 0 only (its left neighbour's marker is the minimum it starts from), except the last, which also
+// compares its left neighbour. The two column chains run on two lanes from shared copies, then the last
+// row on one. 64 images of 1010 x 710: 3.14 ms (one thread per image on global memory) -> 0.2 ms.
+__global__ void __launch_bounds__(128) k_peaks_band_smem(const float *__restrict__ pad, int pw, int ph, int conn8,
+                                                         const int *__restrict__ minval, float *__restrict__ out)
+{
+    extern __shared__ float band[];
+    // image columns 0, 1, pw - 2, pw - 1 and their running values; image and running last row
+    float *gc = band, *tc = gc + 4 * ph, *gl = tc + 4 * ph, *tl = gl + pw;
+    const size_t n = static_cast<size_t>(pw) * ph;
+    const float *g = pad + blockIdx.x * n;
+    float *t = out + blockIdx.x * band_size(pw, ph); // rows 0 and 1 first (band_at)
+    const float mnv = funkey(minval[blockIdx.x]);
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 4 * ph; i += 128) {
+        const int y = i >> 2, c = i & 3;
+        const float gv = g[static_cast<size_t>(y) * pw + (c < 2 ? c : pw - 4 + c)];
+        gc[c * ph + y] = gv;
+        tc[c * ph + y] = (c == 0 || c == 3 || y == 0 || y == ph - 1) ? gv : mnv; // the marker
+    }
+    for (int x = tid; x < pw; x += 128) {
+        gl[x] = g[static_cast<size_t>(ph - 1) * pw + x];
+        t[x] = g[x];
+    }
+    // row 1: pixels 2 .. pw - 2 (and pixel 1 of row 1 below, which has a border pixel to its left)
+    for (int x = 2 + tid; x <= pw - 2; x += 128) {
+        const float gv = g[pw + x];
+        float mx = mnv;
+        const float up = g[x], ul = g[x - 1], ur = g[x + 1];
+        if (up > mx) mx = up;
+        if (conn8) {
+            if (ul > mx) mx = ul;
+            if (ur > mx) mx = ur;
+        }
+        const float r = mx < gv ? mx : gv;
+        t[pw + x] = r;
+        if (x == pw - 2) tc[2 * ph + 1] = r;
+    }
+    __syncthreads();
+    // raised by a neighbour with running value tq and marker value mq
+    auto see = [](float &mx, float tq, float mq) {
+        if (tq > mx) mx = mq;
+    };
+    if (tid == 0) {
+        // row 1 of columns 0 and 1, then the rows below: column 2 holds row 1's values at y = 1 and the
+        // marker's minimum below
+        const float t12 = t[pw + 2];
+        for (int y = 1; y < ph - 1; ++y) {
+            const float g0 = gc[y], g0u = gc[y - 1], t0u = tc[y - 1], t1u = tc[ph + y - 1];
+            float mx = g0;
+            see(mx, t0u, g0u);
+            if (conn8) see(mx, t1u, y == 1 ? gc[ph] : mnv);
+            const float r0 = mx < g0 ? mx : g0;
+            tc[y] = r0;
+            const float g1 = gc[ph + y];
+            mx = mnv;
+            see(mx, r0, g0);
+            see(mx, t1u, y == 1 ? gc[ph] : mnv);
+            if (conn8) {
+                see(mx, t0u, g0u);
+                if (y == 1) see(mx, g[2], g[2]);
+                else if (y == 2) see(mx, t12, mnv);
+            }
+            tc[ph + y] = mx < g1 ? mx : g1;
+        }
+    } else if (tid == 32) {
+        const float t1l = t[pw + pw - 3];
+        for (int y = 1; y < ph - 1; ++y) {
+            const float g2u = gc[2 * ph], t2u = tc[2 * ph + y - 1], g3u = gc[3 * ph + y - 1], t3u = tc[3 * ph + y - 1];
+            if (y > 1 && conn8) {
+                const float g2 = gc[2 * ph + y];
+                float mx = mnv; // its left neighbours hold the minimum, except row 1's at y = 2
+                see(mx, t2u, mnv);
+                if (y == 2) see(mx, t1l, mnv);
+                see(mx, t3u, g3u);
+                tc[2 * ph + y] = mx < g2 ? mx : g2;
+            }
+            const float g3 = gc[3 * ph + y];
+            float mx = g3;
+            see(mx, tc[2 * ph + y], mnv);
+            see(mx, t3u, g3u);
+            if (conn8) see(mx, t2u, y == 1 ? g2u : mnv);
+            tc[3 * ph + y] = mx < g3 ? mx : g3;
+        }
+    }
+    __syncthreads();
+    // the last row: above it the columns' values and the minimum elsewhere (row 1's when ph is 3: not
+    // reached, the padding alone is 10 rows)
+    if (tid == 0) {
+        const int y = ph - 2;
+        auto above = [&](int x) { return x <= 1 ? tc[x * ph + y] : x >= pw - 2 ? tc[(x - pw + 4) * ph + y] : mnv; };
+        auto mark = [&](int x) { return x == 0 ? gc[y] : x == pw - 1 ? gc[3 * ph + y] : mnv; };
+        float left = 0.0f;
+        for (int x = 0; x < pw; ++x) {
+            const float gv = gl[x];
+            float mx = gv;
+            if (x > 0) see(mx, left, gl[x - 1]);
+            see(mx, above(x), mark(x));
+            if (conn8) {
+                if (x > 0) see(mx, above(x - 1), mark(x - 1));
+                if (x < pw - 1) see(mx, above(x + 1), mark(x + 1));
+            }
+            left = mx < gv ? mx : gv;
+            tl[x] = left;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < 4 * (ph - 2); i += 128) {
+        const int y = 1 + (i >> 2), c = i & 3;
+        t[band_at(c < 2 ? c : pw - 4 + c, y, pw, ph)] = tc[c * ph + y];
+    }
+    for (int x = tid; x < pw; x += 128) t[2 * pw + x] = tl[x];
+}
+
+// The band out of a whole marker image (k_peaks_forward_band's).
+__global__ void k_band_of(const float *__restrict__ v, int pw, int ph, float *__restrict__ out)
+{
+    const float *t = v + blockIdx.x * (static_cast<size_t>(pw) * ph);
+    float *o = out + blockIdx.x * band_size(pw, ph);
+    for (int x = threadIdx.x; x < pw; x += blockDim.x) {
+        o[x] = t[x];
+        o[pw + x] = t[pw + x];
+        o[2 * pw + x] = t[static_cast<size_t>(ph - 1) * pw + x];
+    }
+    for (int i = threadIdx.x; i < 4 * (ph - 3); i += blockDim.x) {
+        const int y = 2 + (i >> 2), c = i & 3, x = c < 2 ? c : pw - 4 + c;
+        o[band_at(x, y, pw, ph)] = t[static_cast<size_t>(y) * pw + x];
+    }
+}
+
+// The band into a whole marker image.
+__global__ void k_band_into(const float *__restrict__ band, int pw, int ph, float *__restrict__ v)
+{
+    float *t = v + blockIdx.x * (static_cast<size_t>(pw) * ph);
+    const float *b = band + blockIdx.x * band_size(pw, ph);
+    for (int x = threadIdx.x; x < pw; x += blockDim.x) {
+        t[pw + x] = b[pw + x];
+        t[static_cast<size_t>(ph - 1) * pw + x] = b[2 * pw + x];
+    }
+    for (int i = threadIdx.x; i < 4 * (ph - 3); i += blockDim.x) {
+        const int y = 2 + (i >> 2), c = i & 3, x = c < 2 ? c : pw - 4 + c;
+        t[static_cast<size_t>(y) * pw + x] = b[band_at(x, y, pw, ph)];
+    }
+}
+
+// ---- reconstruction by merging basins
+//
+// The erosion-reconstruction of g from a marker m >= g is a minimax path problem: H(p) is the smallest,
+// over the pixels q and the paths from q to p, of the largest of m(q) and g along the path. FillHole's
+// marker is g on the border and the maximum inside, so only the border's m counts: an "ocean" next to
+// every border pixel, entered at height m. FillPeaks (the dilation) is the same on -g, with the marker
+// of the replayed band. With keys (order-preserving integers) for the heights:
+//
+//  1. every pixel points to the smallest of its neighbourhood by (height, index); the chains end in
+//     local minima, which name the basins (k_descend, k_basins). A path from p may first descend to its
+//     basin's bottom, so H(p) = max(g(p), level of the basin), its minimax height to the ocean;
+//  2. Boruvka rounds on the basins: every component of basins not yet joined to the ocean finds its
+//     lowest edge to another component, of height max(g, g) of two neighbouring pixels, or to the ocean
+//     (k_edges), and is merged over it (k_hook, k_join). Any path out of a component crosses an edge at
+//     least that high, so its basins' levels rise to that height; and a component's inner edges were the
+//     lowest out of some part of it, so that the maximum over the rounds is the level exactly. Edges are
+//     ordered by (height, edge index), a strict order, so the only cycles are pairs that chose the same
+//     edge. Every round at least halves the components that are left; basins of noise shrink to a
+//     third.
+//
+// Every value is a maximum or minimum of pixel values: the result is the unique reconstruction, the
+// reference's bit for bit (NaN counts as the lowest height). There are no chains of dependent
+// relaxations along paths: the work is full passes of 8 bytes per pixel while components are smaller
+// than a tile, then only over tiles that still hold a boundary.
+//
+// Measured against row sweeps finished by a worklist, which are bound by the latency of their relaxation
+// chains: see kFloodUnits.
+
+constexpr int kOcean = -1, kNone = -2;
+constexpr int kStripThreads = 256;
+constexpr uint32_t kOceanEdge = 0xFFFFFFFFu;
+constexpr int kRounds = 12;      // rounds as launches over the whole GPU
+constexpr int kMostRounds = 40;  // 2^31 pixels need 31
+
+typedef unsigned long long u64;
+
+// One or two reconstructions of the same images (holes of the image, and of its negation): unit u <
+// nimg is image u with sign[0], unit nimg + i image i with sign[1].
+struct Flood {
+    const int *pad;       // keys (k_to_keys)
+    int flip0, flip1;     // 0, or -1 for the negated image
+    int *lab0, *lab1;     // per pixel: while basins are found, the pixel pointed to or ~basin; then ~basin
+    const float *band;    // peaks: the marker's border band per image (see band_at), else null
+    int *comp, *lev, *par; // per unit and basin: component (a basin, or kOcean), level key, hook target
+    u64 *best0, *best1;   // per unit and basin: a component's lowest edge, in even and odd rounds
+    int *nbasin;          // per unit
+    int *active;          // [round][unit]: components are left
+    unsigned char *uniform; // per unit and strip: nothing to find here any more
+    int nimg, units, pw, ph, cap;
+    // (chosen by selects: an array indexed by the job would be copied to local memory by every thread)
+    __device__ __forceinline__ int flip(int job) const { return job ? flip1 : flip0; }
+    __device__ __forceinline__ int *lab(int job, int img) const
+    {
+        return (job ? lab1 : lab0) + img * (static_cast<size_t>(pw) * ph);
+    }
+    __device__ __forceinline__ u64 *best(int round) const { return round & 1 ? best1 : best0; }
+};
+
+// Height of a pixel: its key, or its negation's (the complement, flip -1); NaN stays the lowest.
+__device__ __forceinline__ int height(int key, int flip)
+{
+    const int h = key ^ flip;
+    return h == INT_MAX ? INT_MIN : h;
+}
+
+// Height at which the ocean enters pixel (x, y) of height gp; INT_MAX: not here.
+__device__ __forceinline__ int ocean_height(const Flood &F, int job, int img, int x, int y, int gp)
+{
+    if (!F.band) return x == 0 || y == 0 || x == F.pw - 1 || y == F.ph - 1 ? gp : INT_MAX;
+    const int at = band_at(x, y, F.pw, F.ph);
+    return at < 0 ? INT_MAX : max(gp, fkey(F.band[img * band_size(F.pw, F.ph) + at]) ^ F.flip(job));
+}
+
+// The passes over pixels give each warp a strip of kStripX columns by kStripY rows: lanes 1 .. 30 are its
+// columns, lanes 0 and 31 the columns beside it, and the warp walks the rows with the last three in
+// registers, neighbours of a row by shuffles. Bound by instruction issue, so that a value is loaded and
+// turned into its height once per strip and there is no tile in shared memory.
+constexpr int kStripX = 30, kStripY = 32, kStripBatch = 4;
+
+struct Strip {
+    int u, job, img, x, y0, y1, lane;
+    bool in, mine; // a column of the image; of this strip
+    size_t flag;   // of Flood::uniform
+};
+
+// The strip of this warp; false past the last one.
+__device__ __forceinline__ bool strip_of(const Flood &F, int u, int task, Strip &S)
+{
+    const int across = (F.pw + kStripX - 1) / kStripX, down = (F.ph + kStripY - 1) / kStripY;
+    if (task >= across * down) return false;
+    const int sy = task / across, sx = task - sy * across;
+    S.u = u;
+    S.job = u >= F.nimg;
+    S.img = u - S.job * F.nimg;
+    S.lane = threadIdx.x & 31;
+    S.x = sx * kStripX + S.lane - 1;
+    S.y0 = sy * kStripY;
+    S.y1 = min(S.y0 + kStripY, F.ph);
+    S.in = S.x >= 0 && S.x < F.pw;
+    S.mine = S.in && S.lane >= 1 && S.lane <= kStripX;
+    S.flag = static_cast<size_t>(u) * (across * down) + task;
+    return true;
+}
+
+// The padded images as keys, in place; NaN, which the reference's comparisons skip, as the lowest (its
+// float is a NaN again).
+__global__ void __launch_bounds__(256) k_to_keys(float *__restrict__ pad, size_t n)
+{
+    int *key = reinterpret_cast<int *>(pad);
+    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        const float v = pad[i];
+        key[i] = v != v ? INT_MIN : fkey(v);
+    }
+}
+
+// Each pixel's lowest neighbour by (height, index), or a basin of its own.
+template <bool CONN8>
+__global__ void __launch_bounds__(kStripThreads) k_descend(const Flood F)
+{
+    Strip S;
+    if (!strip_of(F, blockIdx.y, blockIdx.x * (kStripThreads / 32) + (threadIdx.x >> 5), S)) return;
+    const size_t n = static_cast<size_t>(F.pw) * F.ph;
+    const int *pad = F.pad + S.img * n + (S.in ? S.x : 0);
+    int *lab = F.lab(S.job, S.img);
+    const int flip = F.flip(S.job);
+    // heights of a row, and (8 neighbours) the lowest of three by index
+    struct Row {
+        int c, l, r, low, dx;
+    };
+    auto fetch = [&](int y) { return S.in && y >= 0 && y < F.ph ? height(__ldg(pad + static_cast<size_t>(y) * F.pw), flip) : INT_MAX; };
+    auto row = [&](int h) {
+        Row R;
+        R.c = h;
+        R.l = __shfl_up_sync(0xffffffffu, h, 1);
+        R.r = __shfl_down_sync(0xffffffffu, h, 1);
+        R.low = R.l;
+        R.dx = -1;
+        if (R.c < R.low) R.low = R.c, R.dx = 0;
+        if (R.r < R.low) R.low = R.r, R.dx = 1;
+        return R;
+    };
+    Row up = row(fetch(S.y0 - 1)), at = row(fetch(S.y0));
+    unsigned rows = 0; // lane k: the bottoms of row k
+    for (int yb = S.y0; yb < S.y1; yb += kStripBatch) {
+        int ahead[kStripBatch];
+#pragma unroll
+        for (int k = 0; k < kStripBatch; ++k) ahead[k] = fetch(yb + 1 + k);
+#pragma unroll
+        for (int k = 0; k < kStripBatch; ++k) {
+            const int y = yb + k;
+            if (y >= S.y1) break; // uniform
+            const Row down = row(ahead[k]);
+            int low, dx = 0, dy = -1;
+            if (CONN8) {
+                low = up.low, dx = up.dx;
+                if (at.low < low) low = at.low, dx = at.dx, dy = 0;
+                if (down.low < low) low = down.low, dx = down.dx, dy = 1;
+            } else {
+                low = up.c;
+                if (at.low < low) low = at.low, dx = at.dx, dy = 0;
+                if (down.c < low) low = down.c, dx = 0, dy = 1;
+            }
+            const bool bottom = S.mine && dx == 0 && dy == 0;
+            const unsigned bottoms = __ballot_sync(0xffffffffu, bottom);
+            if (S.lane == y - S.y0) rows = bottoms;
+            const int p = y * F.pw + S.x;
+            if (S.mine && !bottom) lab[p] = p + dy * F.pw + dx;
+            up = at;
+            at = down;
+        }
+    }
+    // the strip's bottoms numbered by one atomic: lane k holds row k's
+    static_assert(kStripY <= 32, "a lane per row");
+    int upto = __popc(rows);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (S.lane >= o) upto += v;
+    }
+    int first = 0;
+    if (S.lane == 31 && upto) first = atomicAdd(F.nbasin + S.u, upto);
+    first = __shfl_sync(0xffffffffu, first, 31) + upto - __popc(rows);
+    for (int k = 0; k < S.y1 - S.y0; ++k) {
+        const unsigned bottoms = __shfl_sync(0xffffffffu, rows, k);
+        const int id = __shfl_sync(0xffffffffu, first, k) + __popc(bottoms & ((1u << S.lane) - 1));
+        if (!(bottoms >> S.lane & 1) || !MR_IN_BOUNDS(id, F.cap, kSiteSpotNbr)) continue;
+        const size_t b = static_cast<size_t>(S.u) * F.cap + id;
+        F.comp[b] = id;
+        F.lev[b] = INT_MIN;
+        F.best0[b] = ~0ull;
+        lab[(S.y0 + k) * F.pw + S.x] = ~id;
+    }
+}
+
+// Every pixel's basin: the chain to its end. Pixels written meanwhile end other chains early.
+__global__ void __launch_bounds__(256) k_basins(const Flood F)
+{
+    const int u = blockIdx.y, job = u >= F.nimg, img = u - job * F.nimg;
+    const int n = F.pw * F.ph;
+    volatile int *lab = F.lab(job, img);
+    constexpr int U = 4; // chains in flight per thread
+    for (int p0 = blockIdx.x * 256 * U + threadIdx.x; p0 < n; p0 += gridDim.x * 256 * U) {
+        int x[U];
+        bool point[U], more = false;
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int p = p0 + k * 256;
+            x[k] = p < n ? lab[p] : -1;
+            point[k] = x[k] >= 0;
+            more |= point[k];
+        }
+        while (more) {
+            more = false;
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                if (x[k] >= 0) x[k] = lab[x[k]];
+                more |= x[k] >= 0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+            if (point[k]) lab[p0 + k * 256] = x[k];
+    }
+}
+
+// Lowest edges of the components in one strip. The lowest height of a pixel's edges is max(g, least g
+// of the neighbours in other components). A pixel that does not beat its component's edge so far ends
+// there. Edges of one height are ordered by their index, 4 * (smaller pixel) + direction (0 right, 1
+// down, 2 down right, 3 down left): up left, up, up right, left, right, down, down right, down left, and
+// the pixel's is the first of these not above its height. A run of kStripBatch rows in which no pixel
+// has an edge is skipped from then on (a bit of `uniform`).
+template <bool CONN8>
+__device__ __forceinline__ void edges_of_strip(const Flood &F, const Strip &S, int round)
+{
+    static_assert(kStripY / kStripBatch <= 8, "a bit per run of rows");
+    unsigned skip = F.uniform[S.flag];
+    if (skip == 0xFF) return; // warp-uniform
+    const size_t n = static_cast<size_t>(F.pw) * F.ph;
+    const int *pad = F.pad + S.img * n + (S.in ? S.x : 0);
+    const int *lab = F.lab(S.job, S.img) + (S.in ? S.x : 0);
+    const int *comp = F.comp + static_cast<size_t>(S.u) * F.cap;
+    u64 *best = F.best(round) + static_cast<size_t>(S.u) * F.cap;
+    const int flip = F.flip(S.job), pw = F.pw, ph = F.ph;
+    const bool shore = S.mine && (F.band ? S.x <= 1 || S.x >= pw - 2 : S.x == 0 || S.x == pw - 1); // a column the ocean touches
+    struct Row {
+        int c, cl, cr, g, gl, gr;
+    };
+    auto row = [&](int c, int g) {
+        Row R;
+        R.c = c;
+        R.g = g;
+        R.cl = __shfl_up_sync(0xffffffffu, c, 1);
+        R.cr = __shfl_down_sync(0xffffffffu, c, 1);
+        R.gl = __shfl_up_sync(0xffffffffu, g, 1);
+        R.gr = __shfl_down_sync(0xffffffffu, g, 1);
+        return R;
+    };
+    // pixels outside the image are higher than any: never the lowest neighbour
+    auto label = [&](int y) { return S.in && y >= 0 && y < ph ? ~lab[static_cast<size_t>(y) * pw] : -1; };
+    auto value = [&](int y) { return S.in && y >= 0 && y < ph ? height(pad[static_cast<size_t>(y) * pw], flip) : INT_MAX; };
+    auto component = [&](int l) { return l >= 0 ? comp[l] : kNone; };
+    Row up{}, at{};
+    bool have = false;
+    for (int yb = S.y0, run = 0; yb < S.y1; yb += kStripBatch, ++run) {
+        if (skip >> run & 1) { // uniform
+            have = false;
+            continue;
+        }
+        int l[kStripBatch], c[kStripBatch], g[kStripBatch];
+        uint32_t limit[kStripBatch]; // height of the component's edge so far, as ordered unsigned
+#pragma unroll
+        for (int k = 0; k < kStripBatch; ++k) {
+            l[k] = label(yb + 1 + k);
+            g[k] = value(yb + 1 + k);
+        }
+        if (!have) {
+            const int lu = label(yb - 1), la = label(yb);
+            const int gu = value(yb - 1), ga = value(yb);
+            up = row(component(lu), gu);
+            at = row(component(la), ga);
+            have = true;
+        }
+#pragma unroll
+        for (int k = 0; k < kStripBatch; ++k) c[k] = component(l[k]);
+#pragma unroll
+        for (int k = 0; k < kStripBatch; ++k) {
+            const int own = k == 0 ? at.c : c[k - 1];
+            limit[k] = S.mine && own >= 0 ? reinterpret_cast<const uint32_t *>(best + own)[1] : 0;
+        }
+        bool differ = false;
+#pragma unroll
+        for (int k = 0; k < kStripBatch; ++k) {
+            const int y = yb + k;
+            if (y >= S.y1) break; // uniform
+            const Row down = row(c[k], g[k]);
+            int least = INT_MAX;
+            auto see = [&](int cq, int gq) { least = min(least, cq != at.c ? gq : INT_MAX); };
+            see(up.c, up.g), see(at.cl, at.gl), see(at.cr, at.gr), see(down.c, down.g);
+            if (CONN8) see(up.cl, up.gl), see(up.cr, up.gr), see(down.cl, down.gl), see(down.cr, down.gr);
+            int sea = INT_MAX;
+            if ((shore || (F.band ? y <= 1 : y == 0) || y == ph - 1) && S.mine && at.c != kOcean)
+                sea = ocean_height(F, S.job, S.img, S.x, y, at.g);
+            const int low = min(max(at.g, least), sea);
+            const bool any = S.mine && min(least, sea) != INT_MAX;
+            differ |= any;
+            if (any && (static_cast<uint32_t>(low) ^ 0x80000000u) <= limit[k]) {
+                const uint32_t p4 = 4u * (static_cast<uint32_t>(y) * pw + S.x), w4 = 4u * pw;
+                uint32_t edge = kOceanEdge;
+                if (max(at.g, least) <= low) {
+                    auto first = [&](int cq, int gq, uint32_t e) { edge = cq != at.c && gq <= low ? e : edge; };
+                    if (CONN8) first(down.cl, down.gl, p4 + 3), first(down.cr, down.gr, p4 + 2);
+                    first(down.c, down.g, p4 + 1), first(at.cr, at.gr, p4), first(at.cl, at.gl, p4 - 4);
+                    if (CONN8) first(up.cr, up.gr, p4 - w4 + 4 + 3);
+                    first(up.c, up.g, p4 - w4 + 1);
+                    if (CONN8) first(up.cl, up.gl, p4 - w4 - 4 + 2);
+                }
+                const u64 e = static_cast<u64>(static_cast<uint32_t>(low) ^ 0x80000000u) << 32 | edge;
+                if (e < __ldcg(best + at.c)) atomicMin(best + at.c, e);
+            }
+            up = at;
+            at = down;
+        }
+        if (!__any_sync(0xffffffffu, differ)) skip |= 1u << run;
+    }
+    if (S.y1 - S.y0 < kStripY) skip |= 0xFFu << (S.y1 - S.y0 + kStripBatch - 1) / kStripBatch; // rows past the image
+    if (S.lane == 0) F.uniform[S.flag] = static_cast<unsigned char>(skip);
+}
+
+template <bool CONN8>
+__global__ void __launch_bounds__(kStripThreads) k_edges(const Flood F, int round)
+{
+    if (round > 0 && !F.active[static_cast<size_t>(round) * F.units + blockIdx.y]) return;
+    Strip S;
+    if (strip_of(F, blockIdx.y, blockIdx.x * (kStripThreads / 32) + (threadIdx.x >> 5), S)) edges_of_strip<CONN8>(F, S, round);
+}
+
+// A component's hook: the component at the other end of its lowest edge; of a pair that chose the same
+// edge the smaller stays.
+__device__ __forceinline__ void hook(const Flood &F, int u, int r, int round)
+{
+    const size_t base = static_cast<size_t>(u) * F.cap;
+    if (F.comp[base + r] != r) return;
+    F.best(round + 1)[base + r] = ~0ull; // the components left are among these
+    const int job = u >= F.nimg, img = u - job * F.nimg;
+    const int *lab = F.lab(job, img);
+    const u64 e = F.best(round)[base + r];
+    const uint32_t edge = static_cast<uint32_t>(e);
+    int to = kOcean;
+    if (edge != kOceanEdge) {
+        const uint32_t p = edge >> 2, dir = edge & 3;
+        const uint32_t q = p + (dir == 0 ? 1 : dir == 1 ? F.pw : dir == 2 ? F.pw + 1 : F.pw - 1);
+        const int cp = F.comp[base + ~lab[p]], cq = F.comp[base + ~lab[q]];
+        to = cp == r ? cq : cp;
+        if (to >= 0 && r < to && F.best(round)[base + to] == e) to = r;
+    }
+    F.par[base + r] = to;
+}
+
+// A basin's new component and level. True when it is a component that is left.
+__device__ __forceinline__ bool join(const Flood &F, int u, int b, int round)
+{
+    const size_t base = static_cast<size_t>(u) * F.cap;
+    const int c = F.comp[base + b];
+    if (c == kOcean) return false;
+    const int h = static_cast<int>(static_cast<uint32_t>(F.best(round)[base + c] >> 32) ^ 0x80000000u);
+    F.lev[base + b] = max(F.lev[base + b], h);
+    int x = F.par[base + c];
+    while (x >= 0) {
+        const int y = F.par[base + x];
+        if (y == x) break;
+        x = y;
+    }
+    F.comp[base + b] = x;
+    return x == b;
+}
+
+__global__ void __launch_bounds__(256) k_hook(const Flood F, int round)
+{
+    const int u = blockIdx.y;
+    if (round > 0 && !F.active[static_cast<size_t>(round) * F.units + u]) return;
+    const int nb = F.nbasin[u];
+    for (int b = blockIdx.x * 256 + threadIdx.x; b < nb; b += gridDim.x * 256) hook(F, u, b, round);
+}
+
+// comp is written here while other threads follow par only.
+__global__ void __launch_bounds__(256) k_join(const Flood F, int round)
+{
+    const int u = blockIdx.y;
+    if (round > 0 && !F.active[static_cast<size_t>(round) * F.units + u]) return;
+    const int nb = F.nbasin[u];
+    bool left = false;
+    for (int b = blockIdx.x * 256 + threadIdx.x; b < nb; b += gridDim.x * 256) left |= join(F, u, b, round);
+    if (__any_sync(0xffffffffu, left) && (threadIdx.x & 31) == 0) F.active[static_cast<size_t>(round + 1) * F.units + u] = 1;
+}
+
+// The rounds that are left (usually none), one CTA per unit.
+template <bool CONN8>
+__global__ void __launch_bounds__(kStripThreads) k_finish(const Flood F, int round)
+{
+    const int u = blockIdx.x, nb = F.nbasin[u];
+    bool left = F.active[static_cast<size_t>(round) * F.units + u] != 0;
+    for (; left && round < kMostRounds; ++round) { // uniform
+        Strip S;
+        for (int task = threadIdx.x >> 5; strip_of(F, u, task, S); task += kStripThreads / 32) edges_of_strip<CONN8>(F, S, round);
+        __syncthreads();
+        for (int b = threadIdx.x; b < nb; b += kStripThreads) hook(F, u, b, round);
+        __syncthreads();
+        bool more = false;
+        for (int b = threadIdx.x; b < nb; b += kStripThreads) more |= join(F, u, b, round);
+        left = __syncthreads_or(more);
+    }
+    if (left && threadIdx.x == 0) atomicExch(&g_msc_error, 2);
+}
+
+// Basins of an image: local minima are not neighbours, so with 8 neighbours at most one pixel of each
+// 2 x 2 block, with 4 every second one.
+inline size_t most_basins(int pw, int ph, int conn8)
+{
+    const size_t hw = (pw + 1) / 2, hh = (ph + 1) / 2;
+    return conn8 ? hw * hh : (static_cast<size_t>(pw) * ph + 1) / 2;
+}
+
+inline size_t strips_of(int pw, int ph) { return div_up(pw, kStripX) * static_cast<size_t>(div_up(ph, kStripY)); }
+
+// Basin levels of the units (lab and lev on return; see Flood).
+template <bool CONN8>
+static mr_status launch_flood(const Flood &F, cudaStream_t s)
+{
+    const size_t n = static_cast<size_t>(F.pw) * F.ph;
+    MR_CUDA_TRY(cudaMemsetAsync(F.nbasin, 0, F.units * sizeof(int), s));
+    MR_CUDA_TRY(cudaMemsetAsync(F.active, 0, (kMostRounds + 1) * static_cast<size_t>(F.units) * sizeof(int), s));
+    MR_CUDA_TRY(cudaMemsetAsync(F.uniform, 0, F.units * strips_of(F.pw, F.ph), s));
+    const dim3 strips(div_up(strips_of(F.pw, F.ph), kStripThreads / 32), F.units);
+    const unsigned per = std::max(1u, 148 * 8 / static_cast<unsigned>(F.units));
+    const dim3 flat(std::min<unsigned>(div_up(n, 1024), std::max(per, 16u)), F.units);
+    const dim3 basins(std::min<unsigned>(div_up(static_cast<size_t>(F.cap), 256), std::max(per, 4u)), F.units);
+    k_descend<CONN8><<<strips, kStripThreads, 0, s>>>(F);
+    k_basins<<<flat, 256, 0, s>>>(F);
+    for (int r = 0; r < kRounds; ++r) {
+        k_edges<CONN8><<<strips, kStripThreads, 0, s>>>(F, r);
+        k_hook<<<basins, 256, 0, s>>>(F, r);
+        k_join<<<basins, 256, 0, s>>>(F, r);
+    }
+    k_finish<CONN8><<<F.units, kStripThreads, 0, s>>>(F, kRounds);
+    return check_launch("morphspotclean reconstruction");
+}
+
+// ---- reconstruction by row sweeps and a worklist (many images; see kFloodUnits)
+
 // One or two reconstructions of the same images in one launch (FillHole of the image and of its
 // negation in the 'both' mode): CTA b < nimg works on image b with sign[0] into vol[0], CTA
 // nimg + b on image b with sign[1] into vol[1]. Independent images share the SMs, so the long
@@ -296,7 +914,7 @@ struct RecJobs {
     float sign[2];
     float *vol[2];
     int nimg;
-    const float *interior[2]; // per-image interior value of the marker, formed by the sweeps; null:
+    const int *interior[2]; // per-image interior value (key) of the marker, formed by the sweeps; null:
                               // the marker is in vol already
 };
 
@@ -344,15 +962,6 @@ __device__ __forceinline__ void clamp_then(float al, float ah, float &bl, float 
     bh = nh;
 }
 
-// Order-preserving integer keys of floats (the completion's atomics compare them as ints).
-__device__ __forceinline__ int fkey(float f)
-{
-    const int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7FFFFFFF;
-}
-
-__device__ __forceinline__ float funkey(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7FFFFFFF); }
-
 // One image per block of RW warps; lane t of the image owns the row chunk [t*C, t*C + C), held
 // in registers across the vertical step and both scans. C odd: the lanes' chunk positions in
 // the shared row buffers fall in distinct banks.
@@ -394,8 +1003,8 @@ __global__ void __launch_bounds__(32 * RW) k_reconstruct(const float *__restrict
     const int c0 = 1 + t * C; // buffer index of the chunk's first element (index 0 is the lead)
     // row y of the mask into G and of the marker into V; from_marker: the initial marker row,
     // formed here (the image on the border, the interior value inside; morphextrema.h:268-283)
-    const float *inter = jobs.interior[job];
-    const float in_val = inter ? sign * inter[img] : 0.0f;
+    const int *inter = jobs.interior[job];
+    const float in_val = inter ? sign * funkey(inter[img]) : 0.0f;
     auto fetch = [&](int y, float *G, float *V, bool from_marker) {
         const size_t ro = static_cast<size_t>(y) * pw;
         const bool brow = y == 0 || y == ph - 1;
@@ -753,8 +1362,9 @@ static mr_status launch_reconstruct(const RecJobs &jobs, int njobs, const float 
 
 // Replacement / blend and unpadding (MorphSpotClean::ProcessReplace :108-175,
 // kipl::math::SigmoidWeights mathfunctions.hpp:92-99).
-__global__ void k_replace(const float *__restrict__ pad, const float *__restrict__ holes, const float *__restrict__ peaks,
-                          int w, int h, int detect, float th0, float th1, float s0, float s1, float *__restrict__ img)
+template <bool LEVELS>
+__global__ void k_replace(const void *__restrict__ pad, const int *__restrict__ hole_lab, const int *__restrict__ hole_lev,
+                          const int *__restrict__ peak_lab, const int *__restrict__ peak_lev, size_t cap, int w, int h, int detect, float th0, float th1, float s0, float s1, float *__restrict__ img)
 {
     const int pw = w + 2 * kMargin, ph = h + 2 * kMargin;
     const size_t n = static_cast<size_t>(pw) * ph;
@@ -764,12 +1374,20 @@ __global__ void k_replace(const float *__restrict__ pad, const float *__restrict
     for (int x = threadIdx.x; x < w; x += blockDim.x) {
         const size_t idx = static_cast<size_t>(y) * w + x;
         const size_t pi = b * n + static_cast<size_t>(y + kMargin) * pw + x + kMargin;
-        const float val = pad[pi];
+        // LEVELS: the image as keys, a reconstruction the larger of the pixel and its basin's level (peaks:
+        // of the negated image); else reconstructions stored as keys (peaks alone: of the image itself)
+        float val, hv = 0.0f, pv = 0.0f;
+        if (LEVELS) {
+            const int key = static_cast<const int *>(pad)[pi];
+            val = funkey(key);
+            if (hole_lab) hv = funkey(max(height(key, 0), hole_lev[b * cap + ~hole_lab[pi]]));
+            if (peak_lab) pv = -funkey(max(height(key, -1), peak_lev[b * cap + ~peak_lab[pi]]));
+        } else {
+            val = static_cast<const float *>(pad)[pi];
+            if (hole_lab) hv = funkey(hole_lab[pi]);
+            if (peak_lab) pv = detect == 2 ? -funkey(peak_lab[pi]) : funkey(peak_lab[pi]);
+        }
         float out = val;
-        // the reconstructions are stored as keys
-        const float hv = holes ? funkey(__float_as_int(holes[pi])) : 0.0f;
-        const float pk = peaks ? funkey(__float_as_int(peaks[pi])) : 0.0f;
-        const float pv = detect == 2 ? -pk : pk;
         if (s0 == 0.0f && s1 == 0.0f) {
             if (detect != 1 && th0 < fabsf(__fsub_rn(val, hv))) out = hv;
             if (detect != 0 && th1 < fabsf(__fsub_rn(pv, val))) out = pv;
@@ -812,49 +1430,96 @@ mr_status mr_morphspotclean(float *proj_d, size_t nu, size_t nv, size_t nproj, i
     if (pw > 128 * 33) return fail(MR_ERR_UNSUPPORTED, "mr_morphspotclean: rows longer than %d pixels", 128 * 33 - 2 * kMargin);
     const size_t n = static_cast<size_t>(pw) * ph;
     cudaStream_t s = as_stream(stream);
-    // images per batch: three padded buffers and two worklists each; up to a quarter of the
-    // free device memory, so that a block of projections is cleaned concurrently (one CTA per
-    // image)
-    const size_t cap = static_cast<size_t>(complete_cap(n));
-    const size_t per_img = 3 * n * sizeof(float) + 4 * cap * sizeof(int); // two worklists per reconstruction
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = size_t(1) << 30;
-    const size_t budget = std::max<size_t>(size_t(1) << 30, free_b / 4);
-    const size_t batch = std::max<size_t>(1, std::min<size_t>(nproj, budget / per_img));
-    float *scratch = nullptr;
-    MR_TRY(device_alloc(&scratch, batch * per_img + 5 * batch * sizeof(float), s, "mr_morphspotclean: scratch"));
-    float *P = scratch, *H = P + batch * n, *K = H + batch * n, *stats = K + batch * n;
-    float *fmax = stats, *mn = stats + batch, *mx = stats + 2 * batch;
-    int *counts = reinterpret_cast<int *>(stats + 3 * batch); // two words per image (the sweeps' list lengths)
-    int *lists = reinterpret_cast<int *>(stats + 5 * batch);
+    // images per batch: the padded image and, per reconstruction, a result or the labels with the basins'
+    // component, level, hook and two edges, or two worklists; up to a quarter of the free device memory
+    const int jobs = detect == 2 ? 2 : 1;
+    const bool flood = nproj * jobs < kFloodUnits && n < size_t(1) << 30;
+    const size_t cap = flood ? most_basins(pw, ph, conn8) : static_cast<size_t>(complete_cap(n));
+    const size_t band = detect == 1 ? band_size(pw, ph) : 0;
+    const size_t per_unit = n * 4 + (flood ? cap * (3 * 4 + 2 * 8) + strips_of(pw, ph) + (kMostRounds + 2) * 4 : 2 * cap * 4 + 4);
+    const size_t per_img = (n + band + 3) * 4 + jobs * per_unit + 64;
+    const size_t most = std::min<size_t>(nproj, size_t(65535) / jobs);
+    const size_t batch = std::max<size_t>(1, std::min<size_t>(most, scratch_budget(most * per_img) / per_img));
+    char *scratch = nullptr;
+    MR_TRY(device_alloc(&scratch, batch * per_img, s, "mr_morphspotclean: scratch"));
+    const size_t units = batch * jobs;
+    Flood F{};
+    F.best0 = reinterpret_cast<u64 *>(scratch); // (flood) 8-byte words first
+    F.best1 = F.best0 + (flood ? units * cap : 0);
+    float *P = reinterpret_cast<float *>(F.best1 + (flood ? units * cap : 0));
+    int *lab = reinterpret_cast<int *>(P + batch * n); // labels, or results as keys
+    F.comp = lab + units * n;
+    F.lev = F.comp + (flood ? units * cap : 0);
+    F.par = F.lev + (flood ? units * cap : 0);
+    float *bands = reinterpret_cast<float *>(F.par + (flood ? units * cap : 0)), *fmax = bands + batch * band;
+    int *mn = reinterpret_cast<int *>(fmax + batch), *mx = mn + batch; // keys
+    F.nbasin = mx + batch;
+    F.active = F.nbasin + units;
+    F.uniform = reinterpret_cast<unsigned char *>(F.active + (kMostRounds + 1) * units);
+    int *counts = mx + batch, *lists = counts + units; // the sweeps' list lengths and worklists
+    F.pad = reinterpret_cast<const int *>(P);
+    F.band = detect == 1 ? bands : nullptr;
+    F.pw = pw;
+    F.ph = ph;
+    F.cap = static_cast<int>(cap);
+    // peaks are holes of the negated image
+    F.flip0 = detect == 1 ? -1 : 0;
+    F.flip1 = -1;
     mr_status st = MR_OK;
     for (size_t b0 = 0; b0 < nproj && st == MR_OK; b0 += batch) {
         const int nb = static_cast<int>(std::min(batch, nproj - b0));
         float *img = proj_d + b0 * nu * nv;
         const unsigned gx = std::min<unsigned>(div_up(n, 256), 128u);
+        F.nimg = nb;
+        F.units = nb * jobs;
+        F.lab0 = lab;
+        F.lab1 = lab + nb * n;
+        int *peak_lab = jobs == 2 ? F.lab1 : F.lab0;
+        float *H = reinterpret_cast<float *>(F.lab0), *K = reinterpret_cast<float *>(peak_lab);
         if (removeinfnan) k_finite_max<<<nb, 256, 0, s>>>(img, nu * nv, fmax);
-        k_pad<<<dim3(gx, nb), 256, 0, s>>>(img, w, h, removeinfnan ? fmax : nullptr, clamp, minlevel, maxlevel, P);
+        const bool range = !flood || detect == 1;
+        if (range) k_range_init<<<div_up(nb, 256), 256, 0, s>>>(nb, mn, mx);
+        k_pad<<<dim3(gx, nb), 256, 0, s>>>(img, w, h, removeinfnan ? fmax : nullptr, clamp, minlevel, maxlevel, P,
+                                           range ? mn : nullptr, mx);
         k_edge_median<<<2 * nb, 32, pw * sizeof(float), s>>>(P, pw, ph, edge);
-        k_minmax<<<nb, 1024, 0, s>>>(P, n, mn, mx);
-        if (detect == 0) { // FillHole: erosion from a max marker (formed by the first sweep)
-            const RecJobs jobs{{1.0f, 1.0f}, {H, H}, nb, {mx, mx}};
-            if ((st = launch_reconstruct<false>(jobs, 1, P, pw, ph, conn8, lists, counts, s)) != MR_OK) break;
+        if (detect == 1) { // the forward scan's border band; the rest of the marker is the minimum
+            const size_t smem = (8 * static_cast<size_t>(ph) + 2 * static_cast<size_t>(pw)) * sizeof(float);
+            const bool fits = smem <= kBandSmem;
+            if (!fits || !flood) k_marker<<<dim3(gx, nb), 256, 0, s>>>(P, pw, ph, mn, 1.0f, K);
+            if (fits) {
+                const cudaError_t e = cudaFuncSetAttribute(k_peaks_band_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                           static_cast<int>(kBandSmem));
+                if (e != cudaSuccess) {
+                    st = fail(MR_ERR_CUDA, "k_peaks_band_smem: %s", cudaGetErrorString(e));
+                    break;
+                }
+                k_peaks_band_smem<<<nb, 128, smem, s>>>(P, pw, ph, conn8, mn, bands);
+                if (!flood) k_band_into<<<nb, 256, 0, s>>>(bands, pw, ph, K);
+            } else { // columns beyond a CTA's shared memory: replayed on the whole marker image
+                k_peaks_forward_band<<<div_up(nb, 32), 32, 0, s>>>(P, pw, ph, nb, conn8, mn, K);
+                if (flood) k_band_of<<<nb, 256, 0, s>>>(K, pw, ph, bands);
+            }
         }
-        if (detect == 1) { // FillPeaks: forward-scan band replay, then the exact dilation
-            k_marker<<<dim3(gx, nb), 256, 0, s>>>(P, pw, ph, mn, 1.0f, K);
-            k_peaks_forward_band<<<div_up(nb, 32), 32, 0, s>>>(P, pw, ph, nb, conn8, mn, K);
-            const RecJobs jobs{{1.0f, 1.0f}, {K, K}, nb, {nullptr, nullptr}};
-            if ((st = launch_reconstruct<true>(jobs, 1, P, pw, ph, conn8, lists, counts, s)) != MR_OK) break;
+        if (flood) {
+            k_to_keys<<<std::min<unsigned>(div_up(nb * n, 1024), 148 * 16), 256, 0, s>>>(P, nb * n);
+            st = conn8 ? launch_flood<true>(F, s) : launch_flood<false>(F, s);
+        } else if (detect == 1) {
+            const RecJobs rec{{1.0f, 1.0f}, {K, K}, nb, {nullptr, nullptr}};
+            st = launch_reconstruct<true>(rec, 1, P, pw, ph, conn8, lists, counts, s);
+        } else {
+            // FillHole: erosion from a max marker (formed by the first sweep); of the negated image too
+            // for 'both' (marker max(-P) = -min(P)), in the same launches
+            const RecJobs rec{{1.0f, -1.0f}, {H, K}, nb, {mx, mn}};
+            st = launch_reconstruct<false>(rec, jobs, P, pw, ph, conn8, lists, counts, s);
         }
-        if (detect == 2) {
-            // FillHole of the image, and -FillHole(-padded): erosion of the negated image from
-            // marker max(-P) = -min(P); both erosions in the same launches
-            const RecJobs jobs{{1.0f, -1.0f}, {H, K}, nb, {mx, mn}};
-            if ((st = launch_reconstruct<false>(jobs, 2, P, pw, ph, conn8, lists, counts, s)) != MR_OK) break;
-        }
-        if ((st = check_launch("morphspotclean reconstruction")) != MR_OK) break;
-        k_replace<<<dim3(gx, nb), 256, 0, s>>>(P, detect != 1 ? H : nullptr, detect != 0 ? K : nullptr, w, h, detect,
-                                               th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
+        if (st != MR_OK) break;
+        const int *hole_lab = detect != 1 ? F.lab0 : nullptr, *peaks = detect != 0 ? peak_lab : nullptr;
+        if (flood)
+            k_replace<true><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, F.lev, peaks, F.lev + (jobs - 1) * nb * cap, cap, w, h,
+                                                         detect, th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
+        else
+            k_replace<false><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, nullptr, peaks, nullptr, 0, w, h, detect, th_h[0],
+                                                          th_h[1], sigma_h[0], sigma_h[1], img);
         st = check_launch("k_replace");
     }
     cudaFreeAsync(scratch, s);
