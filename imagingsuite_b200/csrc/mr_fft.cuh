@@ -10,7 +10,9 @@
 // reverse order (conjugate twiddle, inverse R-point DFT), so it takes the digit-reversed
 // spectrum and returns the natural-order, unnormalised inverse transform. A real frequency
 // response is applied at the digit-reversed positions (fft_permute_response on the host).
-// Twiddles: exp(-2 pi i k / n), k < n (fft_twiddles on the host).
+// Twiddles: per stage, W_N^(j m) at [m - 1][j] (fft_twiddles on the host), so that the lanes of a warp, which
+// hold consecutive j, read consecutive words. (From one table of exp(-2 pi i k / n) they read words j m N / n
+// apart, up to 32 lines a load: 103 of 143 million LSU wavefronts of a 2^12-point filter, 88 % of the peak.)
 //
 // Element e of a sequence sits at fft_slot(e) = e + e/16 of the shared buffer (one float2 of
 // padding after every 16): the strided stages would otherwise put up to 16 lanes of a warp on
@@ -91,7 +93,7 @@ __device__ __forceinline__ void fft_dif_stage(float2 *buf, int logn, int nsl, co
     constexpr int R = 1 << RL;
     const int qsl = nsl - RL;               // log2 of the input stride N/R
     const int nb = 1 << (logn - RL);        // butterflies
-    const int tws = logn - nsl;             // W_N^e = tw[e << tws]
+    tw += (1 << logn) - (1 << nsl);         // this stage's
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
         const int j = b & ((1 << qsl) - 1);
         const int base = ((b >> qsl) << nsl) + j;
@@ -101,7 +103,7 @@ __device__ __forceinline__ void fft_dif_stage(float2 *buf, int logn, int nsl, co
         dft_small<R>(x);
         buf[fft_slot(base)] = x[0];
 #pragma unroll
-        for (int m = 1; m < R; ++m) buf[fft_slot(base + (m << qsl))] = cmul(x[m], __ldg(tw + ((j * m) << tws)));
+        for (int m = 1; m < R; ++m) buf[fft_slot(base + (m << qsl))] = cmul(x[m], __ldg(tw + ((m - 1) << qsl) + j));
     }
 }
 
@@ -112,14 +114,14 @@ __device__ __forceinline__ void fft_inv_stage(float2 *buf, int logn, int nsl, co
     constexpr int R = 1 << RL;
     const int qsl = nsl - RL;
     const int nb = 1 << (logn - RL);
-    const int tws = logn - nsl;
+    tw += (1 << logn) - (1 << nsl);
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
         const int j = b & ((1 << qsl) - 1);
         const int base = ((b >> qsl) << nsl) + j;
         float2 x[R];
         x[0] = conj2(buf[fft_slot(base)]);
 #pragma unroll
-        for (int m = 1; m < R; ++m) x[m] = conj2(cmulc(buf[fft_slot(base + (m << qsl))], __ldg(tw + ((j * m) << tws))));
+        for (int m = 1; m < R; ++m) x[m] = conj2(cmulc(buf[fft_slot(base + (m << qsl))], __ldg(tw + ((m - 1) << qsl) + j)));
         dft_small<R>(x); // inverse DFT = conj(DFT(conj(.)))
 #pragma unroll
         for (int q = 0; q < R; ++q) buf[fft_slot(base + (q << qsl))] = conj2(x[q]);
@@ -169,13 +171,21 @@ __device__ __forceinline__ void fft_apply_response(float2 *buf, int n, const flo
 
 // ---- host side
 
-// exp(-2 pi i k / n), k < n, in double then rounded
+// The stages' twiddles in double then rounded: the stage on sub-transforms of length N = 2^nsl holds
+// exp(-2 pi i j m / N), j < N / R, 1 <= m < R, at n - N + (m - 1) N / R + j.
 inline std::vector<float2> fft_twiddles(int n)
 {
+    int logn = 0, rl[kFftMaxStages];
+    while ((1 << logn) < n) ++logn;
     std::vector<float2> t(n);
-    for (int k = 0; k < n; ++k) {
-        const double ang = -2.0 * 3.14159265358979323846264338327950288 * static_cast<double>(k) / n;
-        t[k] = make_float2(static_cast<float>(std::cos(ang)), static_cast<float>(std::sin(ang)));
+    for (int s = 0, ns = fft_stages(logn, rl), nsl = logn; s < ns; nsl -= rl[s++]) {
+        const int len = 1 << nsl, q = len >> rl[s];
+        for (int m = 1; m < 1 << rl[s]; ++m)
+            for (int j = 0; j < q; ++j) {
+                // (the fraction of a turn with the whole transform's denominator)
+                const double ang = -2.0 * 3.14159265358979323846264338327950288 * static_cast<double>(j * m * (n / len)) / n;
+                t[n - len + (m - 1) * q + j] = make_float2(static_cast<float>(std::cos(ang)), static_cast<float>(std::sin(ang)));
+            }
     }
     return t;
 }

@@ -13,11 +13,11 @@
 // rows are filtered together as the real and imaginary parts of one complex row (one
 // forward and one inverse complex FFT per two rows, no real-FFT pre/post twiddles).
 //
-// Kernel: one CTA per pair of rows. The padded complex row is built in shared memory in
-// bit-reversed order, transformed with in-place radix-2 decimation-in-time stages,
-// multiplied by H, transformed back with decimation-in-frequency stages (natural in,
-// bit-reversed out) and the crop window is gathered out. Twiddles are a float2 table
-// exp(-2 pi i k / N), k < N/2, built in double on the host.
+// Kernels: one CTA per pair of rows. The padded complex row is transformed with mixed-radix
+// decimation-in-frequency stages (natural in, digit-reversed out), multiplied by H in that order and
+// transformed back with the mirrored stages; the crop window is written from the natural order. Lengths
+// 2^8 .. 2^13 have a kernel of their own (k_rowfilter_t), which keeps the first and last stages' values in
+// registers. Twiddles per stage, built in double on the host (mr_fft.cuh).
 #include "mr_common.cuh"
 #include "mr_fft.cuh"
 
@@ -38,9 +38,7 @@ enum PadMode { kPadProjFilter = 0, kPadFdk = 1, kPadProjCore = 2 };
 
 struct RowFilterArgs {
     const float *in;
-    float *out;           // f32 output (or NULL when out16 is used)
-    uint16_t *out16;      // 16-bit output (bf16/f16 bits), NULL for f32
-    const float *out_scale_inv; // per-projection 1/scale for 16-bit output
+    float *out;
     const float2 *twiddle;
     const float *response; // full-length real response H[k], k < n
     const float *pad;      // projection filter taper (ninsert values)
@@ -56,13 +54,13 @@ struct RowFilterArgs {
     int logn;
     int ninsert;     // projection filter: data offset; FDK: pad_factor/2
     int mode;
-    int out16_kind;  // MR_BF16 / MR_F16
     float scale;     // projection filter: pi/(4*N/2); FDK: 1/padwidth
     float post1, post2; // FDK: sad_sid_2, scale (two sequential products); 1 for the projection filter
+    float *amax;        // largest |output| per projection (nv rows), zeroed by the caller; null: not asked for
 };
 
-// Value of padded position p (0 <= p < n) of one row, reference padding rules.
-__device__ __forceinline__ float padded_value(const RowFilterArgs &a, const float *row, size_t rowidx, int p)
+// Value of padded position p (0 <= p < n) of one row of weight `weight`, reference padding rules.
+__device__ __forceinline__ float padded_value(const RowFilterArgs &a, const float *row, float weight, int p)
 {
     if (a.mode == kPadProjCore) return p < a.nu ? row[p] : 0.0f; // the row alone, zero-padded
     if (a.mode == kPadProjFilter) {
@@ -84,9 +82,7 @@ __device__ __forceinline__ float padded_value(const RowFilterArgs &a, const floa
         if (c >= a.n - 5) c = a.n - 6;
         const int q = c - a.ninsert;
         if (q < 0 || q >= a.nu) return 0.0f;
-        float v = row[q];
-        if (a.row_weight) v = __fmul_rn(v, a.row_weight[rowidx / a.rows_per_weight]); // img *= weight
-        return v;
+        return a.row_weight ? __fmul_rn(row[q], weight) : row[q]; // img *= weight
     }
 }
 
@@ -107,68 +103,159 @@ __device__ __forceinline__ size_t fdk_source_row(size_t r, int nv, int row0, int
     return proj * nv + (v - row0);
 }
 
+// The rows of a CTA (2m, 2m + 1) and the terms of their epilogue.
+struct RowPair {
+    size_t r0, r1;
+    bool has1;
+    const float *row0, *row1;
+    float l0, e0, l1, e1; // kPadProjCore: first and last samples, which the tapers repeat
+    float w0, w1;         // the rows' weights
+    __device__ __forceinline__ explicit RowPair(const RowFilterArgs &a)
+    {
+        r0 = 2 * static_cast<size_t>(blockIdx.x);
+        r1 = r0 + 1;
+        has1 = r1 < a.nrows;
+        const size_t src0 = a.mode == kPadFdk ? fdk_source_row(r0, a.nv, a.row0, a.nvfull) : r0;
+        const size_t src1 = a.mode == kPadFdk ? fdk_source_row(r1, a.nv, a.row0, a.nvfull) : r1;
+        row0 = a.in + src0 * a.nu;
+        row1 = a.in + src1 * a.nu;
+        w0 = a.row_weight ? a.row_weight[r0 / a.rows_per_weight] : 1.0f;
+        w1 = a.row_weight && has1 ? a.row_weight[r1 / a.rows_per_weight] : 1.0f;
+        const bool core = a.mode == kPadProjCore;
+        l0 = core ? row0[0] : 0.0f;
+        e0 = core ? row0[a.nu - 1] : 0.0f;
+        l1 = core && has1 ? row1[0] : 0.0f;
+        e1 = core && has1 ? row1[a.nu - 1] : 0.0f;
+    }
+    // padded complex sample (two real rows as re/im) at position p
+    __device__ __forceinline__ float2 sample(const RowFilterArgs &a, int p) const
+    {
+        return make_float2(padded_value(a, row0, w0, p), has1 ? padded_value(a, row1, w1, p) : 0.0f);
+    }
+    // output column i from its transform value; m0, m1 collect |output|
+    __device__ __forceinline__ void write(const RowFilterArgs &a, int i, float2 v, float &m0, float &m1) const
+    {
+        if (a.mode == kPadProjCore) {
+            // the row's part plus the tapers' (scaled by the edge samples they repeat)
+            const float tl = a.tl[i], tr = a.tr[i];
+            v.x = __fadd_rn(__fadd_rn(v.x, __fmul_rn(l0, tl)), __fmul_rn(e0, tr));
+            v.y = __fadd_rn(__fadd_rn(v.y, __fmul_rn(l1, tl)), __fmul_rn(e1, tr));
+        }
+        float y0 = __fmul_rn(v.x, a.scale);
+        float y1 = __fmul_rn(v.y, a.scale);
+        if (a.mode != kPadFdk) {
+            if (a.row_weight) {
+                y0 = __fmul_rn(y0, w0);
+                y1 = __fmul_rn(y1, w1);
+            }
+        } else {
+            y0 = __fmul_rn(__fmul_rn(y0, a.post1), a.post2);
+            y1 = __fmul_rn(__fmul_rn(y1, a.post1), a.post2);
+        }
+        a.out[r0 * a.nu + i] = y0;
+        if (has1) a.out[r1 * a.nu + i] = y1;
+        m0 = fmaxf(m0, fabsf(y0));
+        m1 = fmaxf(m1, fabsf(y1));
+    }
+    // largest |output| of each row into its projection's
+    __device__ __forceinline__ void put_max(const RowFilterArgs &a, float m0, float m1) const
+    {
+        if (!a.amax) return;
+        const int k0 = __reduce_max_sync(__activemask(), __float_as_int(m0)), k1 = __reduce_max_sync(__activemask(), __float_as_int(m1));
+        if ((threadIdx.x & 31) != 0) return;
+        atomicMax(reinterpret_cast<int *>(a.amax + r0 / a.nv), k0);
+        if (has1) atomicMax(reinterpret_cast<int *>(a.amax + r1 / a.nv), k1);
+    }
+};
+
+// Transforms of any length.
 __global__ void __launch_bounds__(512) k_rowfilter(RowFilterArgs a)
 {
     extern __shared__ float2 buf[];
-    const size_t r0 = 2 * static_cast<size_t>(blockIdx.x);
-    const size_t r1 = r0 + 1;
-    const bool has1 = r1 < a.nrows;
     const int n = a.n;
-    const size_t src0 = a.mode == kPadFdk ? fdk_source_row(r0, a.nv, a.row0, a.nvfull) : r0;
-    const size_t src1 = a.mode == kPadFdk ? fdk_source_row(r1, a.nv, a.row0, a.nvfull) : r1;
-    const float *row0 = a.in + src0 * a.nu;
-    const float *row1 = a.in + src1 * a.nu;
-
-    // padded complex row (two real rows as re/im), natural order
-    for (int p = threadIdx.x; p < n; p += blockDim.x) {
-        float x0 = padded_value(a, row0, r0, p);
-        float x1 = has1 ? padded_value(a, row1, r1, p) : 0.0f;
-        buf[fft_slot(p)] = make_float2(x0, x1);
-    }
+    const RowPair R(a);
+    for (int p = threadIdx.x; p < n; p += blockDim.x) buf[fft_slot(p)] = R.sample(a, p); // natural order
     __syncthreads();
 
     fft_forward(buf, a.logn, a.twiddle);
     fft_apply_response(buf, n, a.response);
     fft_inverse(buf, a.logn, a.twiddle);
 
-    // crop and write
-    const float l0 = a.mode == kPadProjCore ? row0[0] : 0.0f, r0v = a.mode == kPadProjCore ? row0[a.nu - 1] : 0.0f;
-    const float l1 = a.mode == kPadProjCore && has1 ? row1[0] : 0.0f;
-    const float r1v = a.mode == kPadProjCore && has1 ? row1[a.nu - 1] : 0.0f;
-    for (int i = threadIdx.x; i < a.nu; i += blockDim.x) {
-        float2 v = buf[fft_slot(i + (a.mode == kPadProjCore ? 0 : a.ninsert))];
-        if (a.mode == kPadProjCore) {
-            // the row's part plus the tapers' (scaled by the edge samples they repeat)
-            const float tl = a.tl[i], tr = a.tr[i];
-            v.x = __fadd_rn(__fadd_rn(v.x, __fmul_rn(l0, tl)), __fmul_rn(r0v, tr));
-            v.y = __fadd_rn(__fadd_rn(v.y, __fmul_rn(l1, tl)), __fmul_rn(r1v, tr));
-        }
-        float y0 = __fmul_rn(v.x, a.scale);
-        float y1 = __fmul_rn(v.y, a.scale);
-        if (a.mode != kPadFdk) {
-            if (a.row_weight) {
-                y0 = __fmul_rn(y0, a.row_weight[r0 / a.rows_per_weight]);
-                if (has1) y1 = __fmul_rn(y1, a.row_weight[r1 / a.rows_per_weight]);
-            }
-        } else {
-            y0 = __fmul_rn(__fmul_rn(y0, a.post1), a.post2);
-            y1 = __fmul_rn(__fmul_rn(y1, a.post1), a.post2);
-        }
-        if (a.out16) {
-            const float s0 = a.out_scale_inv[r0 / a.nv];
-            const float s1 = has1 ? a.out_scale_inv[r1 / a.nv] : 0.0f;
-            if (a.out16_kind == MR_BF16) {
-                a.out16[r0 * a.nu + i] = __bfloat16_as_ushort(__float2bfloat16_rn(y0 * s0));
-                if (has1) a.out16[r1 * a.nu + i] = __bfloat16_as_ushort(__float2bfloat16_rn(y1 * s1));
-            } else {
-                a.out16[r0 * a.nu + i] = __half_as_ushort(__float2half_rn(y0 * s0));
-                if (has1) a.out16[r1 * a.nu + i] = __half_as_ushort(__float2half_rn(y1 * s1));
-            }
-        } else {
-            a.out[r0 * a.nu + i] = y0;
-            if (has1) a.out[r1 * a.nu + i] = y1;
-        }
+    float m0 = 0.0f, m1 = 0.0f;
+    for (int i = threadIdx.x; i < a.nu; i += blockDim.x)
+        R.write(a, i, buf[fft_slot(i + (a.mode == kPadProjCore ? 0 : a.ninsert))], m0, m1);
+    __syncwarp();
+    R.put_max(a, m0, m1);
+}
+
+// Lengths 2^8 .. 2^13: one radix-8 butterfly per thread and stage, the length a constant. The first stage
+// takes its samples from global memory, the last forward stage, the response and the first inverse stage
+// share a butterfly's registers, and the last inverse stage writes the columns: 6 passes over shared memory
+// instead of 10 and 6 barriers instead of 10, the same operations on every value. Bound by the LSU (shared
+// memory, twiddles) and the barriers. 9600 pairs of 2048-column rows (2^12 points): 702 -> 558 us, 316 with
+// the stages' twiddles in order (mr_fft.cuh); 25600 pairs of 512 columns (FDK): 370 -> 242 us.
+template <int LOGN>
+__global__ void __launch_bounds__(1 << (LOGN - 3), (1 << (LOGN - 3)) >= 1024 ? 1 : 1024 >> (LOGN - 3)) k_rowfilter_t(RowFilterArgs a)
+{
+    extern __shared__ float2 buf[];
+    constexpr int Q = LOGN - 3;                       // log2 of the first stage's stride
+    constexpr int RL = LOGN % 3 == 0 ? 3 : LOGN % 3;  // log2 of the last stage's radix
+    constexpr int RR = 1 << RL, PER = 8 / RR;         // last-stage butterflies per thread
+    constexpr int MID = (LOGN - RL) / 3 - 1;          // radix-8 stages between the first and the last
+    const RowPair R(a);
+    const int j = threadIdx.x;
+    const float2 *__restrict__ tw = a.twiddle;
+    {
+        float2 x[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = R.sample(a, j + (q << Q));
+        dft_small<8>(x);
+        buf[fft_slot(j)] = x[0];
+#pragma unroll
+        for (int m = 1; m < 8; ++m) buf[fft_slot(j + (m << Q))] = cmul(x[m], __ldg(tw + ((m - 1) << Q) + j));
     }
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < MID; ++s) {
+        fft_dif_stage<3>(buf, LOGN, LOGN - 3 - 3 * s, tw);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int base = (j + (k << Q)) << RL;
+        float2 x[RR];
+#pragma unroll
+        for (int m = 0; m < RR; ++m) x[m] = buf[fft_slot(base + m)];
+        dft_small<RR>(x);
+#pragma unroll
+        for (int m = 0; m < RR; ++m) {
+            const float r = __ldg(a.response + base + m); // (products rounded, as when they were stored)
+            x[m] = conj2(make_float2(__fmul_rn(x[m].x, r), __fmul_rn(x[m].y, r)));
+        }
+        dft_small<RR>(x); // inverse DFT = conj(DFT(conj(.)))
+#pragma unroll
+        for (int m = 0; m < RR; ++m) buf[fft_slot(base + m)] = conj2(x[m]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int s = MID - 1; s >= 0; --s) {
+        fft_inv_stage<3>(buf, LOGN, LOGN - 3 - 3 * s, tw);
+        __syncthreads();
+    }
+    float2 x[8];
+    x[0] = conj2(buf[fft_slot(j)]);
+#pragma unroll
+    for (int m = 1; m < 8; ++m) x[m] = conj2(cmulc(buf[fft_slot(j + (m << Q))], __ldg(tw + ((m - 1) << Q) + j)));
+    dft_small<8>(x);
+    float m0 = 0.0f, m1 = 0.0f;
+    const int first = a.mode == kPadProjCore ? 0 : a.ninsert;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int i = j + (q << Q) - first;
+        if (i >= 0 && i < a.nu) R.write(a, i, conj2(x[q]), m0, m1);
+    }
+    __syncwarp();
+    R.put_max(a, m0, m1);
 }
 
 static size_t next_pow2_size(size_t n)
@@ -189,16 +276,24 @@ mr_status launch_rowfilter(RowFilterArgs a, cudaStream_t s)
 {
     if (a.nrows == 0) return MR_OK;
     const size_t smem = static_cast<size_t>(fft_buffer_slots(a.n)) * sizeof(float2);
-    static bool attr_set = false;
-    if (!attr_set) {
-        MR_CUDA_TRY(cudaFuncSetAttribute(k_rowfilter, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        attr_set = true;
-    }
-    const unsigned threads = static_cast<unsigned>(std::min(512, std::max(64, a.n / 8))); // one radix-8 butterfly each
     const size_t blocks = (a.nrows + 1) / 2;
     if (blocks > 0x7fffffffu) return fail(MR_ERR_ARGUMENT, "row filter: too many rows in one call");
-    k_rowfilter<<<static_cast<unsigned>(blocks), threads, smem, s>>>(a);
-    return check_launch("k_rowfilter");
+    auto launch = [&](auto kernel, unsigned threads) -> mr_status {
+        if (smem > 48 * 1024)
+            MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kernel<<<static_cast<unsigned>(blocks), threads, smem, s>>>(a);
+        return check_launch("k_rowfilter");
+    };
+    switch (a.logn) {
+    case 8: return launch(k_rowfilter_t<8>, 32);
+    case 9: return launch(k_rowfilter_t<9>, 64);
+    case 10: return launch(k_rowfilter_t<10>, 128);
+    case 11: return launch(k_rowfilter_t<11>, 256);
+    case 12: return launch(k_rowfilter_t<12>, 512);
+    case 13: return launch(k_rowfilter_t<13>, 1024);
+    // shorter ones leave less than a warp with one butterfly each, 2^14 needs two per thread
+    default: return launch(k_rowfilter, static_cast<unsigned>(std::min(512, std::max(64, a.n / 8))));
+    }
 }
 
 // Per-projection power-of-two scale for 16-bit storage: the largest |value| maps below
@@ -240,16 +335,17 @@ __global__ void k_quantize(const float *__restrict__ x, size_t per, size_t total
     }
 }
 
-// Quantize nproj projections of `per` floats to 16 bits with per-projection scales.
+// Quantize nproj projections of `per` floats to 16 bits with per-projection scales. scratch: 2 * nproj
+// floats; `measured`: its first nproj hold the projections' largest |value| already.
 mr_status quantize_projections(const float *x_d, size_t per, size_t nproj, int kind, uint16_t *out_d, float *scale_d,
-                               cudaStream_t s)
+                               float *scratch, bool measured, cudaStream_t s)
 {
-    float *amax = nullptr, *inv = nullptr;
-    MR_TRY(device_alloc(&amax, 2 * nproj * sizeof(float), s, "16-bit quantisation: scratch"));
-    inv = amax + nproj;
+    float *amax = scratch, *inv = amax + nproj;
     mr_status st = MR_OK;
-    if (cudaMemsetAsync(amax, 0, nproj * sizeof(float), s) != cudaSuccess) st = fail(MR_ERR_CUDA, "memset");
-    if (st == MR_OK) {
+    if (!measured) {
+        if (cudaMemsetAsync(amax, 0, nproj * sizeof(float), s) != cudaSuccess) st = fail(MR_ERR_CUDA, "memset");
+    }
+    if (st == MR_OK && !measured) {
         dim3 g(std::min<unsigned>(div_up(per, 256), 64u), static_cast<unsigned>(nproj));
         k_absmax<<<g, 256, 0, s>>>(x_d, per, amax);
         st = check_launch("k_absmax");
@@ -267,7 +363,6 @@ mr_status quantize_projections(const float *x_d, size_t per, size_t nproj, int k
             k_quantize<MR_F16><<<blocks, 256, 0, s>>>(x_d, per, total, inv, out_d);
         st = check_launch("k_quantize");
     }
-    cudaFreeAsync(amax, s);
     return st;
 }
 
@@ -534,7 +629,11 @@ mr_status mr_quantize(const float *in_d, size_t per, size_t nproj, int dtype, ui
     if (dtype != MR_BF16 && dtype != MR_F16) return fail(MR_ERR_ARGUMENT, "mr_quantize: dtype must be bf16 or f16");
     if (nproj > 65535) return fail(MR_ERR_ARGUMENT, "mr_quantize: more than 65535 projections per call");
     if (per == 0 || nproj == 0) return MR_OK;
-    return quantize_projections(in_d, per, nproj, dtype, out_d, scale_d, as_stream(stream));
+    float *scratch = nullptr;
+    MR_TRY(device_alloc(&scratch, 2 * nproj * sizeof(float), as_stream(stream), "16-bit quantisation: scratch"));
+    const mr_status st = quantize_projections(in_d, per, nproj, dtype, out_d, scale_d, scratch, false, as_stream(stream));
+    cudaFreeAsync(scratch, as_stream(stream));
+    return st;
 }
 
 mr_status mr_quantize_noalloc(const float *in_d, size_t per, size_t nproj, int dtype, uint16_t *out_d, float *scale_d,
@@ -623,7 +722,10 @@ mr_status mr_fdk_filter_rows(const float *in_d, size_t nu, size_t nrows, size_t 
     const size_t total = nu * nv * nproj;
     st = device_alloc(&tw_d, tw.size() * sizeof(float2), s, "mr_fdk_filter: twiddles");
     if (st == MR_OK) st = device_alloc(&resp_d, padwidth * sizeof(float), s, "mr_fdk_filter: response");
-    if (st == MR_OK && out_dtype != MR_F32) st = device_alloc(&tmp, total * sizeof(float), s, "mr_fdk_filter: f32 staging buffer");
+    // 16-bit output: the f32 rows, then the projections' largest |value| (collected by the filter) and scales
+    if (st == MR_OK && out_dtype != MR_F32)
+        st = device_alloc(&tmp, (total + 2 * nproj) * sizeof(float), s, "mr_fdk_filter: f32 staging buffer");
+    if (tmp && cudaMemsetAsync(tmp + total, 0, nproj * sizeof(float), s) != cudaSuccess) st = fail(MR_ERR_CUDA, "memset");
     if (st == MR_OK) {
         if (cudaMemcpyAsync(tw_d, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, s) != cudaSuccess ||
             cudaMemcpyAsync(resp_d, ramp.data(), padwidth * sizeof(float), cudaMemcpyHostToDevice, s) != cudaSuccess)
@@ -649,10 +751,11 @@ mr_status mr_fdk_filter_rows(const float *in_d, size_t nu, size_t nrows, size_t 
         a.scale = 1.0f / padwidth;
         a.post1 = sad_sid_2;
         a.post2 = scale;
+        a.amax = tmp ? tmp + total : nullptr;
         st = launch_rowfilter(a, s);
     }
     if (st == MR_OK && out_dtype != MR_F32)
-        st = quantize_projections(tmp, nu * nv, nproj, out_dtype, static_cast<uint16_t *>(out_d), scale_out_d, s);
+        st = quantize_projections(tmp, nu * nv, nproj, out_dtype, static_cast<uint16_t *>(out_d), scale_out_d, tmp + total, true, s);
     // pageable-host uploads above are synchronous with respect to the host buffers, so the
     // vectors may go out of scope; device tables are released in stream order
     if (tw_d) cudaFreeAsync(tw_d, s);
