@@ -66,6 +66,7 @@ int bounds_take_ring(unsigned long long *w);    // mr_ringclean.cu
 int bounds_take_spot(unsigned long long *w);    // mr_spotclean.cu
 MR_BOUNDS_TAKE(bounds_take_fdk)
 int msc_device_status_take(); // mr_spotclean.cu
+int mbp_device_status_take(); // mr_matched.cu
 
 namespace fdk2 {
 
@@ -1121,9 +1122,9 @@ mr_status mr_device_status(int *status)
     int v = 0, zero = 0;
     MR_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_device_error, sizeof(int)));
     MR_CUDA_TRY(cudaMemcpyToSymbol(g_device_error, &zero, sizeof(int)));
-    const int b = bp_device_status_take(), m = msc_device_status_take();
-    if (b < 0 || m < 0) return fail(MR_ERR_CUDA, "mr_device_status: reading an error word failed");
-    *status = v | b | m;
+    const int b = bp_device_status_take(), m = msc_device_status_take(), a = mbp_device_status_take();
+    if (b < 0 || m < 0 || a < 0) return fail(MR_ERR_CUDA, "mr_device_status: reading an error word failed");
+    *status = v | b | m | a;
     return MR_OK;
 }
 
