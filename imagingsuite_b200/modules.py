@@ -301,9 +301,9 @@ class FullLogNorm:
             dl = np.empty_like(doses)
             check(L.lib().mr_lognorm_doselog(doses.ctypes.data_as(L.P_float), nproj, self.fDarkDose,
                                              dl.ctypes.data_as(L.P_float)))
+            doselog = torch.from_numpy(dl).to(img.device)
         else:
-            dl = np.zeros(1, np.float32)
-        doselog = torch.from_numpy(dl).to(img.device)
+            doselog = torch.zeros(1, dtype=torch.float32, device=img.device)  # (a host copy would wait for the stream)
         if out is None:
             out = img if img.dtype == torch.float32 else torch.empty(img.shape, dtype=torch.float32, device=img.device)
         elif out.shape != img.shape or out.dtype != torch.float32 or not out.is_contiguous():
