@@ -109,9 +109,22 @@ __global__ void k_stripe_fft(float *__restrict__ band, int bw, int bh, int n, in
 // upsampling (adding a product with 0 leaves a nonzero sum unchanged, so only the sign of an
 // exactly zero result can differ). Blocks that touch a border take a per-output form with the
 // mirrored indices.
+//
+// Bound by instruction issue: the sums of two filters, or of two neighbouring outputs, go through the
+// paired FP32 pipe together (mac2). 30 taps, 400 x 2048-column blocks, four levels: synthesis rows 1955 ->
+// 1771 us, synthesis columns 1530 -> 1375, analysis rows 984 -> 950 (which had paired products before).
+// The analysis columns keep scalar sums: paired, their taps' register pairs took 884 us instead of 781.
 constexpr int kConvThreads = 128;
 constexpr int kBlk = 8;    // column passes: consecutive outputs per thread
 constexpr int kRowBlk = 6; // synthesis rows: consecutive outputs per thread (lanes' inputs 3 words apart)
+
+// acc += t * x for a pair of sums, product and sum rounded on their own as the reference's: the product is
+// an fma with an addend of -0 that the compiler cannot see (a kernel argument; p + -0 is p bit for bit),
+// because a paired multiply that feeds a paired add would be contracted.
+__device__ __forceinline__ void mac2(float2 &acc, float2 t, float x, float nz)
+{
+    acc = __fadd2_rn(acc, __ffma2_rn(t, make_float2(x, x), make_float2(nz, nz)));
+}
 
 __device__ __forceinline__ void load_taps(const float *__restrict__ taps, int n, float *sm)
 {
@@ -143,15 +156,13 @@ struct Taps {
 // row mirror-padded as pad_mirror. A CTA covers kConvThreads * kRowOut outputs of a row; it
 // stages the inputs they read, mirrored indices resolved, split by parity (E[e] = x[2e],
 // O[e] = x[2e + 1]), so that consecutive outputs read consecutive words (no bank conflicts) and
-// the border outputs need no separate path. A thread computes outputs kConvThreads apart; the
-// two products of a tap are one paired multiply (each element rounded as the scalar one; a
-// paired multiply feeding scalar adds is not contracted).
+// the border outputs need no separate path. A thread computes outputs kConvThreads apart.
 constexpr int kRowOut = 4;
 
 template <int K>
 __global__ void __launch_bounds__(kConvThreads) k_dwt_rows_t(const float *__restrict__ src, RowMap in, int sx,
                                                              int nrows, const float *__restrict__ taps, int dx,
-                                                             float *__restrict__ tmpH, float *__restrict__ tmpG)
+                                                             float *__restrict__ tmpH, float *__restrict__ tmpG, float nz)
 {
     constexpr int SEG = kConvThreads * kRowOut, KH = K / 2, NE = SEG + KH - 1;
     __shared__ float2 tp2[K];
@@ -170,9 +181,9 @@ __global__ void __launch_bounds__(kConvThreads) k_dwt_rows_t(const float *__rest
             od[i] = used ? r[mirror_index(sx, K, p + 1)] : 0.0f;
         }
         __syncthreads();
-        float aH[kRowOut], aG[kRowOut];
+        float2 aHG[kRowOut];
 #pragma unroll
-        for (int o = 0; o < kRowOut; ++o) aH[o] = aG[o] = 0.0f;
+        for (int o = 0; o < kRowOut; ++o) aHG[o] = make_float2(0.0f, 0.0f);
         const int t0 = threadIdx.x + KH - 1; // (k - kc) + KH - 1 for o = 0
 #pragma unroll
         for (int j = 0; j < K; ++j) {
@@ -183,17 +194,15 @@ __global__ void __launch_bounds__(kConvThreads) k_dwt_rows_t(const float *__rest
                 const int ix = (j & 1) ? i - (j - 1) / 2 : i - j / 2;
                 if (!MR_IN_BOUNDS(ix, NE, kSiteRingRows)) continue;
                 const float x = (j & 1) ? ev[ix] : od[ix];
-                const float2 pr = __fmul2_rn(tt, make_float2(x, x));
-                aH[o] = __fadd_rn(aH[o], pr.x);
-                aG[o] = __fadd_rn(aG[o], pr.y);
+                mac2(aHG[o], tt, x, nz);
             }
         }
 #pragma unroll
         for (int o = 0; o < kRowOut; ++o) {
             const int k = kc + threadIdx.x + o * kConvThreads;
             if (k < dx) {
-                tmpH[static_cast<size_t>(row) * dx + k] = aH[o];
-                tmpG[static_cast<size_t>(row) * dx + k] = aG[o];
+                tmpH[static_cast<size_t>(row) * dx + k] = aHG[o].x;
+                tmpG[static_cast<size_t>(row) * dx + k] = aHG[o].y;
             }
         }
     }
@@ -277,29 +286,32 @@ __global__ void __launch_bounds__(kConvThreads) k_dwt_cols_t(const float *__rest
 // src[(k0 + c) / 2 + g]. F is the band's filter offset in the tap pair.
 template <int K, int F>
 __device__ __forceinline__ void up_rows_block(const float *tp, const float *xin, int in0, int xoff, int k0, int kc,
-                                              int w, int dx, float *yout)
+                                              int w, int dx, float *yout, float nz)
 {
     constexpr int c = K - 2, KH = K / 2;
     if (k0 >= 1 && k0 + kRowBlk - 1 < 2 * w - K + 2 && k0 + kRowBlk <= dx) {
         float f[K];
 #pragma unroll
         for (int m = 0; m < K; ++m) f[m] = tp[F + m];
-        float acc[kRowBlk];
+        float2 acc[kRowBlk / 2]; // outputs 2i, 2i + 1: taps m, m + 1 of the same input
 #pragma unroll
-        for (int o = 0; o < kRowBlk; ++o) acc[o] = 0.0f;
+        for (int o = 0; o < kRowBlk / 2; ++o) acc[o] = make_float2(0.0f, 0.0f);
         const float *s0 = xin + xoff; // src[(k0 + c) / 2]
 #pragma unroll
         for (int g = kRowBlk / 2 - 1; g >= 1 - KH; --g) {
             if (!MR_IN_BOUNDS(xoff + g, kConvThreads * kRowBlk / 2 + KH + 2, kSiteRingRows)) continue;
             const float xv = s0[g];
 #pragma unroll
-            for (int o = 0; o < kRowBlk; ++o) {
-                const int m = o - 2 * g;
-                if (m >= 0 && m < K) acc[o] = __fadd_rn(acc[o], __fmul_rn(xv, f[m]));
+            for (int o = 0; o < kRowBlk / 2; ++o) {
+                const int m = 2 * (o - g);
+                if (m >= 0 && m < K) mac2(acc[o], make_float2(f[m], f[m + 1]), xv, nz);
             }
         }
 #pragma unroll
-        for (int o = 0; o < kRowBlk; ++o) yout[k0 - kc + o] = acc[o];
+        for (int o = 0; o < kRowBlk / 2; ++o) {
+            yout[k0 - kc + 2 * o] = acc[o].x;
+            yout[k0 - kc + 2 * o + 1] = acc[o].y;
+        }
         return;
     }
     // a block that reaches a border: its interior outputs here, its border outputs in the CTA's
@@ -338,7 +350,7 @@ template <int K>
 __global__ void __launch_bounds__(kConvThreads) k_up_rows_t(const float *__restrict__ a, const float *__restrict__ hb,
                                                             const float *__restrict__ vb, const float *__restrict__ db,
                                                             int w, int nrows, const float *__restrict__ taps, int dx,
-                                                            float *__restrict__ out)
+                                                            float *__restrict__ out, float nz)
 {
     constexpr int c = K - 2, KH = K / 2, SEG = kConvThreads * kRowBlk, NIN = SEG / 2 + KH + 2;
     __shared__ float tp[2 * K];
@@ -361,8 +373,8 @@ __global__ void __launch_bounds__(kConvThreads) k_up_rows_t(const float *__restr
         }
         __syncthreads();
         if (k0 < dx) {
-            if (q < 2) up_rows_block<K, 0>(tp, xin, in0, xoff, k0, kc, w, dx, yout);
-            else up_rows_block<K, K>(tp, xin, in0, xoff, k0, kc, w, dx, yout);
+            if (q < 2) up_rows_block<K, 0>(tp, xin, in0, xoff, k0, kc, w, dx, yout, nz);
+            else up_rows_block<K, K>(tp, xin, in0, xoff, k0, kc, w, dx, yout, nz);
         }
         // border outputs of the CTA (output 0, and 2w - K + 2 .. dx - 1), one per thread
         {
@@ -384,7 +396,7 @@ __global__ void __launch_bounds__(kConvThreads) k_up_rows_t(const float *__restr
 template <int K>
 __global__ void __launch_bounds__(kConvThreads) k_up_cols_t(const float *__restrict__ rows, int dx, int h, int nb,
                                                             const float *__restrict__ taps, int ox, int oy,
-                                                            float *__restrict__ out, RowMap om)
+                                                            float *__restrict__ out, RowMap om, float nz)
 {
     __shared__ float tp[2 * K];
     load_taps(taps + 2 * K, 2 * K, tp);
@@ -397,28 +409,31 @@ __global__ void __launch_bounds__(kConvThreads) k_up_cols_t(const float *__restr
     const int k1 = min(k0 + kBlk, oy);
     const bool inner = k0 >= 1 && k1 - 1 < 2 * h - K + 2 && k1 - k0 == kBlk;
     if (inner) {
-        float sum[kBlk];
+        float2 sum[kBlk / 2]; // outputs 2i, 2i + 1: taps m, m + 1 of the same input
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int f = (q == 0 || q == 2) ? 0 : K;
             const float *col = rows + q * plane + base + static_cast<size_t>((k0 + c) / 2) * dx;
-            float acc[kBlk];
+            float2 acc[kBlk / 2];
 #pragma unroll
-            for (int o = 0; o < kBlk; ++o) acc[o] = 0.0f;
+            for (int o = 0; o < kBlk / 2; ++o) acc[o] = make_float2(0.0f, 0.0f);
 #pragma unroll
             for (int g = kBlk / 2 - 1; g >= 1 - KH; --g) {
                 const float xv = __ldg(col + static_cast<ptrdiff_t>(g) * dx);
 #pragma unroll
-                for (int o = 0; o < kBlk; ++o) {
-                    const int m = o - 2 * g;
-                    if (m >= 0 && m < K) acc[o] = __fadd_rn(acc[o], __fmul_rn(xv, t[f + m]));
+                for (int o = 0; o < kBlk / 2; ++o) {
+                    const int m = 2 * (o - g);
+                    if (m >= 0 && m < K) mac2(acc[o], make_float2(t[f + m], t[f + m + 1]), xv, nz);
                 }
             }
 #pragma unroll
-            for (int o = 0; o < kBlk; ++o) sum[o] = q == 0 ? acc[o] : __fadd_rn(sum[o], acc[o]);
+            for (int o = 0; o < kBlk / 2; ++o) sum[o] = q == 0 ? acc[o] : __fadd2_rn(sum[o], acc[o]);
         }
 #pragma unroll
-        for (int o = 0; o < kBlk; ++o) out[b * om.bstride + (k0 + o) * om.rstride + x] = sum[o];
+        for (int o = 0; o < kBlk / 2; ++o) {
+            out[b * om.bstride + (k0 + 2 * o) * om.rstride + x] = sum[o].x;
+            out[b * om.bstride + (k0 + 2 * o + 1) * om.rstride + x] = sum[o].y;
+        }
         return;
     }
     for (int k = k0; k < k1; ++k) {
@@ -569,7 +584,7 @@ static void conv_analysis_t(const float *src, rc::RowMap in, int sx, int sy, int
     using namespace rc;
     const int rows = nb * sy;
     k_dwt_rows_t<K><<<dim3(div_up(dx, kConvThreads * kRowOut), std::min(rows, 65535)), kConvThreads, 0, st>>>(
-        src, in, sx, rows, taps_d, dx, tH, tG);
+        src, in, sx, rows, taps_d, dx, tH, tG, -0.0f);
     k_dwt_cols_t<K><<<dim3(div_up(dx, kConvThreads), div_up(dy, kBlk), nb), kConvThreads, 0, st>>>(
         tH, tG, dx, sy, taps_d, dy, a, h, v, d);
 }
@@ -582,9 +597,9 @@ static void conv_synthesis_t(const float *a, const float *h, const float *v, con
     using namespace rc;
     const int rows = nb * hgt;
     k_up_rows_t<K><<<dim3(div_up(dx, kConvThreads * kRowBlk), std::min(rows, 65535), 4), kConvThreads, 0, st>>>(
-        a, h, v, d, w, rows, taps_d, dx, tmp);
+        a, h, v, d, w, rows, taps_d, dx, tmp, -0.0f);
     k_up_cols_t<K><<<dim3(div_up(ox, kConvThreads), div_up(oy, kBlk), nb), kConvThreads, 0, st>>>(
-        tmp, dx, hgt, nb, taps_d, ox, oy, out, om);
+        tmp, dx, hgt, nb, taps_d, ox, oy, out, om, -0.0f);
 }
 
 // every daubN filter length (2N) except daub28's, which the library refuses
