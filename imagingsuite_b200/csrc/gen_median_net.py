@@ -1,7 +1,6 @@
-"""Generate mr_median_net.cuh: median selectors for windows of n = 3, 5, 9, 11, 15 and 25 values.
+"""Generate mr_median_net.cuh: median selectors for windows of n = 3, 5, 9, 15 and 25 values.
 
-Also a rank selector that leaves ranks 7..12 of 20 values on wires 7..12 (for pairs of 5 x 5
-windows). Each selector is Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their
+Each selector is Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their
 applications", AFIPS 1968) on the next power of two, with the padding wires known to hold +inf
 at generation time (compare-exchanges against them vanish or become moves) and every
 compare-exchange that cannot reach the kept outputs removed. What is left is a straight
@@ -34,9 +33,8 @@ def oddeven_merge_sort(n):
     return ces
 
 
-def selector(n, outs=None):
-    """Pruned network for the middle output of n values, or for the output wires in outs (each
-    wire k then holds the k-th smallest value, 0-based)."""
+def selector(n):
+    """Pruned network for the middle output of n values."""
     size = 1
     while size < n:
         size *= 2
@@ -51,7 +49,7 @@ def selector(n, outs=None):
             continue
         ops.append(("ce", a, b))
     out = n // 2
-    live = {out} if outs is None else set(outs)
+    live = {out}
     kept = []
     for op, a, b in reversed(ops):
         if op == "mov":
@@ -93,23 +91,12 @@ def emit(n, f):
     f.write(f"    return v[{out}];\n}}\n\n")
 
 
-def emit_range(n, lo, hi, f):
-    ops, _ = selector(n, range(lo, hi + 1))
-    f.write(f"// ranks {lo}..{hi} (0-based) of {n} values into v[{lo}..{hi}]: {count(ops)} min/max operations\n")
-    f.write(f"__device__ __forceinline__ void rank_net{n}_{lo}_{hi}(float (&v)[{n}])\n{{\n")
-    _body(ops, f)
-    f.write("}\n\n")
-
-
 def main():
     f = sys.stdout
     f.write("// Generated by gen_median_net.py (Batcher odd-even merge sort, pruned to the middle output).\n")
     f.write("#pragma once\n\nnamespace mr {\nnamespace ringalt {\n\n")
-    for n in (3, 5, 9, 11, 15, 25):
+    for n in (3, 5, 9, 15, 25):
         emit(n, f)
-    # two horizontally adjacent 5x5 windows share 20 values; only their ranks 7..12 can be the
-    # middle of either window, which is then the middle of those 6 and the window's own 5
-    emit_range(20, 7, 12, f)
     f.write("} // namespace ringalt\n} // namespace mr\n")
 
 

@@ -57,44 +57,6 @@ __device__ __forceinline__ float median_net9(float (&v)[9])
     return v[4];
 }
 
-// middle of 11 values: 54 min/max operations
-__device__ __forceinline__ float median_net11(float (&v)[11])
-{
-    { const float t = fminf(v[0], v[1]); v[1] = fmaxf(v[0], v[1]); v[0] = t; }
-    { const float t = fminf(v[2], v[3]); v[3] = fmaxf(v[2], v[3]); v[2] = t; }
-    { const float t = fminf(v[0], v[2]); v[2] = fmaxf(v[0], v[2]); v[0] = t; }
-    { const float t = fminf(v[1], v[3]); v[3] = fmaxf(v[1], v[3]); v[1] = t; }
-    { const float t = fminf(v[1], v[2]); v[2] = fmaxf(v[1], v[2]); v[1] = t; }
-    { const float t = fminf(v[4], v[5]); v[5] = fmaxf(v[4], v[5]); v[4] = t; }
-    { const float t = fminf(v[6], v[7]); v[7] = fmaxf(v[6], v[7]); v[6] = t; }
-    { const float t = fminf(v[4], v[6]); v[6] = fmaxf(v[4], v[6]); v[4] = t; }
-    { const float t = fminf(v[5], v[7]); v[7] = fmaxf(v[5], v[7]); v[5] = t; }
-    { const float t = fminf(v[5], v[6]); v[6] = fmaxf(v[5], v[6]); v[5] = t; }
-    { const float t = fminf(v[0], v[4]); v[4] = fmaxf(v[0], v[4]); v[0] = t; }
-    { const float t = fminf(v[2], v[6]); v[6] = fmaxf(v[2], v[6]); v[2] = t; }
-    { const float t = fminf(v[2], v[4]); v[4] = fmaxf(v[2], v[4]); v[2] = t; }
-    { const float t = fminf(v[1], v[5]); v[5] = fmaxf(v[1], v[5]); v[1] = t; }
-    v[3] = fminf(v[3], v[7]);
-    { const float t = fminf(v[3], v[5]); v[5] = fmaxf(v[3], v[5]); v[3] = t; }
-    { const float t = fminf(v[1], v[2]); v[2] = fmaxf(v[1], v[2]); v[1] = t; }
-    { const float t = fminf(v[3], v[4]); v[4] = fmaxf(v[3], v[4]); v[3] = t; }
-    { const float t = fminf(v[5], v[6]); v[6] = fmaxf(v[5], v[6]); v[5] = t; }
-    { const float t = fminf(v[8], v[9]); v[9] = fmaxf(v[8], v[9]); v[8] = t; }
-    { const float t = fminf(v[8], v[10]); v[10] = fmaxf(v[8], v[10]); v[8] = t; }
-    { const float t = fminf(v[9], v[10]); v[10] = fmaxf(v[9], v[10]); v[9] = t; }
-    { const float t = fminf(v[9], v[10]); v[10] = fmaxf(v[9], v[10]); v[9] = t; }
-    v[8] = fmaxf(v[0], v[8]);
-    v[8] = fmaxf(v[4], v[8]);
-    v[10] = fmaxf(v[2], v[10]);
-    v[6] = fminf(v[6], v[10]);
-    v[6] = fminf(v[6], v[8]);
-    v[9] = fmaxf(v[1], v[9]);
-    v[5] = fminf(v[5], v[9]);
-    v[5] = fmaxf(v[3], v[5]);
-    v[5] = fminf(v[5], v[6]);
-    return v[5];
-}
-
 // middle of 15 values: 84 min/max operations
 __device__ __forceinline__ float median_net15(float (&v)[15])
 {
@@ -267,102 +229,6 @@ __device__ __forceinline__ float median_net25(float (&v)[25])
     v[11] = fminf(v[11], v[13]);
     v[12] = fmaxf(v[11], v[12]);
     return v[12];
-}
-
-// ranks 7..12 (0-based) of 20 values into v[7..12]: 168 min/max operations
-__device__ __forceinline__ void rank_net20_7_12(float (&v)[20])
-{
-    { const float t = fminf(v[0], v[1]); v[1] = fmaxf(v[0], v[1]); v[0] = t; }
-    { const float t = fminf(v[2], v[3]); v[3] = fmaxf(v[2], v[3]); v[2] = t; }
-    { const float t = fminf(v[0], v[2]); v[2] = fmaxf(v[0], v[2]); v[0] = t; }
-    { const float t = fminf(v[1], v[3]); v[3] = fmaxf(v[1], v[3]); v[1] = t; }
-    { const float t = fminf(v[1], v[2]); v[2] = fmaxf(v[1], v[2]); v[1] = t; }
-    { const float t = fminf(v[4], v[5]); v[5] = fmaxf(v[4], v[5]); v[4] = t; }
-    { const float t = fminf(v[6], v[7]); v[7] = fmaxf(v[6], v[7]); v[6] = t; }
-    { const float t = fminf(v[4], v[6]); v[6] = fmaxf(v[4], v[6]); v[4] = t; }
-    { const float t = fminf(v[5], v[7]); v[7] = fmaxf(v[5], v[7]); v[5] = t; }
-    { const float t = fminf(v[5], v[6]); v[6] = fmaxf(v[5], v[6]); v[5] = t; }
-    { const float t = fminf(v[0], v[4]); v[4] = fmaxf(v[0], v[4]); v[0] = t; }
-    { const float t = fminf(v[2], v[6]); v[6] = fmaxf(v[2], v[6]); v[2] = t; }
-    { const float t = fminf(v[2], v[4]); v[4] = fmaxf(v[2], v[4]); v[2] = t; }
-    { const float t = fminf(v[1], v[5]); v[5] = fmaxf(v[1], v[5]); v[1] = t; }
-    { const float t = fminf(v[3], v[7]); v[7] = fmaxf(v[3], v[7]); v[3] = t; }
-    { const float t = fminf(v[3], v[5]); v[5] = fmaxf(v[3], v[5]); v[3] = t; }
-    { const float t = fminf(v[1], v[2]); v[2] = fmaxf(v[1], v[2]); v[1] = t; }
-    { const float t = fminf(v[3], v[4]); v[4] = fmaxf(v[3], v[4]); v[3] = t; }
-    { const float t = fminf(v[5], v[6]); v[6] = fmaxf(v[5], v[6]); v[5] = t; }
-    { const float t = fminf(v[8], v[9]); v[9] = fmaxf(v[8], v[9]); v[8] = t; }
-    { const float t = fminf(v[10], v[11]); v[11] = fmaxf(v[10], v[11]); v[10] = t; }
-    { const float t = fminf(v[8], v[10]); v[10] = fmaxf(v[8], v[10]); v[8] = t; }
-    { const float t = fminf(v[9], v[11]); v[11] = fmaxf(v[9], v[11]); v[9] = t; }
-    { const float t = fminf(v[9], v[10]); v[10] = fmaxf(v[9], v[10]); v[9] = t; }
-    { const float t = fminf(v[12], v[13]); v[13] = fmaxf(v[12], v[13]); v[12] = t; }
-    { const float t = fminf(v[14], v[15]); v[15] = fmaxf(v[14], v[15]); v[14] = t; }
-    { const float t = fminf(v[12], v[14]); v[14] = fmaxf(v[12], v[14]); v[12] = t; }
-    { const float t = fminf(v[13], v[15]); v[15] = fmaxf(v[13], v[15]); v[13] = t; }
-    { const float t = fminf(v[13], v[14]); v[14] = fmaxf(v[13], v[14]); v[13] = t; }
-    { const float t = fminf(v[8], v[12]); v[12] = fmaxf(v[8], v[12]); v[8] = t; }
-    { const float t = fminf(v[10], v[14]); v[14] = fmaxf(v[10], v[14]); v[10] = t; }
-    { const float t = fminf(v[10], v[12]); v[12] = fmaxf(v[10], v[12]); v[10] = t; }
-    { const float t = fminf(v[9], v[13]); v[13] = fmaxf(v[9], v[13]); v[9] = t; }
-    { const float t = fminf(v[11], v[15]); v[15] = fmaxf(v[11], v[15]); v[11] = t; }
-    { const float t = fminf(v[11], v[13]); v[13] = fmaxf(v[11], v[13]); v[11] = t; }
-    { const float t = fminf(v[9], v[10]); v[10] = fmaxf(v[9], v[10]); v[9] = t; }
-    { const float t = fminf(v[11], v[12]); v[12] = fmaxf(v[11], v[12]); v[11] = t; }
-    { const float t = fminf(v[13], v[14]); v[14] = fmaxf(v[13], v[14]); v[13] = t; }
-    { const float t = fminf(v[0], v[8]); v[8] = fmaxf(v[0], v[8]); v[0] = t; }
-    { const float t = fminf(v[4], v[12]); v[12] = fmaxf(v[4], v[12]); v[4] = t; }
-    { const float t = fminf(v[4], v[8]); v[8] = fmaxf(v[4], v[8]); v[4] = t; }
-    { const float t = fminf(v[2], v[10]); v[10] = fmaxf(v[2], v[10]); v[2] = t; }
-    { const float t = fminf(v[6], v[14]); v[14] = fmaxf(v[6], v[14]); v[6] = t; }
-    { const float t = fminf(v[6], v[10]); v[10] = fmaxf(v[6], v[10]); v[6] = t; }
-    { const float t = fminf(v[2], v[4]); v[4] = fmaxf(v[2], v[4]); v[2] = t; }
-    { const float t = fminf(v[6], v[8]); v[8] = fmaxf(v[6], v[8]); v[6] = t; }
-    { const float t = fminf(v[10], v[12]); v[12] = fmaxf(v[10], v[12]); v[10] = t; }
-    { const float t = fminf(v[1], v[9]); v[9] = fmaxf(v[1], v[9]); v[1] = t; }
-    { const float t = fminf(v[5], v[13]); v[13] = fmaxf(v[5], v[13]); v[5] = t; }
-    { const float t = fminf(v[5], v[9]); v[9] = fmaxf(v[5], v[9]); v[5] = t; }
-    { const float t = fminf(v[3], v[11]); v[11] = fmaxf(v[3], v[11]); v[3] = t; }
-    v[7] = fminf(v[7], v[15]);
-    { const float t = fminf(v[7], v[11]); v[11] = fmaxf(v[7], v[11]); v[7] = t; }
-    { const float t = fminf(v[3], v[5]); v[5] = fmaxf(v[3], v[5]); v[3] = t; }
-    { const float t = fminf(v[7], v[9]); v[9] = fmaxf(v[7], v[9]); v[7] = t; }
-    { const float t = fminf(v[11], v[13]); v[13] = fmaxf(v[11], v[13]); v[11] = t; }
-    { const float t = fminf(v[1], v[2]); v[2] = fmaxf(v[1], v[2]); v[1] = t; }
-    { const float t = fminf(v[3], v[4]); v[4] = fmaxf(v[3], v[4]); v[3] = t; }
-    { const float t = fminf(v[5], v[6]); v[6] = fmaxf(v[5], v[6]); v[5] = t; }
-    { const float t = fminf(v[7], v[8]); v[8] = fmaxf(v[7], v[8]); v[7] = t; }
-    { const float t = fminf(v[9], v[10]); v[10] = fmaxf(v[9], v[10]); v[9] = t; }
-    { const float t = fminf(v[11], v[12]); v[12] = fmaxf(v[11], v[12]); v[11] = t; }
-    v[13] = fminf(v[13], v[14]);
-    { const float t = fminf(v[16], v[17]); v[17] = fmaxf(v[16], v[17]); v[16] = t; }
-    { const float t = fminf(v[18], v[19]); v[19] = fmaxf(v[18], v[19]); v[18] = t; }
-    { const float t = fminf(v[16], v[18]); v[18] = fmaxf(v[16], v[18]); v[16] = t; }
-    { const float t = fminf(v[17], v[19]); v[19] = fmaxf(v[17], v[19]); v[17] = t; }
-    { const float t = fminf(v[17], v[18]); v[18] = fmaxf(v[17], v[18]); v[17] = t; }
-    { const float t = fminf(v[17], v[18]); v[18] = fmaxf(v[17], v[18]); v[17] = t; }
-    { const float t = fminf(v[17], v[18]); v[18] = fmaxf(v[17], v[18]); v[17] = t; }
-    v[16] = fmaxf(v[0], v[16]);
-    { const float t = fminf(v[8], v[16]); v[16] = fmaxf(v[8], v[16]); v[8] = t; }
-    v[8] = fmaxf(v[4], v[8]);
-    v[12] = fminf(v[12], v[16]);
-    v[18] = fmaxf(v[2], v[18]);
-    v[10] = fminf(v[10], v[18]);
-    { const float t = fminf(v[6], v[10]); v[10] = fmaxf(v[6], v[10]); v[6] = t; }
-    v[8] = fmaxf(v[6], v[8]);
-    { const float t = fminf(v[10], v[12]); v[12] = fmaxf(v[10], v[12]); v[10] = t; }
-    v[17] = fmaxf(v[1], v[17]);
-    { const float t = fminf(v[9], v[17]); v[17] = fmaxf(v[9], v[17]); v[9] = t; }
-    v[9] = fmaxf(v[5], v[9]);
-    v[13] = fminf(v[13], v[17]);
-    v[19] = fmaxf(v[3], v[19]);
-    v[11] = fminf(v[11], v[19]);
-    { const float t = fminf(v[7], v[11]); v[11] = fmaxf(v[7], v[11]); v[7] = t; }
-    { const float t = fminf(v[7], v[9]); v[9] = fmaxf(v[7], v[9]); v[7] = t; }
-    v[11] = fminf(v[11], v[13]);
-    { const float t = fminf(v[7], v[8]); v[8] = fmaxf(v[7], v[8]); v[7] = t; }
-    { const float t = fminf(v[9], v[10]); v[10] = fmaxf(v[9], v[10]); v[9] = t; }
-    { const float t = fminf(v[11], v[12]); v[12] = fmaxf(v[11], v[12]); v[11] = t; }
 }
 
 } // namespace ringalt

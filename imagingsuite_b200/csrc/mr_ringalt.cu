@@ -161,6 +161,23 @@ __device__ __noinline__ float careful_median(const float *img, int w, int h, int
     return win[N / 2];
 }
 
+// The same for a zero middle value of a 5x5 window without NaN inside the image: zeros of one sign only (the
+// usual case, and not rare where an image is flat) need no copy of the window.
+__device__ __noinline__ float zero_median55(const float *img, int w, int h, int x, int y)
+{
+    const float *p = img + static_cast<size_t>(y - 2) * w + (x - 2);
+    bool pos = false, neg = false;
+    for (int r = 0; r < 5; ++r, p += w)
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+            const unsigned b = __float_as_uint(__ldg(p + c));
+            pos |= b == 0u;
+            neg |= b == 0x80000000u;
+        }
+    if (!(pos && neg)) return neg ? -0.0f : 0.0f;
+    return careful_median<5, 5>(img, w, h, x, y, false);
+}
+
 template <int KX, int KY>
 __device__ __forceinline__ float window_median(const float *img, int w, int h, int x, int y)
 {
@@ -200,6 +217,19 @@ __device__ __forceinline__ float median_epilogue(const float *img, const float *
     return m;
 }
 
+// Two pixels at i and i + 1, i even, images 8-byte aligned.
+template <int MODE>
+__device__ __forceinline__ float2 median_epilogue2(const float *img, const float *wt, size_t i, float m0, float m1)
+{
+    if (MODE == MODE_MEDIAN) return make_float2(m0, m1);
+    const float2 p = __ldg(reinterpret_cast<const float2 *>(img + i));
+    if (MODE == MODE_DIFF) return make_float2(__fsub_rn(p.x, m0), __fsub_rn(p.y, m1));
+    if (MODE == MODE_ABSDIFF) return make_float2(fabsf(__fsub_rn(p.x, m0)), fabsf(__fsub_rn(p.y, m1)));
+    const float2 a = __ldg(reinterpret_cast<const float2 *>(wt + i));
+    return make_float2(__fadd_rn(__fmul_rn(__fsub_rn(1.0f, a.x), p.x), __fmul_rn(a.x, m0)),
+                       __fadd_rn(__fmul_rn(__fsub_rn(1.0f, a.y), p.y), __fmul_rn(a.y, m1)));
+}
+
 // One pixel per thread, images along z. MODE_MEDIAN writes the median, MODE_DIFF the image
 // minus it (BasicRingClean.cpp:84-86), MODE_ABSDIFF its absolute difference
 // (MedianMixRingClean.cpp:133-135), MODE_MIX (1 - wt) * p + wt * median
@@ -215,59 +245,207 @@ __global__ void __launch_bounds__(256) k_median(const float *__restrict__ src, i
     dst[blockIdx.z * npix + i] = median_epilogue<MODE>(img, wt, i, window_median<KX, KY>(img, w, h, x, y));
 }
 
-// 5x5 median of two horizontally adjacent pixels per thread. Their windows share the 20 values
-// of columns x-1 .. x+2. A value of rank r among those 20 has rank r .. r+5 in either window,
-// so only ranks 7..12 (0-based) can be a window's middle (rank 12 of 25), and that middle is
-// the middle of the 6 candidates and the window's own 5 values: 168 min/max for the shared
-// ranks plus 54 per window, instead of 202 per window. Pixels whose windows leave the image go
-// through window_median one by one.
-template <int MODE>
-__global__ void __launch_bounds__(256) k_median55_pair(const float *__restrict__ src, int w, int h,
-                                                       const float *__restrict__ wt, float *__restrict__ dst)
+// Batcher's odd-even merge of two sorted lists, unrolled (outputs that nobody reads cost nothing).
+template <int M, int N>
+__device__ __forceinline__ void merge_sorted(const float (&a)[M], const float (&b)[N], float (&o)[M + N])
 {
-    const int x = 2 * (blockIdx.x * 32 + threadIdx.x), y = blockIdx.y * 8 + threadIdx.y;
-    if (x >= w || y >= h) return;
-    const size_t npix = static_cast<size_t>(w) * h, i = static_cast<size_t>(y) * w + x;
+    if constexpr (M == 1 && N == 1) {
+        o[0] = fminf(a[0], b[0]);
+        o[1] = fmaxf(a[0], b[0]);
+    } else {
+        constexpr int ME = (M + 1) / 2, NE = (N + 1) / 2, MO = M / 2, NO = N / 2;
+        float ae[ME], be[NE], e[ME + NE], od[MO + NO];
+#pragma unroll
+        for (int i = 0; i < ME; ++i) ae[i] = a[2 * i];
+#pragma unroll
+        for (int i = 0; i < NE; ++i) be[i] = b[2 * i];
+        merge_sorted(ae, be, e);
+        if constexpr (MO > 0 && NO > 0) {
+            float ao[MO], bo[NO];
+#pragma unroll
+            for (int i = 0; i < MO; ++i) ao[i] = a[2 * i + 1];
+#pragma unroll
+            for (int i = 0; i < NO; ++i) bo[i] = b[2 * i + 1];
+            merge_sorted(ao, bo, od);
+        } else {
+#pragma unroll
+            for (int i = 0; i < MO; ++i) od[i] = a[2 * i + 1];
+#pragma unroll
+            for (int i = 0; i < NO; ++i) od[i] = b[2 * i + 1];
+        }
+        o[0] = e[0];
+#pragma unroll
+        for (int i = 0; i < MO + NO; ++i) {
+            if (i + 1 < ME + NE) {
+                o[2 * i + 1] = fminf(e[i + 1], od[i]);
+                o[2 * i + 2] = fmaxf(e[i + 1], od[i]);
+            } else o[2 * i + 1] = od[i]; // (both lengths even)
+        }
+        if constexpr (ME + NE == MO + NO + 2) o[M + N - 1] = e[ME + NE - 1]; // (both odd)
+    }
+}
+
+__device__ __forceinline__ void sort_pair(float a, float b, float (&o)[2])
+{
+    o[0] = fminf(a, b);
+    o[1] = fmaxf(a, b);
+}
+
+// Middle of 11 values: 6 sorted ones (a), 4 sorted ones (b) and c. The k-th smallest of a and b is the
+// smallest of max(a[i - 1], b[j - 1]) over i + j = k; c is between or beside the fifth and sixth.
+__device__ __forceinline__ float median_6_4_1(const float (&a)[6], const float (&b)[4], float c)
+{
+    const float r4 = fminf(fminf(fminf(a[4], fmaxf(a[3], b[0])), fmaxf(a[2], b[1])), fminf(fmaxf(a[1], b[2]), fmaxf(a[0], b[3])));
+    const float r5 = fminf(fminf(fminf(a[5], fmaxf(a[4], b[0])), fmaxf(a[3], b[1])), fminf(fmaxf(a[2], b[2]), fmaxf(a[1], b[3])));
+    return fmaxf(r4, fminf(r5, c));
+}
+
+// A row of the six columns x - 2 .. x + 3 that two adjacent windows cover: the four inner values sorted,
+// the outer ones, and the sum.
+struct Row6 {
+    float in[4], left, right, sum;
+    template <bool VEC>
+    __device__ __forceinline__ void load(const float *p)
+    {
+        float a, b, c, d;
+        if constexpr (VEC) {
+            const float2 l = __ldg(reinterpret_cast<const float2 *>(p)), m = __ldg(reinterpret_cast<const float2 *>(p + 2)),
+                         r = __ldg(reinterpret_cast<const float2 *>(p + 4));
+            left = l.x, a = l.y, b = m.x, c = m.y, d = r.x, right = r.y;
+        } else {
+            left = __ldg(p), a = __ldg(p + 1), b = __ldg(p + 2), c = __ldg(p + 3), d = __ldg(p + 4), right = __ldg(p + 5);
+        }
+        float lo[2], hi[2];
+        sort_pair(a, b, lo);
+        sort_pair(c, d, hi);
+        merge_sorted(lo, hi, in);
+        sum = ((left + a) + (b + c)) + (d + right);
+    }
+};
+
+// Two such rows.
+struct RowPair6 {
+    float in[8], left[2], right[2], sum;
+    __device__ __forceinline__ void join(const Row6 &a, const Row6 &b)
+    {
+        merge_sorted(a.in, b.in, in);
+        sort_pair(a.left, b.left, left);
+        sort_pair(a.right, b.right, right);
+        sum = a.sum + b.sum;
+    }
+};
+
+// 5x5 median, 2 x 2 pixels at a time. Their windows share the 16 values of rows r1 .. r4 and columns c1 .. c4
+// (of the 6 x 6 values r0 .. r5, c0 .. c5 that they cover); each adds 4 values of row r0 or r5, 4 of column c0
+// or c5, and the corner between them. A value of rank r among the 16 has rank r .. r + 9 in a window, so only
+// ranks 3 .. 12 can be its middle (rank 12 of 25); with the row's 4, ranks 7 .. 12 of the 20; with the
+// column's 4, the fifth and sixth of those 10, and the corner. A thread goes down its two columns two rows
+// at a time: sorted rows, merged pairs of rows and column pairs serve the next pixels as well. Bound by
+// the ALU pipe (min and max at half rate): 168 + 2 x 54 min/max per pixel pair before, about 230 per four
+// pixels now.
+//
+// Pixels whose windows leave the image (x or y in the outer two) go to CTAs of their own: their windows
+// are built value by value, and as a few lanes of the other warps they took half of the time.
+//
+// 180 x 500 x 750: 907 -> 327 us, mixed with a weight image 1028 -> 394 (values in pairs where rows are
+// aligned: 438 -> 417 of it; a zero middle without a copy of the window: 417 -> 394).
+constexpr int kMedianWarps = 4;
+constexpr int kMedianMin = 6; // least width and height
+
+__device__ __noinline__ float edge_median55(const float *img, int w, int h, int x, int y)
+{
+    return window_median<5, 5>(img, w, h, x, y);
+}
+
+// steps: pairs of rows per thread, at most (h - 4) / 2. The last threads of a row and of a column are
+// moved back to end with the image (the pixels they share with others get the same value twice).
+// The first `outer` rows of CTAs take the outer pixels.
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(32 * kMedianWarps, 5) k_median55(const float *__restrict__ src, int w, int h, int steps, int outer,
+                                                                const float *__restrict__ wt, float *__restrict__ dst)
+{
+    const size_t npix = static_cast<size_t>(w) * h;
     const float *img = src + blockIdx.z * npix;
     float *out = dst + blockIdx.z * npix;
-    if (x >= 2 && x + 3 < w && y >= 2 && y + 2 < h) {
-        float c[20], a[5], b[5];
+    if (static_cast<int>(blockIdx.y) < outer) {
+        // the upper and lower two rows, then the outer columns of the others
+        const int j = (blockIdx.y * gridDim.x + blockIdx.x) * 32 * kMedianWarps + threadIdx.y * 32 + threadIdx.x;
+        if (j >= 4 * (w + h - 4)) return;
+        int x, y;
+        if (j < 4 * w) {
+            y = j / w;
+            x = j - y * w;
+            y = y < 2 ? y : h - 4 + y;
+        } else {
+            const int k = j - 4 * w, rows = h - 4;
+            x = k / rows;
+            y = 2 + k - x * rows;
+            x = x < 2 ? x : w - 4 + x;
+        }
+        const size_t i = static_cast<size_t>(y) * w + x;
+        out[i] = median_epilogue<MODE>(img, wt, i, edge_median55(img, w, h, x, y));
+        return;
+    }
+    int x = 2 + 2 * (blockIdx.x * 32 + threadIdx.x);
+    int y0 = 2 + ((blockIdx.y - outer) * kMedianWarps + threadIdx.y) * 2 * steps;
+    if (x > w - 3 || y0 > h - 3) return;
+    x = min(x, w - 4);
+    y0 = min(y0, h - 2 - 2 * steps);
+    Row6 r0, r2, r3;
+    RowPair6 p12;
+    {
+        const float *p = img + static_cast<size_t>(y0 - 2) * w + (x - 2);
+        Row6 r1;
+        r0.load<VEC>(p);
+        r1.load<VEC>(p + w);
+        r2.load<VEC>(p + 2 * static_cast<size_t>(w));
+        r3.load<VEC>(p + 3 * static_cast<size_t>(w));
+        p12.join(r1, r2);
+    }
+#pragma unroll 1
+    for (int y = y0; y < y0 + 2 * steps; y += 2) {
         const float *p = img + static_cast<size_t>(y - 2) * w + (x - 2);
+        Row6 r4, r5;
+        r4.load<VEC>(p + 4 * static_cast<size_t>(w));
+        r5.load<VEC>(p + 5 * static_cast<size_t>(w));
+        RowPair6 p34;
+        p34.join(r3, r4);
+        const float sum = (r0.sum + p12.sum) + (p34.sum + r5.sum); // NaN if a NaN (or +inf and -inf) is among the 36
+
+        float all[16], core[10], left[4], right[4];
+        merge_sorted(p12.in, p34.in, all);
 #pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            const float *q = p + static_cast<size_t>(r) * w;
-            a[r] = __ldg(q);
+        for (int k = 0; k < 10; ++k) core[k] = all[3 + k];
+        merge_sorted(p12.left, p34.left, left);
+        merge_sorted(p12.right, p34.right, right);
+        float m[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) c[r * 4 + k] = __ldg(q + 1 + k);
-            b[r] = __ldg(q + 5);
+        for (int d = 0; d < 2; ++d) {
+            float both[14], mid[6];
+            merge_sorted(core, d ? r5.in : r0.in, both);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) mid[k] = both[4 + k];
+            m[2 * d] = median_6_4_1(mid, left, d ? r5.left : r0.left);
+            m[2 * d + 1] = median_6_4_1(mid, right, d ? r5.right : r0.right);
         }
-        float sc = 0.0f, sa = 0.0f, sb = 0.0f;
+        const bool has_nan = isnan(sum);
 #pragma unroll
-        for (int k = 0; k < 20; ++k) sc += c[k];
+        for (int d = 0; d < 2; ++d) {
 #pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            sa += a[r];
-            sb += b[r];
+            for (int q = 2 * d; q < 2 * d + 2; ++q)
+                if (has_nan) m[q] = careful_median<5, 5>(img, w, h, x + (q & 1), y + d, true);
+                else if (m[q] == 0.0f) m[q] = zero_median55(img, w, h, x + (q & 1), y + d);
+            const size_t i = static_cast<size_t>(y + d) * w + x;
+            if constexpr (VEC) *reinterpret_cast<float2 *>(out + i) = median_epilogue2<MODE>(img, wt, i, m[2 * d], m[2 * d + 1]);
+            else {
+                out[i] = median_epilogue<MODE>(img, wt, i, m[2 * d]);
+                out[i + 1] = median_epilogue<MODE>(img, wt, i + 1, m[2 * d + 1]);
+            }
         }
-        sa += sc; // NaN iff a NaN (or +inf and -inf) is in the window
-        sb += sc;
-        rank_net20_7_12(c);
-        float va[11], vb[11];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) va[k] = vb[k] = c[7 + k];
-#pragma unroll
-        for (int r = 0; r < 5; ++r) {
-            va[6 + r] = a[r];
-            vb[6 + r] = b[r];
-        }
-        float m0 = median_net11(va), m1 = median_net11(vb);
-        if (isnan(sa) || m0 == 0.0f) m0 = careful_median<5, 5>(img, w, h, x, y, isnan(sa));
-        if (isnan(sb) || m1 == 0.0f) m1 = careful_median<5, 5>(img, w, h, x + 1, y, isnan(sb));
-        out[i] = median_epilogue<MODE>(img, wt, i, m0);
-        out[i + 1] = median_epilogue<MODE>(img, wt, i + 1, m1);
-    } else {
-        out[i] = median_epilogue<MODE>(img, wt, i, window_median<5, 5>(img, w, h, x, y));
-        if (x + 1 < w) out[i + 1] = median_epilogue<MODE>(img, wt, i + 1, window_median<5, 5>(img, w, h, x + 1, y));
+        r0 = r2;
+        r2 = r4;
+        r3 = r5;
+        p12 = p34;
     }
 }
 
@@ -403,8 +581,14 @@ static mr_status launch_median(const float *src, int w, int h, size_t nimg, int 
         const dim3 grid(div_up(w, 32), div_up(h, 8), nz), block(32, 8);
         const float *a = src + i0 * npix;
         float *b = dst + i0 * npix;
-        if (kx == 5 && ky == 5) {
-            k_median55_pair<MODE><<<dim3(div_up(w, 64), div_up(h, 8), nz), block, 0, s>>>(a, w, h, wt, b);
+        if (kx == 5 && ky == 5 && w >= ringalt::kMedianMin && h >= ringalt::kMedianMin) {
+            const int steps = std::min(8, (h - 4) / 2);
+            const unsigned gx = div_up((w - 3) / 2, 32), outer = div_up(4 * (static_cast<size_t>(w) + h - 4), 32 * kMedianWarps * gx);
+            // rows that begin on 8 bytes: values in pairs
+            const bool vec = w % 2 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(wt)) % 8 == 0;
+            const auto kernel = vec ? k_median55<MODE, true> : k_median55<MODE, false>;
+            kernel<<<dim3(gx, outer + div_up((h - 4 + 2 * steps - 1) / (2 * steps), kMedianWarps), nz), dim3(32, kMedianWarps), 0, s>>>(
+                a, w, h, steps, static_cast<int>(outer), wt, b);
             continue;
         }
 #define MR_MEDIAN_CASE(KX, KY)                                                                                         \
@@ -420,6 +604,7 @@ static mr_status launch_median(const float *src, int w, int h, size_t nimg, int 
         MR_MEDIAN_CASE(1, 5)
         MR_MEDIAN_CASE(5, 3)
         MR_MEDIAN_CASE(3, 5)
+        MR_MEDIAN_CASE(5, 5)
 #undef MR_MEDIAN_CASE
         return fail(MR_ERR_UNSUPPORTED, "median filter: kernel %dx%d", kx, ky);
     }
