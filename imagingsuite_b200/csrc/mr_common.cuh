@@ -88,8 +88,8 @@ enum BoundsSite {
     kSiteFdkDirect = 2,  // k_fdk: detector row and column of a sample
     kSiteBpStaged = 3,   // k_bp_par_staged: staged box sample
     kSiteFdkStaged = 4,  // k_fdk_staged: staged box sample (byte offset in the stage buffers)
-    kSiteMbpBins = 5,    // k_mbp_forward_smem: bin in shared memory
-    kSiteMbpAdjoint = 6, // k_mbp_adjoint: projection sample
+    kSiteMbpBins = 5,    // k_mbp_forward_*: bin
+    kSiteMbpAdjoint = 6, // k_mbp_adjoint_staged: projection sample
     kSiteRingRows = 7,   // k_dwt_rows_t / k_up_rows_t: staged row input
     kSiteSpotNbr = 8     // k_complete: neighbour pixel
 };

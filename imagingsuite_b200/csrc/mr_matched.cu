@@ -13,20 +13,18 @@
 // Forward projection (the exact transpose): detector bin m of slice z and projection i collects
 // wa * vol from every voxel whose n is m and wb * vol from every voxel whose n is m - 1, with the
 // same u, n, wa and wb evaluated by the same expressions, so <A x, p> = <x, A^T p> holds to float
-// summation. Two kernels: a voxel-driven one (k_mbp_forward_smem, below) while a projection's
-// bins for 32 slices fit in shared memory, else a ray-driven one: a warp owns one (i, m) and 32 consecutive slices (lanes), walks the
-// volume rows when |sin_i| >= |cos_i| (else the columns) and, in each, only the candidate
-// voxels whose u can fall in [m - 1, m + 1): the interval of the affine u, widened by one voxel
-// on each side for the float evaluation (u is exact to ~1e-4 pixel, the walk's step is at least
-// 1/sqrt(2) pixel). Each candidate's contribution is decided by its own n, as in the adjoint.
+// summation. Two kernels, both driven by the voxels: k_mbp_forward_smem holds a projection's bins for 32
+// slices in shared memory, k_mbp_forward_strip (wider detectors) gives each warp a few bins of its own.
 // The derivative d proj / d c_z (-vol for the wa term, +vol for the wb term: d wa / du = -1,
-// d wb / du = +1, du / dc_z = 1) comes out of the same walk.
+// d wb / du = +1, du / dc_z = 1) comes out of the same walks.
 #include "mr_common.cuh"
 #include "mr_tma.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <vector>
 
@@ -293,92 +291,234 @@ static mr_status launch_adjoint(AdjParams P, int width, cudaStream_t s)
     return check_launch("k_mbp_adjoint_staged");
 }
 
-// One warp per (projection i, bin m), lanes = 32 consecutive slices from z0.
+// Forward projection. Both kernels walk lines of voxels along the axis on which u changes least (x when
+// |sin| <= |cos|, else y; |du| <= 1/sqrt(2) per step, so a lane's bin moves by at most one between steps), one
+// slice per lane, with the adjoint's u, n, wa and wb. A lane keeps the sums of its current pair of bins
+// (n, n + 1) in registers and hands a bin on (Put) when its walk leaves it. On a line whose positions all lie on
+// the detector the floor comes from the bits of u + 1.5 * 2^23 added rounding down, without conversions.
+constexpr int kFwdPad = 33; // words between bins: 32 lanes' slices hit 32 banks, the write-out's bins do too
+constexpr int kFwdU = 4;    // voxels loaded ahead
+
+// Sums of a walk whose u grows (UP) or falls: bins cur and cur + 1 (as kAdjMagic bits, 0: none yet), the
+// values a0, a1, and for the derivative the sum s of v over the current run (-v for the lower bin, +v for
+// the upper) with what the run before left in the bin that the walk leaves next (carry).
+template <bool DERIV, bool UP, class Put>
+struct BinRun {
+    int cur = 0;
+    float a0 = 0.0f, a1 = 0.0f, s = 0.0f, carry = 0.0f;
+    Put put;
+    __device__ __forceinline__ explicit BinRun(const Put &p) : put(p) {}
+    __device__ __forceinline__ void done()
+    {
+        if (cur == 0) return;
+        put(cur, a0, UP ? carry - s : -s);
+        put(cur + 1, a1, UP ? s : carry + s);
+        cur = 0;
+        a0 = a1 = s = carry = 0.0f;
+    }
+    // one voxel of value v: bin m (bits), weights 1 - wb and wb
+    __device__ __forceinline__ void add(int m, float wb, float v)
+    {
+        if (m != cur) {
+            if (m == cur + (UP ? 1 : -1)) {
+                put(UP ? cur : cur + 1, UP ? a0 : a1, UP ? carry - s : carry + s);
+                if (UP) a0 = a1, a1 = 0.0f;
+                else a1 = a0, a0 = 0.0f;
+                carry = UP ? s : -s;
+                s = 0.0f;
+            } else done();
+            cur = m;
+        }
+        a0 = fmaf(v, __fsub_rn(1.0f, wb), a0);
+        a1 = fmaf(v, wb, a1);
+        if (DERIV) s = __fadd_rn(s, v);
+    }
+};
+
+// Wide detectors: a warp owns kStripBins consecutive bins of a projection for 32 slices and collects them
+// alone, so nothing is added atomically and a result does not depend on timing. It walks, on each line, the
+// voxels that can reach one of its bins: the interval of the affine u for its 32 slices, widened by a bound
+// of u's float evaluation; each voxel's contribution is decided by its own n. Bins beyond the warp's own are
+// dropped when the walk leaves them (their own warp has the voxel too).
+//
+// Bound by instruction issue (80 %). With the derivative, 512^2 x 20 slices x 120 projections 2010 -> 1411 us
+// (by all of a projection's bins in shared memory before), 1024^2 x 32 x 60 11520 -> 3010 (by one warp per bin
+// before). 4 bins per warp: 1744 and 3720, the ends of a strip being visited twice; 16: 1480 and 3511.
+constexpr int kStripBins = 8;
+constexpr int kStripWarps = 4; // projections per CTA (neighbours walk almost the same voxels)
+
+struct FwdParams {
+    const float *vol;
+    const float2 *sc;
+    const float *startu;
+    int nproj, n, nz;
+    const uint32_t *mask;
+    float *proj, *dproj;
+};
+
+// adds to the lane's column in shared memory, for the warp's own bins; the derivative's column follows
 template <bool DERIV>
-__global__ void __launch_bounds__(128) k_mbp_forward(const float *__restrict__ vol, const float2 *__restrict__ sc,
-                                                     const float *__restrict__ startu, int nproj, int n, int nz,
-                                                     const uint32_t *__restrict__ mask, float *__restrict__ proj,
-                                                     float *__restrict__ dproj)
+struct StripPut {
+    float *bins;
+    int base; // bits of the first bin
+    __device__ __forceinline__ void operator()(int bin, float v, float d) const
+    {
+        const unsigned k = static_cast<unsigned>(bin - base);
+        if (k >= kStripBins) return;
+        bins[k * kFwdPad] = __fadd_rn(bins[k * kFwdPad], v);
+        if (DERIV) bins[(k + kStripBins) * kFwdPad] = __fadd_rn(bins[(k + kStripBins) * kFwdPad], d);
+    }
+};
+
+// The integers from lo to hi within [first, last] that t0 .. t1 (in either order) spans; a NaN end is open.
+__device__ __forceinline__ void fwd_span(float t0, float t1, int first, int last, int &lo, int &hi)
+{
+    const float a = fminf(t0, t1), b = fmaxf(t0, t1);
+    lo = static_cast<int>(fminf(fmaxf(floorf(a), static_cast<float>(first)), static_cast<float>(last) + 1.0f));
+    hi = static_cast<int>(fmaxf(fminf(ceilf(b), static_cast<float>(last)), static_cast<float>(first) - 1.0f));
+}
+
+// ROWS: lines are rows y, walked along x; else columns x, walked along y.
+template <bool DERIV, bool ROWS, bool UP>
+__device__ __forceinline__ void strip_walk(const FwdParams &P, float2 s, float suz, int z, int first, float *bins)
 {
     const int lane = threadIdx.x & 31;
-    const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int i = blockIdx.y;
-    const int z0 = blockIdx.z * 32, z = z0 + lane;
-    if (m >= n) return;
-    const bool zok = z < nz;
-    const float2 s = sc[i];
-    const float *su = startu + static_cast<size_t>(i) * nz;
-    const float suz = zok ? su[z] : 0.0f;
-    // the warp's extreme start positions (startu is affine in z), for the candidate interval
-    const int zl = min(z0 + 31, nz - 1);
-    const float sua = fminf(su[z0], su[zl]), sub = fmaxf(su[z0], su[zl]);
-    const float fm = static_cast<float>(m);
-    float acc = 0.0f, dacc = 0.0f;
-    auto visit = [&](int x1, int y1) {
-        const float u = __fsub_rn(__fadd_rn(suz, __fmul_rn(s.y, static_cast<float>(y1))), __fmul_rn(s.x, static_cast<float>(x1)));
-        const int k = __float2int_rz(u);
-        if (k < 0 || k > n - 2 || (k != m && k != m - 1)) return;
-        const float wb = fabsf(__fsub_rn(u, static_cast<float>(k)));
-        const float v = __ldg(vol + (static_cast<size_t>(y1 - 1) * n + (x1 - 1)) * nz + z);
-        if (k == m) {
-            acc = __fadd_rn(acc, __fmul_rn(v, __fsub_rn(1.0f, wb)));
-            if (DERIV) dacc = __fsub_rn(dacc, v);
-        } else {
-            acc = __fadd_rn(acc, __fmul_rn(v, wb));
-            if (DERIV) dacc = __fadd_rn(dacc, v);
-        }
-    };
-    if (fabsf(s.x) >= fabsf(s.y)) {
-        // walk the rows y; in row y, u = (su + cos y) - sin x lies in [m - 1, m + 1) for x in
-        // ((su + cos y - m - 1) / sin, (su + cos y - m + 1) / sin] (sin > 0; reversed for sin < 0)
-        const float inv = 1.0f / s.x;
-        for (int y1 = 1; y1 <= n; ++y1) {
-            const uint32_t first = mask[2 * (y1 - 1)], second = mask[2 * (y1 - 1) + 1];
-            if (second <= first) continue;
-            const float cy = s.y * static_cast<float>(y1);
-            const float e0 = (sua + cy - fm - 1.0f) * inv, e1 = (sub + cy - fm + 1.0f) * inv;
-            int xa = static_cast<int>(floorf(fminf(e0, e1))) - 1, xb = static_cast<int>(ceilf(fmaxf(e0, e1))) + 1;
-            xa = max(xa, static_cast<int>(first) + 1);
-            xb = min(xb, static_cast<int>(second));
-            if (zok)
-                for (int x1 = xa; x1 <= xb; ++x1) visit(x1, y1);
-        }
-    } else {
-        // walk the columns x; u lies in [m - 1, m + 1) for y in
-        // ((m - 1 - su + sin x) / cos, (m + 1 - su + sin x) / cos] (cos > 0; reversed otherwise)
-        const float inv = 1.0f / s.y;
-        for (int x1 = 1; x1 <= n; ++x1) {
-            const float sx = s.x * static_cast<float>(x1);
-            const float e0 = (fm - 1.0f - sub + sx) * inv, e1 = (fm + 1.0f - sua + sx) * inv;
-            int ya = max(static_cast<int>(floorf(fminf(e0, e1))) - 1, 1);
-            int yb = min(static_cast<int>(ceilf(fmaxf(e0, e1))) + 1, n);
-            if (zok)
-                for (int y1 = ya; y1 <= yb; ++y1) {
-                    const uint32_t first = mask[2 * (y1 - 1)], second = mask[2 * (y1 - 1) + 1];
-                    if (static_cast<uint32_t>(x1) > first && static_cast<uint32_t>(x1) <= second) visit(x1, y1);
-                }
-        }
+    BinRun<DERIV, UP, StripPut<DERIV>> run({bins, first + kAdjMagicBits});
+    // u = su + h line + g f, with the warp's range of su
+    const float g = ROWS ? -s.x : s.y, h = ROWS ? s.y : -s.x, fn = static_cast<float>(P.n);
+    float sul = suz, suh = suz;
+    for (int o = 16; o > 0; o >>= 1) {
+        sul = fminf(sul, __shfl_xor_sync(0xffffffffu, sul, o));
+        suh = fmaxf(suh, __shfl_xor_sync(0xffffffffu, suh, o));
     }
-    if (zok) {
-        const size_t o = (static_cast<size_t>(i) * nz + z) * n + m;
-        proj[o] = acc;
-        if (DERIV) dproj[o] = dacc;
+    if (__any_sync(0xffffffffu, !(fabsf(suz) <= FLT_MAX))) sul = -INFINITY, suh = INFINITY;
+    // u (and the bounds below) are a few roundings of terms of at most 2 n + |su|
+    const float eps = (fn + fmaxf(fabsf(sul), fabsf(suh))) * 0x1p-18f;
+    const float u0 = static_cast<float>(first) - 1.0f - eps - suh, u1 = static_cast<float>(first + kStripBins) + eps - sul;
+    const float inv = 1.0f / g;
+    int l0, l1;
+    {
+        const float ih = 1.0f / h;
+        fwd_span((u0 - fmaxf(g, g * fn)) * ih, (u1 - fminf(g, g * fn)) * ih, 1, P.n, l0, l1);
+    }
+    const uint32_t stride = ROWS ? static_cast<uint32_t>(P.nz) : static_cast<uint32_t>(P.n) * static_cast<uint32_t>(P.nz);
+    for (int l = l0; l <= l1; ++l) {
+        const float fl = static_cast<float>(l), at = h * fl;
+        int lo = 0, hi = 0; // 1-based
+        if (ROWS) {
+            const uint32_t ma = P.mask[2 * (l - 1)], mb = P.mask[2 * (l - 1) + 1];
+            fwd_span((u0 - at) * inv, (u1 - at) * inv, static_cast<int>(min(ma, static_cast<uint32_t>(P.n))) + 1,
+                     static_cast<int>(min(mb, static_cast<uint32_t>(P.n))), lo, hi);
+        } else
+            fwd_span((u0 - at) * inv, (u1 - at) * inv, 1, P.n, lo, hi);
+        const float fixed = ROWS ? __fadd_rn(suz, __fmul_rn(s.y, fl)) : __fmul_rn(s.x, fl);
+        auto position = [&](float f) {
+            return ROWS ? __fsub_rn(fixed, __fmul_rn(s.x, f)) : __fsub_rn(__fadd_rn(suz, __fmul_rn(s.y, f)), fixed);
+        };
+        for (int f = lo; f <= hi; f += 32) {
+            // the voxels of the mask among the next 32
+            int cnt = min(32, hi - f + 1), skip = 0;
+            uint32_t word = 0xffffffffu >> (32 - cnt);
+            if (!ROWS) {
+                bool in = lane < cnt;
+                if (in) {
+                    const uint32_t ma = P.mask[2 * (f + lane - 1)], mb = P.mask[2 * (f + lane - 1) + 1];
+                    in = static_cast<uint32_t>(l) > ma && static_cast<uint32_t>(l) <= mb;
+                }
+                word = __ballot_sync(0xffffffffu, in);
+                if (word == 0) continue;
+                skip = __ffs(word) - 1;
+                word >>= skip;
+                cnt = 32 - __clz(word);
+            }
+            const int f0 = f + skip;
+            float ff = static_cast<float>(f0);
+            const float *p = P.vol + (ROWS ? (static_cast<size_t>(l - 1) * P.n + (f0 - 1)) * P.nz
+                                           : (static_cast<size_t>(f0 - 1) * P.n + (l - 1)) * P.nz) + z;
+            // (position is monotone: the ends bound it)
+            const float ua = position(ff), ub = position(static_cast<float>(f0 + cnt - 1));
+            const bool clean = __all_sync(0xffffffffu, fminf(ua, ub) >= 0.0f && fmaxf(ua, ub) < fn - 1.0f);
+            for (int q = 0; q < cnt; q += kFwdU, word >>= kFwdU - 1, word >>= 1) {
+                constexpr uint32_t ALL = (1u << kFwdU) - 1;
+                float v[kFwdU];
+                if (clean && (word & ALL) == ALL) {
+#pragma unroll
+                    for (int j = 0; j < kFwdU; ++j) v[j] = __ldg(p + static_cast<size_t>(stride) * j);
+#pragma unroll
+                    for (int j = 0; j < kFwdU; ++j) {
+                        const float u = position(ff + static_cast<float>(j));
+                        const float k = __fadd_rd(u, kAdjMagic);
+                        run.add(__float_as_int(k), __fsub_rn(u, __fsub_rn(k, kAdjMagic)), v[j]);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kFwdU; ++j) v[j] = (word >> j & 1) ? __ldg(p + static_cast<size_t>(stride) * j) : 0.0f;
+#pragma unroll 1
+                    for (int j = 0; j < kFwdU; ++j) {
+                        if (!(word >> j & 1)) continue;
+                        const float u = position(ff + static_cast<float>(j));
+                        const int m = __float2int_rz(u);
+                        float vj = v[0];
+#pragma unroll
+                        for (int i = 1; i < kFwdU; ++i) vj = j == i ? v[i] : vj;
+                        if (m >= 0 && m <= P.n - 2) run.add(m + kAdjMagicBits, fabsf(__fsub_rn(u, static_cast<float>(m))), vj);
+                    }
+                }
+                ff += static_cast<float>(kFwdU);
+                p += static_cast<size_t>(stride) * kFwdU;
+            }
+        }
+        run.done();
     }
 }
 
-// The same forward projection, voxel-driven (used while the bins fit in shared memory): one CTA
-// per (projection i, 32 slices) holds that projection's bins of its slices in shared memory
-// (bin-major rows padded to 33 words, so the 32 lanes - one slice each - of a warp hit 32 banks
-// and the write-out reads 32 consecutive bins without conflicts). Its warps walk the masked
-// voxels line by line, along the axis on which u changes least (x when |sin| <= |cos|, else y;
-// |du| <= 1/sqrt(2) per step, so a lane's bin moves by at most one between steps), each voxel
-// once, with the adjoint's u, n, wa and wb. A lane keeps the running sums of its current pair of
-// bins (n, n + 1) in registers and adds a bin to shared memory (atomically) when its walk leaves
-// it, so most voxels cost no shared-memory access. The order of the additions into a bin depends
-// on the warps' timing: results agree with the ray-driven kernel to float summation, not bit for
-// bit.
-constexpr int kFwdPad = 33;
+template <bool DERIV>
+__global__ void __launch_bounds__(kStripWarps * 32, 10) k_mbp_forward_strip(const __grid_constant__ FwdParams P)
+{
+    constexpr int WORDS = kStripBins * kFwdPad * (DERIV ? 2 : 1);
+    __shared__ float sums[kStripWarps][WORDS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * kStripWarps + warp;
+    if (i >= P.nproj) return;
+    // chunks of bins from the middle outwards: those that cross most of the mask start first
+    const int c = blockIdx.y, first = (static_cast<int>(gridDim.y) / 2 + (c & 1 ? -((c + 1) / 2) : c / 2)) * kStripBins;
+    const int z0 = blockIdx.z * 32, z = min(z0 + lane, P.nz - 1); // (lanes beyond the last slice repeat it)
+    float *mine = sums[warp];
+    for (int e = lane; e < WORDS; e += 32) mine[e] = 0.0f;
+    __syncwarp();
+    const float2 s = P.sc[i];
+    const float suz = P.startu[static_cast<size_t>(i) * P.nz + z];
+    // u falls along x by sin and grows along y by cos
+    if (fabsf(s.x) <= fabsf(s.y)) {
+        if (s.x <= 0.0f) strip_walk<DERIV, true, true>(P, s, suz, z, first, mine + lane);
+        else strip_walk<DERIV, true, false>(P, s, suz, z, first, mine + lane);
+    } else if (s.y >= 0.0f) strip_walk<DERIV, false, true>(P, s, suz, z, first, mine + lane);
+    else strip_walk<DERIV, false, false>(P, s, suz, z, first, mine + lane);
+    __syncwarp();
+    for (int e = lane; e < 32 * kStripBins; e += 32) {
+        const int zz = e / kStripBins, k = e % kStripBins;
+        if (z0 + zz >= P.nz || first + k >= P.n) continue;
+        const size_t o = (static_cast<size_t>(i) * P.nz + z0 + zz) * P.n + first + k;
+        if (!MR_IN_BOUNDS(o, static_cast<size_t>(P.nproj) * P.nz * P.n, kSiteMbpBins)) continue;
+        P.proj[o] = mine[k * kFwdPad + zz];
+        if (DERIV) P.dproj[o] = mine[(k + kStripBins) * kFwdPad + zz];
+    }
+}
+
+// Narrow detectors: a cluster of one or two CTAs per (projection i, 32 slices) holds that projection's bins of
+// its slices in shared memory; its warps share the lines of voxels and add a bin atomically when a walk leaves
+// it, so most voxels cost no shared-memory access. Two CTAs' bins are summed on the way out. The order of
+// the additions into a bin depends on the warps' timing: results agree with the strips' to float summation,
+// not bit for bit.
+//
+// Bound by instruction issue. 256^2 x 64 slices, 180 projections, with the derivative: 1231 -> 965 us (two CTAs
+// where they shorten the last wave: 991 with one), 192^2 x 16 x 60 307 -> 125 (one: 216), 64^2 x 8 x 60 42 -> 22.
+// Clusters of four and eight find too few places for CTAs that fill an SM (192^2 x 64 x 360: 994 -> 3661 with
+// eight). Up to kFwdSmemBins, two CTAs' bins fit an SM and this beats the strips: 384^2 x 20 x 120 815 against
+// 887 us, 64^2 x 8 x 60 22 against 86; at 512^2 1455 against 1401, and 1387 against 888 with 8 slices and 60
+// projections.
 constexpr int kFwdThreads = 1024;
+constexpr size_t kFwdSmemBins = 400;
 
 __host__ __device__ inline size_t fwd_smem_bytes(int n, bool deriv)
 {
@@ -386,64 +526,80 @@ __host__ __device__ inline size_t fwd_smem_bytes(int n, bool deriv)
 }
 
 template <bool DERIV>
-struct BinRun {
-    int mc = -2; // current bin (-2: none yet)
-    float a0 = 0.0f, a1 = 0.0f, d0 = 0.0f, d1 = 0.0f;
-    // one voxel: bin m (0 <= m <= n - 2), weights wa, wb, value v
-    __device__ __forceinline__ void add(float *bins, float *dbins, int lane, int m, float wa, float wb, float v)
+struct AtomicPut {
+    float *bins, *dbins; // of this lane, bin 0
+    __device__ __forceinline__ void operator()(int bin, float v, float d) const
     {
-        (void)dbins; // (the derivative bins follow the value bins)
-        const float pa = __fmul_rn(v, wa), pb = __fmul_rn(v, wb);
-        const int diff = m - mc;
-        if (diff == 0) {
-            a0 = __fadd_rn(a0, pa);
-            a1 = __fadd_rn(a1, pb);
-            if (DERIV) {
-                d0 = __fsub_rn(d0, v);
-                d1 = __fadd_rn(d1, v);
-            }
-        } else if (diff == -1) { // bin mc + 1 is left behind
-            atomicAdd(bins + (mc + 1) * kFwdPad + lane, a1);
-            a1 = __fadd_rn(a0, pb);
-            a0 = pa;
-            if (DERIV) {
-                atomicAdd(dbins + (mc + 1) * kFwdPad + lane, d1);
-                d1 = __fadd_rn(d0, v);
-                d0 = -v;
-            }
-            mc = m;
-        } else if (diff == 1) { // bin mc is left behind
-            atomicAdd(bins + mc * kFwdPad + lane, a0);
-            a0 = __fadd_rn(a1, pa);
-            a1 = pb;
-            if (DERIV) {
-                atomicAdd(dbins + mc * kFwdPad + lane, d0);
-                d0 = __fsub_rn(d1, v);
-                d1 = v;
-            }
-            mc = m;
-        } else {
-            done(bins, dbins, lane);
-            a0 = pa;
-            a1 = pb;
-            if (DERIV) {
-                d0 = -v;
-                d1 = v;
-            }
-            mc = m;
-        }
-    }
-    __device__ __forceinline__ void done(float *bins, float *dbins, int lane) const
-    {
-        if (mc < 0) return;
-        atomicAdd(bins + mc * kFwdPad + lane, a0);
-        atomicAdd(bins + (mc + 1) * kFwdPad + lane, a1);
-        if (DERIV) {
-            atomicAdd(dbins + mc * kFwdPad + lane, d0);
-            atomicAdd(dbins + (mc + 1) * kFwdPad + lane, d1);
-        }
+        atomicAdd(bins + (bin - kAdjMagicBits) * kFwdPad, v);
+        if (DERIV) atomicAdd(dbins + (bin - kAdjMagicBits) * kFwdPad, d);
     }
 };
+
+// (warp: of nwarps in the cluster)
+template <bool DERIV, bool UP>
+__device__ __forceinline__ void forward_walk(const float *__restrict__ vol, float2 s, float suz, int n, int nz, int z, bool by_rows,
+                                             int warp, int nwarps,
+                                             const uint2 *rowmask, const uint2 *colspan, float *bins, float *dbins)
+{
+    BinRun<DERIV, UP, AtomicPut<DERIV>> run({bins, dbins});
+    constexpr int U = kFwdU;
+    // positions of a line: u(f) for the line coordinate f
+    auto visit = [&](float u, float v, bool clean) {
+        if (clean) {
+            const float k = __fadd_rd(u, kAdjMagic);
+            if (!MR_IN_BOUNDS(__float_as_int(k) - kAdjMagicBits + 1, n, kSiteMbpBins)) return;
+            run.add(__float_as_int(k), __fsub_rn(u, __fsub_rn(k, kAdjMagic)), v);
+        } else {
+            const int m = __float2int_rz(u);
+            if (m < 0 || m > n - 2 || !MR_IN_BOUNDS(m + 1, n, kSiteMbpBins)) return;
+            run.add(m + kAdjMagicBits, fabsf(__fsub_rn(u, static_cast<float>(m))), v);
+        }
+    };
+    auto line = [&](int from, int to, const float *p, size_t stride, auto position, auto inside) {
+        // (position is monotone: its ends bound it)
+        const float ua = position(static_cast<float>(from + 1)), ub = position(static_cast<float>(to));
+        const bool clean = __all_sync(__activemask(), fminf(ua, ub) >= 0.0f && fmaxf(ua, ub) < static_cast<float>(n - 1));
+        float f = static_cast<float>(from + 1);
+        for (int q = from; q < to; q += U, p += U * stride) {
+            float v[U];
+            bool in[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                in[j] = q + j < to && inside(q + j);
+                v[j] = in[j] ? __ldg(p + j * stride) : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j, f = __fadd_rn(f, 1.0f))
+                if (in[j]) visit(position(f), v[j], clean);
+        }
+    };
+    if (by_rows) {
+        // line y: voxels x in (first, second], u = (su + cos y) - sin x
+        for (int y = warp; y < n; y += nwarps) {
+            const uint2 r = rowmask[y];
+            const int xa = static_cast<int>(r.x), xe = min(static_cast<int>(r.y), n);
+            if (xe <= xa) continue;
+            const float a = __fadd_rn(suz, __fmul_rn(s.y, static_cast<float>(y + 1)));
+            line(xa, xe, vol + (static_cast<size_t>(y) * n + xa) * nz + z, nz,
+                 [&](float f) { return __fsub_rn(a, __fmul_rn(s.x, f)); }, [](int) { return true; });
+        }
+    } else {
+        // line x: voxels y in the column's span that the row masks hold (bit 31 of its end: all of them)
+        for (int x = warp; x < n; x += nwarps) {
+            const uint2 span = colspan[x];
+            const uint32_t x1 = static_cast<uint32_t>(x) + 1;
+            const int ya = static_cast<int>(span.x), ye = static_cast<int>(span.y & 0x7FFFFFFFu);
+            if (ye <= ya) continue;
+            const float sx = __fmul_rn(s.x, static_cast<float>(x1));
+            const float *p = vol + (static_cast<size_t>(ya) * n + x) * nz + z;
+            const size_t stride = static_cast<size_t>(n) * nz;
+            auto position = [&](float f) { return __fsub_rn(__fadd_rn(suz, __fmul_rn(s.y, f)), sx); };
+            if (span.y >> 31) line(ya, ye, p, stride, position, [](int) { return true; });
+            else line(ya, ye, p, stride, position, [&](int y) { return x1 > rowmask[y].x && x1 <= rowmask[y].y; });
+        }
+    }
+    run.done();
+}
 
 template <bool DERIV>
 __global__ void __launch_bounds__(kFwdThreads, 1) k_mbp_forward_smem(const float *__restrict__ vol, const float2 *__restrict__ sc,
@@ -451,12 +607,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mbp_forward_smem(const float
                                                                   int nz, const uint32_t *__restrict__ mask,
                                                                   float *__restrict__ proj, float *__restrict__ dproj)
 {
-    extern __shared__ float bins[]; // [n][kFwdPad] (+ [n][kFwdPad] for the derivative), then the masks
-    float *dbins = bins + static_cast<size_t>(n) * kFwdPad;
-    uint2 *rowmask = reinterpret_cast<uint2 *>(bins + static_cast<size_t>(n) * kFwdPad * (DERIV ? 2 : 1));
-    uint2 *colspan = rowmask + n; // per column x: the rows [lo, hi] that hold voxels of it
-    const int i = blockIdx.x, z0 = blockIdx.y * 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    extern __shared__ uint2 rowmask[]; // the masks, then bins [n][kFwdPad] (+ [n][kFwdPad] for the derivative)
+    float *bins = reinterpret_cast<float *>(rowmask + 2 * n), *dbins = bins + static_cast<size_t>(n) * kFwdPad;
+    uint2 *colspan = rowmask + n; // per column x: the rows [lo, hi) that hold voxels of it; bit 31: all of them do
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = cluster.block_rank(), ctas = cluster.num_blocks();
+    const int i = blockIdx.x / ctas, z0 = blockIdx.y * 32;
+    const int lane = threadIdx.x & 31;
     const int z = z0 + lane;
     const bool zok = z < nz;
     for (int e = threadIdx.x; e < n * kFwdPad * (DERIV ? 2 : 1); e += blockDim.x) bins[e] = 0.0f;
@@ -467,93 +624,41 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mbp_forward_smem(const float
     if (!by_rows)
         for (int x = threadIdx.x; x < n; x += blockDim.x) {
             const uint32_t x1 = static_cast<uint32_t>(x) + 1;
-            int lo = 0, hi = -1;
+            int lo = 0, hi = -1, count = 0;
             for (int y = 0; y < n; ++y)
                 if (x1 > rowmask[y].x && x1 <= rowmask[y].y) {
-                    lo = y;
-                    break;
-                }
-            for (int y = n - 1; y >= lo; --y)
-                if (x1 > rowmask[y].x && x1 <= rowmask[y].y) {
+                    if (count++ == 0) lo = y;
                     hi = y;
-                    break;
                 }
-            colspan[x] = make_uint2(static_cast<uint32_t>(lo), static_cast<uint32_t>(hi + 1));
+            const uint32_t all = count == hi + 1 - lo ? 0x80000000u : 0u;
+            colspan[x] = make_uint2(static_cast<uint32_t>(lo), static_cast<uint32_t>(hi + 1) | all);
         }
     __syncthreads();
-    BinRun<DERIV> run;
-    const float suz = zok ? startu[static_cast<size_t>(i) * nz + z] : 0.0f;
     if (zok) {
-        if (by_rows) {
-            // line y: voxels x in (first, second], u = (su + cos y) - sin x
-            for (int y = warp; y < n; y += nwarps) {
-                const uint2 r = rowmask[y];
-                const float a = __fadd_rn(suz, __fmul_rn(s.y, static_cast<float>(y + 1)));
-                const float *p = vol + (static_cast<size_t>(y) * n + r.x) * nz + z;
-                constexpr int U = 4;
-                int x = static_cast<int>(r.x);
-                const int xe = min(static_cast<int>(r.y), n);
-                for (; x < xe; x += U) {
-                    float v[U];
-#pragma unroll
-                    for (int j = 0; j < U; ++j) v[j] = (x + j < xe) ? __ldg(p + static_cast<size_t>(j) * nz) : 0.0f;
-#pragma unroll
-                    for (int j = 0; j < U; ++j) {
-                        if (x + j >= xe) continue;
-                        const float u = __fsub_rn(a, __fmul_rn(s.x, static_cast<float>(x + j + 1)));
-                        const int m = __float2int_rz(u);
-                        if (m < 0 || m > n - 2) continue;
-                        const float wb = fabsf(__fsub_rn(u, static_cast<float>(m)));
-                        if (!MR_IN_BOUNDS(m + 1, n, kSiteMbpBins)) continue;
-                        run.add(bins, dbins, lane, m, __fsub_rn(1.0f, wb), wb, v[j]);
-                    }
-                    p += static_cast<size_t>(U) * nz;
-                }
-            }
-        } else {
-            // line x: voxels y in the column's span that the row masks hold
-            for (int x = warp; x < n; x += nwarps) {
-                const uint2 span = colspan[x];
-                const uint32_t x1 = static_cast<uint32_t>(x) + 1;
-                const float sx = __fmul_rn(s.x, static_cast<float>(x1));
-                const size_t ystride = static_cast<size_t>(n) * nz;
-                const float *p = vol + (static_cast<size_t>(span.x) * n + x) * nz + z;
-                constexpr int U = 4;
-                int y = static_cast<int>(span.x);
-                const int ye = static_cast<int>(span.y);
-                for (; y < ye; y += U) {
-                    float v[U];
-                    bool in[U];
-#pragma unroll
-                    for (int j = 0; j < U; ++j) {
-                        in[j] = y + j < ye && x1 > rowmask[y + j].x && x1 <= rowmask[y + j].y;
-                        v[j] = in[j] ? __ldg(p + static_cast<size_t>(j) * ystride) : 0.0f;
-                    }
-#pragma unroll
-                    for (int j = 0; j < U; ++j) {
-                        if (!in[j]) continue;
-                        const float u = __fsub_rn(__fadd_rn(suz, __fmul_rn(s.y, static_cast<float>(y + j + 1))), sx);
-                        const int m = __float2int_rz(u);
-                        if (m < 0 || m > n - 2) continue;
-                        const float wb = fabsf(__fsub_rn(u, static_cast<float>(m)));
-                        if (!MR_IN_BOUNDS(m + 1, n, kSiteMbpBins)) continue;
-                        run.add(bins, dbins, lane, m, __fsub_rn(1.0f, wb), wb, v[j]);
-                    }
-                    p += static_cast<size_t>(U) * ystride;
-                }
-            }
-        }
-        run.done(bins, dbins, lane);
+        const float suz = startu[static_cast<size_t>(i) * nz + z];
+        const int warp = rank * (kFwdThreads / 32) + static_cast<int>(threadIdx.x >> 5), nwarps = ctas * (kFwdThreads / 32);
+        // u falls along x by sin and grows along y by cos
+        if (by_rows ? s.x <= 0.0f : s.y >= 0.0f)
+            forward_walk<DERIV, true>(vol, s, suz, n, nz, z, by_rows, warp, nwarps, rowmask, colspan, bins + lane, dbins + lane);
+        else
+            forward_walk<DERIV, false>(vol, s, suz, n, nz, z, by_rows, warp, nwarps, rowmask, colspan, bins + lane, dbins + lane);
     }
-    __syncthreads();
-    // write-out: consecutive threads take consecutive bins of one slice (coalesced stores)
+    cluster.sync();
+    // write-out: consecutive threads take consecutive bins of one slice (coalesced stores), summed over the CTAs
     const int zs = min(32, nz - z0);
-    for (int e = threadIdx.x; e < zs * n; e += blockDim.x) {
+    for (int e = rank * kFwdThreads + threadIdx.x; e < zs * n; e += ctas * kFwdThreads) {
         const int zz = e / n, m = e - zz * n;
         const size_t o = (static_cast<size_t>(i) * nz + z0 + zz) * n + m;
-        proj[o] = bins[m * kFwdPad + zz];
-        if (DERIV) dproj[o] = dbins[m * kFwdPad + zz];
+        float a = 0.0f, d = 0.0f;
+        for (int r = 0; r < ctas; ++r) {
+            const float *there = cluster.map_shared_rank(bins, r);
+            a = __fadd_rn(a, there[m * kFwdPad + zz]);
+            if (DERIV) d = __fadd_rn(d, there[(n + m) * kFwdPad + zz]);
+        }
+        proj[o] = a;
+        if (DERIV) dproj[o] = d;
     }
+    cluster.sync(); // (the others may still read these bins)
 }
 
 } // namespace mr
@@ -643,32 +748,43 @@ mr_status mr_mbp_forward(const float *vol_d, size_t n, size_t nz, const float *s
     if (n < 2 || n > 65536 || nz == 0 || nz > 65536 || nproj == 0 || nproj > 65535)
         return fail(MR_ERR_ARGUMENT, "mr_mbp_forward: unsupported size");
     const float2 *sc = reinterpret_cast<const float2 *>(sincos_d);
-    int dev = 0, optin = 0;
-    MR_CUDA_TRY(cudaGetDevice(&dev));
-    MR_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t smem = fwd_smem_bytes(static_cast<int>(n), dproj_d != nullptr);
-    if (smem <= static_cast<size_t>(optin)) {
-        dim3 sgrid(static_cast<unsigned>(nproj), div_up(nz, 32));
-        auto launch = [&](auto kernel, float *d) -> mr_status {
+    if (n <= kFwdSmemBins) {
+        // two CTAs per (projection, 32 slices) where that shortens the last wave
+        const size_t units = nproj * div_up(nz, 32);
+        const unsigned ctas = div_up(2 * units, 148) < 2 * div_up(units, 148) ? 2 : 1;
+        const size_t smem = fwd_smem_bytes(static_cast<int>(n), dproj_d != nullptr);
+        auto launch = [&](auto kernel) -> mr_status {
             MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-            kernel<<<sgrid, kFwdThreads, smem, as_stream(stream)>>>(vol_d, sc, startu_d, static_cast<int>(nproj),
-                                                                   static_cast<int>(n), static_cast<int>(nz), mask_d,
-                                                                   proj_d, d);
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim = {ctas, 1, 1};
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(static_cast<unsigned>(nproj) * ctas, div_up(nz, 32));
+            cfg.blockDim = dim3(kFwdThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = as_stream(stream);
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            MR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, vol_d, sc, startu_d, static_cast<int>(nproj), static_cast<int>(n),
+                                           static_cast<int>(nz), mask_d, proj_d, dproj_d));
             return check_launch("k_mbp_forward_smem");
         };
-        return dproj_d ? launch(k_mbp_forward_smem<true>, dproj_d) : launch(k_mbp_forward_smem<false>, nullptr);
+        return dproj_d ? launch(k_mbp_forward_smem<true>) : launch(k_mbp_forward_smem<false>);
     }
-    // bins beyond shared memory: the ray-driven kernel
-    dim3 grid(div_up(n, 4), static_cast<unsigned>(nproj), div_up(nz, 32));
-    if (dproj_d)
-        k_mbp_forward<true><<<grid, 128, 0, as_stream(stream)>>>(vol_d, reinterpret_cast<const float2 *>(sincos_d),
-                                                               startu_d, static_cast<int>(nproj), static_cast<int>(n),
-                                                               static_cast<int>(nz), mask_d, proj_d, dproj_d);
-    else
-        k_mbp_forward<false><<<grid, 128, 0, as_stream(stream)>>>(vol_d, reinterpret_cast<const float2 *>(sincos_d),
-                                                                startu_d, static_cast<int>(nproj), static_cast<int>(n),
-                                                                static_cast<int>(nz), mask_d, proj_d, nullptr);
-    return check_launch("k_mbp_forward");
+    FwdParams P;
+    P.vol = vol_d;
+    P.sc = reinterpret_cast<const float2 *>(sincos_d);
+    P.startu = startu_d;
+    P.nproj = static_cast<int>(nproj);
+    P.n = static_cast<int>(n);
+    P.nz = static_cast<int>(nz);
+    P.mask = mask_d;
+    P.proj = proj_d;
+    P.dproj = dproj_d;
+    const dim3 grid(div_up(nproj, kStripWarps), div_up(n, kStripBins), div_up(nz, 32));
+    if (dproj_d) k_mbp_forward_strip<true><<<grid, kStripWarps * 32, 0, as_stream(stream)>>>(P);
+    else k_mbp_forward_strip<false><<<grid, kStripWarps * 32, 0, as_stream(stream)>>>(P);
+    return check_launch("k_mbp_forward_strip");
 }
 
 } // extern "C"
