@@ -33,8 +33,9 @@ def oddeven_merge_sort(n):
     return ces
 
 
-def selector(n):
-    """Pruned network for the middle output of n values."""
+def selector(n, outs=None):
+    """Pruned network for the middle output of n values, or for the output wires in outs (each
+    wire k then holds the k-th smallest value, 0-based)."""
     size = 1
     while size < n:
         size *= 2
@@ -49,7 +50,7 @@ def selector(n):
             continue
         ops.append(("ce", a, b))
     out = n // 2
-    live = {out}
+    live = {out} if outs is None else set(outs)
     kept = []
     for op, a, b in reversed(ops):
         if op == "mov":
