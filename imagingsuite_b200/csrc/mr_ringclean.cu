@@ -111,7 +111,7 @@ __global__ void k_stripe_fft(float *__restrict__ band, int bw, int bh, int n, in
 // mirrored indices.
 //
 // Bound by instruction issue: the sums of two filters, or of two neighbouring outputs, go through the
-// paired FP32 pipe together (mac2). 30 taps, 400 x 2048-column blocks, four levels: synthesis rows 1955 ->
+// paired FP32 pipe together (mac2). 30 taps, 1125 x 64 x 2048, two levels: synthesis rows 1955 ->
 // 1771 us, synthesis columns 1530 -> 1375, analysis rows 984 -> 950 (which had paired products before).
 // The analysis columns keep scalar sums: paired, their taps' register pairs took 884 us instead of 781.
 constexpr int kConvThreads = 128;
