@@ -152,6 +152,36 @@ __device__ __forceinline__ void staged_column(float2 (&acc)[TZ / 2], const float
     }
 }
 
+// Two voxel columns at once, each only where it reaches the detector (on0, on1): footprints that lie partly
+// outside it, on tiles of few slices. One column after the other, behind a branch each, their latency held up
+// the tiles at the volume's corners: 128^2 x 8 slices from 180 projections 59 -> 53 us. (32-slice tiles have
+// the warps to hide it: 256^2 x 64 from 360 takes 388 us that way, 399 this way.)
+template <int MODE, int TZ>
+__device__ __forceinline__ void staged_columns(float2 (&acc0)[TZ / 2], float2 (&acc1)[TZ / 2], const float *p0, const float *p1,
+                                               float d0, float d1, bool on0, bool on1, float g0, float tinc, float2 nz)
+{
+#pragma unroll
+    for (int q4 = 0; q4 < TZ; q4 += 4) {
+        const float g = g0 + static_cast<float>(q4 / 4);
+        const float wb0 = group_weight<MODE>(d0, g, tinc), wa0 = __fsub_rn(1.0f, wb0);
+        const float wb1 = group_weight<MODE>(d1, g, tinc), wa1 = __fsub_rn(1.0f, wb1);
+#pragma unroll
+        for (int q = q4; q < q4 + 4; q += 2) {
+            float2 s0 = acc0[q / 2], s1 = acc1[q / 2];
+            const float2 a0 = make_float2(p0[q * BW], p0[(q + 1) * BW]), a1 = make_float2(p1[q * BW], p1[(q + 1) * BW]);
+            if constexpr (MODE == kNearest || MODE == kTiltNearest) {
+                s0 = __fadd2_rn(s0, a0);
+                s1 = __fadd2_rn(s1, a1);
+            } else {
+                blend_add(s0, a0, make_float2(p0[q * BW + 1], p0[(q + 1) * BW + 1]), both(wa0), both(wb0), nz);
+                blend_add(s1, a1, make_float2(p1[q * BW + 1], p1[(q + 1) * BW + 1]), both(wa1), both(wb1), nz);
+            }
+            acc0[q / 2] = make_float2(on0 ? s0.x : acc0[q / 2].x, on0 ? s0.y : acc0[q / 2].y);
+            acc1[q / 2] = make_float2(on1 ? s1.x : acc1[q / 2].x, on1 ? s1.y : acc1[q / 2].y);
+        }
+    }
+}
+
 // The slices of two voxels of neighbouring rows for one staged projection. u changes by cos between
 // them, so the second voxel's pair of samples is the first one's (step false) or the next (step
 // true): three samples serve both, where each alone loads two. lo is the voxel with the smaller n.
@@ -327,14 +357,14 @@ __global__ void __launch_bounds__(32 * NW, CTAS) k_bp_par_staged(const __grid_co
                 if constexpr (MODE == kTilt)
                     for (int g = 0; g < group0; ++g) d = __fsub_rn(d, P.tinc);
             };
-            // One row's column from any footprint (fallback and edges: positions formed here).
+            // One row's column from any footprint (fallback, and edges of 32-slice tiles: positions formed here).
             auto row = [&](float2 (&acc)[TZ / 2], int b, float4 g, int4 m, float fy) {
                 const float u = posu<MODE>(g.x, g.y, g.z, fx, fy, P.toff);
                 const int n = __float2int_rz(u);
                 if (n < 0 || n > um2) return;
                 float d = __fsub_rn(u, static_cast<float>(n));
                 skip_groups(d);
-                if (m.y != kUnfit) {
+                if (TZ >= 32 && m.y != kUnfit) {
                     // the box holds all TZ rows (zeros beyond the detector); slices from zmax on are not stored
                     const uint32_t off = static_cast<uint32_t>((st * NB + b) * (BW * TZ) + (n - m.x));
                     if (MR_IN_BOUNDS(off + (TZ - 1) * BW + 1, 2 * NB * BW * TZ, kSiteBpStaged))
@@ -405,6 +435,20 @@ __global__ void __launch_bounds__(32 * NW, CTAS) k_bp_par_staged(const __grid_co
                         } else {
                             staged_pair<MODE, TZ>(acc1, acc0, S.box + at, step, q_d1[0], q_d0[0], g0, P.tinc, nz);
                         }
+                    } else if (m.y == kStaged && TZ < 32) {
+                        // positions formed here, truncated as the reference does. The box holds all TZ rows
+                        // (zeros beyond the detector); slices from zmax on are not stored
+                        const float u0 = posu<MODE>(g.x, g.y, g.z, fx, fy0, P.toff), u1 = posu<MODE>(g.x, g.y, g.z, fx, fy1, P.toff);
+                        const int n0 = __float2int_rz(u0), n1 = __float2int_rz(u1);
+                        bool on0 = inside[0] && n0 >= 0 && n0 <= um2, on1 = inside[1] && n1 >= 0 && n1 <= um2;
+                        float d0 = __fsub_rn(u0, static_cast<float>(n0)), d1 = __fsub_rn(u1, static_cast<float>(n1));
+                        skip_groups(d0);
+                        skip_groups(d1);
+                        const uint32_t at = static_cast<uint32_t>((st * NB + b) * (BW * TZ));
+                        const uint32_t a0 = at + (on0 ? n0 - m.x : 0), a1 = at + (on1 ? n1 - m.x : 0);
+                        if (!MR_IN_BOUNDS(a0 + (TZ - 1) * BW + 1, 2 * NB * BW * TZ, kSiteBpStaged)) on0 = false;
+                        if (!MR_IN_BOUNDS(a1 + (TZ - 1) * BW + 1, 2 * NB * BW * TZ, kSiteBpStaged)) on1 = false;
+                        staged_columns<MODE, TZ>(acc0, acc1, S.box + (on0 ? a0 : at), S.box + (on1 ? a1 : at), d0, d1, on0, on1, g0, P.tinc, nz);
                     } else if (m.y != kNothing) {
                         if (inside[0]) row(acc0, b, g, m, fy0);
                         if (inside[1]) row(acc1, b, g, m, fy1);
@@ -492,7 +536,9 @@ static mr_status launch_tile(PFN_cuTensorMapEncodeTiled enc, const Params &P, si
 // projections), and the slices a tile holds beyond the volume's cost the same: 40 slices at 500^2
 // from 500 projections take 1.49, 1.33 and 1.46 ms, 12 slices at 700^2 from 400 1.18, 0.69 and 0.92.
 // A volume with fewer 16-slice tiles than SMs is bound by the latency of one tile's projection loop:
-// 96^2 x 16 from 200 projections takes 136, 81 and 66 us.
+// 96^2 x 16 from 200 projections takes 136, 81 and 66 us (59 since two columns go at once). With fewer than
+// half as many, 4-slice tiles are shorter still and batches of 32 projections put half the barriers in them:
+// 49 us, and 128^2 x 8 from 180 53 -> 45 (16 projections per batch: 54 -> 52 before).
 template <int MODE>
 static mr_status launch_mode(PFN_cuTensorMapEncodeTiled enc, const Params &P, size_t nslabs, cudaStream_t s)
 {
@@ -500,6 +546,7 @@ static mr_status launch_mode(PFN_cuTensorMapEncodeTiled enc, const Params &P, si
     const int cost32 = 10 * padded(32), cost16 = 12 * padded(16), cost8 = 15 * padded(8);
     const size_t tiles16 = static_cast<size_t>(div_up(static_cast<size_t>(P.nu), TX)) *
                            div_up(static_cast<size_t>(P.yend - P.ybegin), 8) * div_up(static_cast<size_t>(P.nz4), 16);
+    if (2 * tiles16 < 148) return launch_tile<MODE, 4, 4, 32, 4>(enc, P, nslabs, s);
     if (tiles16 < 148 || (cost8 < cost16 && cost8 < cost32)) return launch_tile<MODE, 8, 4, 16, 4>(enc, P, nslabs, s);
     if (cost16 < cost32) return launch_tile<MODE, 16, 4, 8, 4>(enc, P, nslabs, s);
     return launch_tile<MODE, 32, 8, 8, 2>(enc, P, nslabs, s);
