@@ -69,6 +69,7 @@ struct AdjParams {
     const uint32_t *mask;
     float *vol;
     int nproj, n, nz, pitch, accumulate, wait_limit;
+    int staged; // 0: rows that TMA cannot address, every sample by guarded global loads
     float neg_zero;
 };
 
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(co
             int mode = kAdjNothing;
             const int w0 = (lo - 1) & ~3;
             if (i < P.nproj) {
-                if (!ok || hi + 2 >= w0 + kAdjBW) mode = kAdjUnfit;
+                if (!ok || !P.staged || hi + 2 >= w0 + kAdjBW) mode = kAdjUnfit;
                 else if (hi >= -1 && lo <= n) mode = lo >= 1 && hi <= n - 3 ? kAdjClean : kAdjStaged;
             }
             const bool head = corner == 0, load = head && mode >= kAdjStaged;
@@ -273,16 +274,18 @@ __global__ void __launch_bounds__(256) k_pad_rows(const float *__restrict__ src,
 
 static mr_status launch_adjoint(AdjParams P, int width, cudaStream_t s)
 {
-    PFN_cuTensorMapEncodeTiled enc = tma::encode_fn();
-    if (!enc) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-    CUtensorMap map;
-    cuuint64_t dims[3] = {static_cast<cuuint64_t>(width), static_cast<cuuint64_t>(P.nz), static_cast<cuuint64_t>(P.nproj)};
-    cuuint64_t strides[2] = {static_cast<cuuint64_t>(P.pitch) * 4, static_cast<cuuint64_t>(P.pitch) * P.nz * 4};
-    cuuint32_t box[3] = {kAdjBW, kAdjTZ, 1}, estr[3] = {1, 1, 1};
-    const CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(P.proj), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
+    CUtensorMap map = {};
+    if (P.staged) {
+        PFN_cuTensorMapEncodeTiled enc = tma::encode_fn();
+        if (!enc) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+        cuuint64_t dims[3] = {static_cast<cuuint64_t>(width), static_cast<cuuint64_t>(P.nz), static_cast<cuuint64_t>(P.nproj)};
+        cuuint64_t strides[2] = {static_cast<cuuint64_t>(P.pitch) * 4, static_cast<cuuint64_t>(P.pitch) * P.nz * 4};
+        cuuint32_t box[3] = {kAdjBW, kAdjTZ, 1}, estr[3] = {1, 1, 1};
+        const CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(P.proj), dims, strides, box, estr,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (cr != CUDA_SUCCESS) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
+    }
     MR_CUDA_TRY(cudaFuncSetAttribute(k_mbp_adjoint_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(adj_smem_bytes())));
     const dim3 grid(div_up(static_cast<size_t>(P.n), kAdjTX), div_up(static_cast<size_t>(P.n), kAdjTY),
@@ -706,6 +709,7 @@ mr_status mr_mbp_adjoint(const float *proj_d, size_t n, size_t nz, const float *
     P.accumulate = accumulate;
     P.wait_limit = tma::g_batch_wait_limit.load();
     P.neg_zero = -0.0f;
+    P.staged = 1;
     cudaStream_t s = as_stream(stream);
     const bool direct = n % 4 == 0 && n >= kAdjBW && reinterpret_cast<uintptr_t>(proj_d) % 16 == 0;
     if (nproj == 0) { // an empty sum
@@ -722,7 +726,13 @@ mr_status mr_mbp_adjoint(const float *proj_d, size_t n, size_t nz, const float *
     const size_t pitch = std::max<size_t>(kAdjBW, (n + 3) / 4 * 4), per = nz * pitch;
     const size_t run = std::min(nproj, std::max<size_t>(kAdjNB, (size_t(64) << 20) / (per * 4)));
     float *scratch = nullptr;
-    MR_TRY(device_alloc(&scratch, run * per * sizeof(float), s, "mr_mbp_adjoint: padded projections"));
+    if (device_alloc(&scratch, run * per * sizeof(float), s, "mr_mbp_adjoint: padded projections") != MR_OK) {
+        P.proj = proj_d; // no room for copies
+        P.pitch = P.n;
+        P.nproj = static_cast<int>(nproj);
+        P.staged = 0;
+        return launch_adjoint(P, P.n, s);
+    }
     mr_status st = MR_OK;
     for (size_t i = 0; i < nproj && st == MR_OK; i += run) {
         const size_t m = std::min(run, nproj - i);

@@ -276,10 +276,12 @@ mr_status mr_bp_parallel(const void *proj_d, int dtype, const float *scale_d, co
                          const int32_t *index_d, const float *sin_d, const float *cos_d, const float *startu_d,
                          size_t nproj, size_t nu, size_t nv, const uint32_t *mask_d, int correcttilt, float tiltoffset,
                          float tiltinc, float *vol_d, void *stream);
-/* The same backprojection with the projection rows of each 32 x 8 x 32 voxel tile staged in
- * shared memory by TMA (FP32, no tilt correction, row pitch a multiple of 16 bytes);
- * nslabs = number of projection slabs in proj_d (the bound of every TMA load). Other
- * requests run mr_bp_parallel. Results are bit-identical on both paths. */
+/* The same backprojection with the projection rows of each voxel tile staged in shared memory by
+ * TMA (FP32, with and without tilt correction); nslabs = number of projection slabs in proj_d (the
+ * bound of every TMA load). Rows that TMA cannot address (nu not a multiple of 4, proj_d not on 16
+ * bytes) and weighted slabs go through aligned copies, up to 1 GiB of scratch at a time; other
+ * requests, and any without that scratch, run mr_bp_parallel. Results are bit-identical on every
+ * path. */
 mr_status mr_bp_parallel_staged(const void *proj_d, size_t nslabs, int dtype, const float *scale_d,
                                 const float *weight_d, const int32_t *index_d, const float *sin_d, const float *cos_d,
                                 const float *startu_d, size_t nproj, size_t nu, size_t nv, const uint32_t *mask_d,
@@ -378,9 +380,10 @@ mr_status mr_fdk_backproject_slab(const void *proj_d, int dtype, const float *sc
                                   size_t k_end, float *vol_d, void *stream);
 /* Shared-memory staging box for mr_fdk_backproject (host): the largest detector footprint
  * (columns box_w, rows box_h) of a 32 x 8 x 32 voxel tile over a sample of the geometry,
- * from the host copies of the partials. With box_w = box_h = 0, or when the projection
- * layout does not allow TMA (row pitch not a multiple of 16 bytes), or without uniform_z,
- * mr_fdk_backproject uses direct global loads; tiles whose footprint exceeds the box fall
+ * from the host copies of the partials. Projections whose layout does not allow TMA (row pitch not
+ * a multiple of 16 bytes) go through aligned copies, up to 1 GiB of scratch at a time. With box_w =
+ * box_h = 0, or without uniform_z, or without that scratch, mr_fdk_backproject uses direct global
+ * loads; tiles whose footprint exceeds the box fall
  * back to direct loads for that projection. Results are identical on every path. */
 mr_status mr_fdk_box(const float *xip_h, const float *yip_h, const float *zip_h, size_t nu, size_t nv, size_t nproj,
                      int dtype, int *box_w, int *box_h);
@@ -470,7 +473,9 @@ mr_status mr_slice_dot(const float *a_d, const float *b_d, size_t nproj, size_t 
  * 0, nz)), projections [nproj][nz][n] (the detector is n bins wide, as the reference's
  * backprojector takes it). mr_mbp_geometry (host): sincos_h [nproj][2] = sin, cos of the
  * direction-signed angle and startu_h [nproj][nz] = (n/2)(sin - cos) + c_z, the reference's float
- * expressions. mr_mbp_forward also returns d proj / d c_z in dproj_d when it is not NULL. */
+ * expressions. mr_mbp_forward also returns d proj / d c_z in dproj_d when it is not NULL.
+ * Adjoint rows that TMA cannot address (n not a multiple of 4 or below 48, proj_d not on 16 bytes)
+ * go through padded copies, up to 64 MiB of scratch at a time; without it, guarded global loads. */
 mr_status mr_mbp_geometry(const float *angles_h, size_t nproj, size_t n, size_t nz, float centre, float tan_tilt,
                           float pivot, int direction, float *sincos_h, float *startu_h);
 mr_status mr_mbp_adjoint(const float *proj_d, size_t n, size_t nz, const float *sincos_d, const float *startu_d,
@@ -486,7 +491,7 @@ mr_status mr_device_status(int *status);
  * exceptions at each level, ReconEngine.cpp:810-833, and times modules with a CPU timer,
  * ProcessModuleBase.cpp:129-149).
  * mr_set_wait_limit: tries of each per-batch mbarrier wait in the TMA-staged backprojectors
- *   (default 4194304; a negative value restores it), read at each launch. A wait that runs
+ *   (and the matched adjoint; default 4194304; a negative value restores it), read at each launch. A wait that runs
  *   out sets the device error word (mr_device_status returns 1), skips the rest of the block's
  *   projections, waits for the block's copies still in flight (with the default limit) and
  *   returns; the context stays usable. 0 makes every such wait expire at once.

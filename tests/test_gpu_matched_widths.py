@@ -52,3 +52,19 @@ def test_padded_runs_continue_the_sums(cuda):
     for a, b in ((0, 100), (100, 230), (230, 400)):
         J.MatchedOperator(n, nz, ang[a:b]).adjoint(p[a:b].contiguous(), n / 2, 0.3, out=out, accumulate=True)
     assert torch.equal(whole, out)
+
+
+@pytest.mark.parametrize("n,tilt", [(31, 0.4), (65, -0.9)])
+def test_adjoint_without_scratch(cuda, n, tilt):
+    """No room for the padded copies: the same values by guarded loads."""
+    nz, ang = 8, (np.arange(40) * 4.5).astype(np.float32)
+    g = torch.Generator(device=cuda).manual_seed(n)
+    p = torch.randn((40, nz, n), device=cuda, generator=g)
+    op = J.MatchedOperator(n, nz, ang)
+    exp = op.adjoint(p, n / 2 + 1.3, tilt)
+    L.check(L.lib().mr_debug_fail_allocation(0))
+    try:
+        got = op.adjoint(p, n / 2 + 1.3, tilt)
+    finally:
+        L.check(L.lib().mr_debug_fail_allocation(-1))
+    assert torch.equal(got, exp)
