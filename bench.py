@@ -791,16 +791,16 @@ def run_parallel(args, production: bool):
     hbm = float(peaks.get("hbm_gbs", 6650.0))
     tbp = times["backprojection"] / 1e3
     ach = 8.0 * updates / tbp / 1e9
-    # shared-memory load wavefronts of the staged backprojector: two per warp and update (the
-    # two samples of the linear interpolation, consecutive x in a warp: no bank conflicts),
-    # counted for the warps that have a voxel inside the circle mask
+    # shared-memory load wavefronts of the staged backprojector: three per warp and two updates (two
+    # neighbouring rows' linear interpolations share three samples, consecutive x in a warp: no bank
+    # conflicts), counted for the warps that have a voxel inside the circle mask
     m = bp._mask.cpu().numpy().view(np.uint32).reshape(-1, 2).astype(np.int64)
     warps = 0
     for first, second in m:
         lo, hi = first + 1, second  # 1-based x inside: first < x <= second
         if hi >= lo:
             warps += (hi - 1) // 32 - (lo - 1) // 32 + 1
-    wavefronts = 2.0 * warps * ((nrows // 4) * 4) * sel
+    wavefronts = 1.5 * warps * ((nrows // 4) * 4) * sel
     sm_mhz = clocks.get("sm_mhz") or float(peaks.get("sm_max_mhz", 1965.0))
     from imagingsuite_b200 import _lib as L
 
