@@ -451,10 +451,13 @@ __global__ void __launch_bounds__(32 * kMedianWarps, 5) k_median55(const float *
 
 // Mean projection accumulated in projection order (BasicRingClean.cpp:56-69 starts from a copy
 // of the first projection, MedianMixRingClean.cpp:113-125 from zero), times 1 / nproj.
-// VEC: four pixels per thread.
-template <bool VEC>
+// VEC: four pixels per thread. COPY: the projections are also copied, to be filtered from there into their
+// places: MedianMixRingClean on 180 x 500 x 750 (mean 62 us, filter out of place 394, copy back 92) takes
+// 93 us for this pass and has no copy back.
+template <bool VEC, bool COPY>
 __global__ void __launch_bounds__(256) k_mean_projection(const float *__restrict__ proj, size_t npix, size_t nproj,
-                                                         int from_zero, float scale, float *__restrict__ mean)
+                                                         int from_zero, float scale, float *__restrict__ mean,
+                                                         float *__restrict__ copy)
 {
     if constexpr (VEC) {
         const size_t j = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
@@ -463,11 +466,13 @@ __global__ void __launch_bounds__(256) k_mean_projection(const float *__restrict
         size_t i = 0;
         if (!from_zero) {
             acc = __ldg(reinterpret_cast<const float4 *>(proj + j));
+            if (COPY) *reinterpret_cast<float4 *>(copy + j) = acc;
             i = 1;
         }
 #pragma unroll 8
         for (; i < nproj; ++i) {
             const float4 v = __ldg(reinterpret_cast<const float4 *>(proj + i * npix + j));
+            if (COPY) *reinterpret_cast<float4 *>(copy + i * npix + j) = v;
             acc.x = __fadd_rn(acc.x, v.x);
             acc.y = __fadd_rn(acc.y, v.y);
             acc.z = __fadd_rn(acc.z, v.z);
@@ -485,10 +490,15 @@ __global__ void __launch_bounds__(256) k_mean_projection(const float *__restrict
         size_t i = 0;
         if (!from_zero) {
             acc = __ldg(proj + j);
+            if (COPY) copy[j] = acc;
             i = 1;
         }
 #pragma unroll 8
-        for (; i < nproj; ++i) acc = __fadd_rn(acc, __ldg(proj + i * npix + j));
+        for (; i < nproj; ++i) {
+            const float v = __ldg(proj + i * npix + j);
+            if (COPY) copy[i * npix + j] = v;
+            acc = __fadd_rn(acc, v);
+        }
         mean[j] = __fmul_rn(acc, scale);
     }
 }
@@ -617,15 +627,15 @@ static bool median_size_ok(size_t w, size_t h, int kx, int ky)
            w >= static_cast<size_t>(2 * (kx / 2)) && h >= static_cast<size_t>(2 * (ky / 2));
 }
 
-static mr_status mean_projection(const float *proj, size_t npix, size_t nproj, int from_zero, float *mean,
+// Mean projection; copy: null, or nproj projections to copy them to.
+static mr_status mean_projection(const float *proj, size_t npix, size_t nproj, int from_zero, float *mean, float *copy,
                                  cudaStream_t s)
 {
     const float scale = 1.0f / static_cast<float>(nproj);
-    const bool vec = npix % 4 == 0 && reinterpret_cast<uintptr_t>(proj) % 16 == 0;
-    if (vec)
-        ringalt::k_mean_projection<true><<<div_up(npix / 4, 256), 256, 0, s>>>(proj, npix, nproj, from_zero, scale, mean);
-    else
-        ringalt::k_mean_projection<false><<<div_up(npix, 256), 256, 0, s>>>(proj, npix, nproj, from_zero, scale, mean);
+    const bool vec = npix % 4 == 0 && (reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(copy)) % 16 == 0;
+    const auto kernel = vec ? (copy ? ringalt::k_mean_projection<true, true> : ringalt::k_mean_projection<true, false>)
+                            : (copy ? ringalt::k_mean_projection<false, true> : ringalt::k_mean_projection<false, false>);
+    kernel<<<div_up(vec ? npix / 4 : npix, 256), 256, 0, s>>>(proj, npix, nproj, from_zero, scale, mean, copy);
     return check_launch("k_mean_projection");
 }
 
@@ -673,7 +683,7 @@ mr_status mr_basicringclean(float *proj_d, size_t nu, size_t nv, size_t nproj, v
     float *work = nullptr;
     MR_TRY(device_alloc(&work, 2 * npix * sizeof(float), s, "mr_basicringclean: scratch"));
     float *mean = work, *diff = work + npix;
-    mr_status st = mean_projection(proj_d, npix, nproj, 0, mean, s);
+    mr_status st = mean_projection(proj_d, npix, nproj, 0, mean, nullptr, s);
     if (st == MR_OK)
         st = launch_median<ringalt::MODE_DIFF>(mean, static_cast<int>(nu), static_cast<int>(nv), 1, 3, 3, nullptr,
                                                diff, s);
@@ -706,7 +716,8 @@ mr_status mr_medianmixringclean(float *proj_d, size_t nu, size_t nv, size_t npro
     const size_t npix = nu * nv, len = 1024;
     std::vector<float> table(len + 4);
     sigmoid_lut(len, threshold, width, table.data(), table.data() + len);
-    // batch of projections filtered out of place: about 512 MiB
+    // projections are filtered out of place, about 512 MiB at a time: the mean's pass copies a block of that
+    // size, which is filtered into its place; of a larger one each batch is copied back
     const size_t batch = std::max<size_t>(1, std::min<size_t>(nproj, (size_t(1) << 27) / npix));
     float *work = nullptr;
     MR_TRY(device_alloc(&work, (2 * npix + len + 4 + batch * npix) * sizeof(float), s, "mr_medianmixringclean: scratch"));
@@ -714,7 +725,7 @@ mr_status mr_medianmixringclean(float *proj_d, size_t nu, size_t nv, size_t npro
     mr_status st = MR_OK;
     cudaError_t e = cudaMemcpyAsync(lut, table.data(), table.size() * sizeof(float), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) st = fail(MR_ERR_CUDA, "mr_medianmixringclean: table upload: %s", cudaGetErrorString(e));
-    if (st == MR_OK) st = mean_projection(proj_d, npix, nproj, 1, mean, s);
+    if (st == MR_OK) st = mean_projection(proj_d, npix, nproj, 1, mean, batch == nproj ? out : nullptr, s);
     if (st == MR_OK)
         st = launch_median<ringalt::MODE_ABSDIFF>(mean, static_cast<int>(nu), static_cast<int>(nv), 1, pkx, pky,
                                                   nullptr, wt, s);
@@ -722,7 +733,9 @@ mr_status mr_medianmixringclean(float *proj_d, size_t nu, size_t nv, size_t npro
         ringalt::k_lut<<<div_up(npix, 256), 256, 0, s>>>(wt, npix, lut, static_cast<int>(len));
         st = check_launch("k_lut");
     }
-    for (size_t i0 = 0; i0 < nproj && st == MR_OK; i0 += batch) {
+    if (st == MR_OK && batch == nproj)
+        st = launch_median<ringalt::MODE_MIX>(out, static_cast<int>(nu), static_cast<int>(nv), nproj, 5, mky, wt, proj_d, s);
+    for (size_t i0 = 0; i0 < nproj && batch < nproj && st == MR_OK; i0 += batch) {
         const size_t b = std::min(batch, nproj - i0);
         float *p = proj_d + i0 * npix;
         st = launch_median<ringalt::MODE_MIX>(p, static_cast<int>(nu), static_cast<int>(nv), b, 5, mky, wt, out, s);
