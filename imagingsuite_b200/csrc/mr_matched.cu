@@ -35,7 +35,7 @@ static const float kFPi = 3.1415926535897932384626f;
 MR_BOUNDS_TAKE(bounds_take_matched)
 
 // The adjoint with its projection rows staged in shared memory by TMA, as the production backprojector
-// (mr_bp_tma.cu): a CTA owns 32 (x) x 8 (y) voxel columns x 32 slices, a thread one column's 32 slices in
+// (mr_bp_tma.cu): a CTA owns 32 (x) x 8 or 4 (y) voxel columns x 32 slices, a thread one column's 32 slices in
 // registers over all projections. Each slice has its own position (the detector centre moves with it):
 // u is affine in x, y and, through the slice centre, z, so its floor is extreme at the tile's corners;
 // a projection's box of 48 columns x 32 slices starts at most four columns before the smallest (the TMA
@@ -47,9 +47,8 @@ MR_BOUNDS_TAKE(bounds_take_matched)
 // sums. Slices go in pairs through the paired FP32 pipe (products as fmas with a -0 addend the compiler
 // cannot see, so that they are not contracted with their sum), the floor from the bits of u + 1.5 * 2^23
 // added rounding down, and boxes come by one instruction of one thread instead of 48 cp.async per thread
-// and batch: 256^2 x 64 slices from 180 projections 1061 -> 602 us.
-constexpr int kAdjTX = 32, kAdjTY = 8, kAdjTZ = 32, kAdjNB = 8, kAdjBW = 48;
-constexpr int kAdjThreads = kAdjTX * kAdjTY, kAdjCtas = 2;
+// and batch: 256^2 x 64 slices from 180 projections 1061 -> 605 us, 564 in shorter tiles (launch_adjoint).
+constexpr int kAdjTX = 32, kAdjTZ = 32, kAdjBW = 48;
 constexpr int kAdjBox = kAdjBW * kAdjTZ;     // floats
 constexpr int kAdjGeo = kAdjTZ + 4;          // slice start positions, sin, cos, pad
 constexpr float kAdjMagic = 12582912.0f;     // 1.5 * 2^23
@@ -57,9 +56,9 @@ constexpr int kAdjMagicBits = 0x4B400000;
 // how a tile reads a projection: footprint beyond the box, nothing, staged, staged and on the detector
 enum { kAdjUnfit, kAdjNothing, kAdjStaged, kAdjClean };
 
-__host__ __device__ constexpr size_t adj_smem_bytes()
+__host__ __device__ constexpr size_t adj_smem_bytes(int nb)
 {
-    return sizeof(float) * (2ull * kAdjNB * kAdjBox + 3ull * kAdjNB * kAdjGeo) + sizeof(int2) * 2 * kAdjNB + 2 * sizeof(uint64_t);
+    return sizeof(float) * (2ull * nb * kAdjBox + 3ull * nb * kAdjGeo) + sizeof(int2) * 2 * nb + 2 * sizeof(uint64_t);
 }
 
 struct AdjParams {
@@ -83,17 +82,19 @@ int mbp_device_status_take()
     return v;
 }
 
-__global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(const __grid_constant__ CUtensorMap tmap,
+// Tiles of 32 x TY columns, batches of NB projections.
+template <int TY, int NB, int CTAS>
+__global__ void __launch_bounds__(kAdjTX * TY, CTAS) k_mbp_adjoint_staged(const __grid_constant__ CUtensorMap tmap,
                                                                               const AdjParams P)
 {
     extern __shared__ __align__(1024) float adj_smem[];
     float *box = adj_smem;                                          // [2][NB][TZ][BW]
-    float *geo = box + 2 * kAdjNB * kAdjBox;                        // [3][NB][kAdjGeo]
-    int2 *meta = reinterpret_cast<int2 *>(geo + 3 * kAdjNB * kAdjGeo); // [2][NB]: first staged column, mode
-    uint64_t *bars = reinterpret_cast<uint64_t *>(meta + 2 * kAdjNB);
+    float *geo = box + 2 * NB * kAdjBox;                        // [3][NB][kAdjGeo]
+    int2 *meta = reinterpret_cast<int2 *>(geo + 3 * NB * kAdjGeo); // [2][NB]: first staged column, mode
+    uint64_t *bars = reinterpret_cast<uint64_t *>(meta + 2 * NB);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = P.n, nz = P.nz;
-    const int x0 = blockIdx.x * kAdjTX, y0 = blockIdx.y * kAdjTY, z0 = blockIdx.z * kAdjTZ;
+    const int x0 = blockIdx.x * kAdjTX, y0 = blockIdx.y * TY, z0 = blockIdx.z * kAdjTZ;
     const int x1 = x0 + lane + 1, y1 = y0 + warp + 1; // 1-based voxel
     const bool valid = x1 <= n && y1 <= n;
     const bool inside = valid && static_cast<uint32_t>(x1) > P.mask[2 * (y1 - 1)] &&
@@ -106,8 +107,8 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(co
         const float v = (P.accumulate && inside && c < zmax) ? col[c] : 0.0f;
         if (c & 1) acc[c >> 1].y = v; else acc[c >> 1].x = v;
     }
-    const int nbatch = (P.nproj + kAdjNB - 1) / kAdjNB;
-    const int xa = x0 + 1, xb = min(x0 + kAdjTX, n), ya = y0 + 1, yb = min(y0 + kAdjTY, n);
+    const int nbatch = (P.nproj + NB - 1) / NB;
+    const int xa = x0 + 1, xb = min(x0 + kAdjTX, n), ya = y0 + 1, yb = min(y0 + TY, n);
     const bool any = __syncthreads_or(inside);
     if (threadIdx.x == 0) {
         tma::mbar_init(&bars[0], 1);
@@ -118,20 +119,20 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(co
     // geometry of batch s into buffer gb; slices past the volume repeat the last one, projections past
     // the list the first
     auto stage_geometry = [&](int s, int gb) {
-        for (int e = threadIdx.x; e < kAdjNB * (kAdjTZ + 2); e += kAdjThreads) {
-            const int b = e / (kAdjTZ + 2), c = e - b * (kAdjTZ + 2), i = s * kAdjNB + b < P.nproj ? s * kAdjNB + b : 0;
+        for (int e = threadIdx.x; e < NB * (kAdjTZ + 2); e += kAdjTX * TY) {
+            const int b = e / (kAdjTZ + 2), c = e - b * (kAdjTZ + 2), i = s * NB + b < P.nproj ? s * NB + b : 0;
             const float *src = c < kAdjTZ ? P.startu + static_cast<size_t>(i) * nz + min(z0 + c, nz - 1)
                                           : reinterpret_cast<const float *>(P.sc + i) + (c - kAdjTZ);
-            tma::copy4_zfill(geo + (gb * kAdjNB + b) * kAdjGeo + c, src, true);
+            tma::copy4_zfill(geo + (gb * NB + b) * kAdjGeo + c, src, true);
         }
     };
     // batch s (geometry in buffer gb) into stage st: windows from 8 corner lanes per projection
     auto issue = [&](int s, int st, int gb) {
         if (warp != 0) return;
 #pragma unroll 1
-        for (int r = 0; r < kAdjNB; r += 4) {
-            const int b = r + (lane >> 3), corner = lane & 7, i = s * kAdjNB + b;
-            const float *g = geo + (gb * kAdjNB + b) * kAdjGeo;
+        for (int r = 0; r < NB; r += 4) {
+            const int b = r + (lane >> 3), corner = lane & 7, i = s * NB + b;
+            const float *g = geo + (gb * NB + b) * kAdjGeo;
             const float fx = static_cast<float>((corner & 1) ? xb : xa), fy = static_cast<float>((corner & 2) ? yb : ya);
             const float u = __fsub_rn(__fadd_rn(g[(corner & 4) ? zmax - 1 : 0], __fmul_rn(g[kAdjTZ + 1], fy)),
                                       __fmul_rn(g[kAdjTZ], fx));
@@ -152,14 +153,14 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(co
             const bool head = corner == 0, load = head && mode >= kAdjStaged;
             const uint32_t bytes = __popc(__ballot_sync(0xffffffffu, load)) * kAdjBox * sizeof(float);
             if (lane == 0) { // the phase completes on the last round's arrival
-                if (r + 4 < kAdjNB) tma::mbar_add_tx(&bars[st], bytes);
+                if (r + 4 < NB) tma::mbar_add_tx(&bars[st], bytes);
                 else tma::mbar_expect_tx(&bars[st], bytes);
             }
             __syncwarp();
-            if (head) meta[st * kAdjNB + b] = make_int2(w0, mode);
+            if (head) meta[st * NB + b] = make_int2(w0, mode);
             if (load) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tma::load_3d(box + (st * kAdjNB + b) * kAdjBox, &tmap, w0, z0, i, &bars[st]);
+                tma::load_3d(box + (st * NB + b) * kAdjBox, &tmap, w0, z0, i, &bars[st]);
             }
         }
     };
@@ -188,12 +189,12 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(co
         }
         if (got && inside) {
 #pragma unroll 1
-            for (int b = 0; b < kAdjNB && s * kAdjNB + b < P.nproj; ++b) {
-                const int2 m = meta[st * kAdjNB + b];
+            for (int b = 0; b < NB && s * NB + b < P.nproj; ++b) {
+                const int2 m = meta[st * NB + b];
                 if (m.y == kAdjNothing) continue;
-                const float *g = geo + (gb * kAdjNB + b) * kAdjGeo;
+                const float *g = geo + (gb * NB + b) * kAdjGeo;
                 const float cy = __fmul_rn(g[kAdjTZ + 1], fy), sx = __fmul_rn(g[kAdjTZ], fx);
-                const float *bx = box + (st * kAdjNB + b) * kAdjBox;
+                const float *bx = box + (st * NB + b) * kAdjBox;
                 if (m.y == kAdjClean) {
                     const float2 cy2 = make_float2(cy, cy), sx2 = make_float2(-sx, -sx);
                     const int base = -kAdjMagicBits - m.x;
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjCtas) k_mbp_adjoint_staged(co
                     continue;
                 }
                 // edges of the detector, or a footprint beyond the box: slice by slice
-                const float *img = P.proj + (static_cast<size_t>(s * kAdjNB + b) * nz + z0) * P.pitch;
+                const float *img = P.proj + (static_cast<size_t>(s * NB + b) * nz + z0) * P.pitch;
 #pragma unroll
                 for (int c = 0; c < kAdjTZ; ++c) {
                     const float u = __fsub_rn(__fadd_rn(g[c], cy), sx);
@@ -286,12 +287,19 @@ static mr_status launch_adjoint(AdjParams P, int width, cudaStream_t s)
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) return fail(MR_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(cr));
     }
-    MR_CUDA_TRY(cudaFuncSetAttribute(k_mbp_adjoint_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(adj_smem_bytes())));
-    const dim3 grid(div_up(static_cast<size_t>(P.n), kAdjTX), div_up(static_cast<size_t>(P.n), kAdjTY),
-                    div_up(static_cast<size_t>(P.nz), kAdjTZ));
-    k_mbp_adjoint_staged<<<grid, kAdjThreads, adj_smem_bytes(), s>>>(map, P);
-    return check_launch("k_mbp_adjoint_staged");
+    // 32 x 8 columns, two CTAs per SM, while these fill the last wave; else 32 x 4, whose shorter CTAs even it
+    // out for up to 3 % more work: 256^2 x 64 slices from 180 projections (512 CTAs on 296 places) 605 -> 561
+    // us, 64^2 x 8 from 60 79 -> 73, but 192^2 x 64 from 360 (288 CTAs) 795 -> 817
+    const size_t across = div_up(static_cast<size_t>(P.n), kAdjTX), deep = div_up(static_cast<size_t>(P.nz), kAdjTZ);
+    const size_t tiles = across * div_up(static_cast<size_t>(P.n), 8) * deep, places = 2 * 148;
+    auto launch = [&](auto kernel, int ty, int nb) -> mr_status {
+        MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(adj_smem_bytes(nb))));
+        const dim3 grid(static_cast<unsigned>(across), div_up(static_cast<size_t>(P.n), ty), static_cast<unsigned>(deep));
+        kernel<<<grid, kAdjTX * ty, adj_smem_bytes(nb), s>>>(map, P);
+        return check_launch("k_mbp_adjoint_staged");
+    };
+    if (20 * tiles < 19 * places * div_up(tiles, places)) return launch(k_mbp_adjoint_staged<4, 4, 4>, 4, 4);
+    return launch(k_mbp_adjoint_staged<8, 8, 2>, 8, 8);
 }
 
 // Forward projection. Both kernels walk lines of voxels along the axis on which u changes least (x when
@@ -724,7 +732,7 @@ mr_status mr_mbp_adjoint(const float *proj_d, size_t n, size_t nz, const float *
     }
     // padded copies, a run of projections (64 MiB of scratch) at a time; the volume carries the sums
     const size_t pitch = std::max<size_t>(kAdjBW, (n + 3) / 4 * 4), per = nz * pitch;
-    const size_t run = std::min(nproj, std::max<size_t>(kAdjNB, (size_t(64) << 20) / (per * 4)));
+    const size_t run = std::min(nproj, std::max<size_t>(8, (size_t(64) << 20) / (per * 4)));
     float *scratch = nullptr;
     if (device_alloc(&scratch, run * per * sizeof(float), s, "mr_mbp_adjoint: padded projections") != MR_OK) {
         P.proj = proj_d; // no room for copies

@@ -15,7 +15,7 @@ from imagingsuite_b200 import joseph as J
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,nz", [(17, 4), (31, 36), (47, 32), (48, 8), (50, 40), (63, 68), (64, 33), (97, 32)])
+@pytest.mark.parametrize("n,nz", [(17, 4), (31, 36), (47, 32), (48, 8), (50, 40), (63, 68), (64, 33), (97, 32), (190, 36)])
 @pytest.mark.parametrize("tilt,shift", [(0.4, 0.2), (-0.9, 17.3), (35.0, 0.0)])
 def test_adjoint_bit_exact(cuda, n, nz, tilt, shift):
     rng = np.random.default_rng(n * nz)
