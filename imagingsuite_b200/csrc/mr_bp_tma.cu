@@ -65,7 +65,7 @@ enum Mode { kLinear, kNearest, kTilt, kTiltSerial, kTiltNearest };
 
 // How a tile reads one projection: its footprint does not fit the box (guarded global loads), no
 // voxel of the tile lies on the detector, staged, staged with every voxel of the tile on the detector
-// and cos away from +-1 (n of neighbouring rows is then the same or one apart).
+// and n of neighbouring rows the same or one apart (rows_share).
 enum Footprint { kUnfit, kNothing, kStaged, kClean };
 
 struct Params {
@@ -112,6 +112,19 @@ __device__ __forceinline__ float posu(float sn, float cs, float su, float fx, fl
     const float u = __fsub_rn(local, __fmul_rn(sn, fx));
     if constexpr (MODE == kTiltSerial || MODE == kTiltNearest) return __fsub_rn(u, toff);
     return u;
+}
+
+// Are n(x, y) and n(x, y + 1) at most one apart? u changes by cos between the two, plus the rounding of
+// cos y, of the sum and of the differences that follow, half a step of each value per row (sin x is the
+// same value in both). The values' sum is convex in x and y, so that of the tile's corners bounds it. At
+// 2048 columns |cos| may reach 0.999, at 65536 columns 0.97.
+template <int MODE>
+__device__ __forceinline__ bool rows_share(float cs, float su, float fy, float toff, float u)
+{
+    const float cy = cs * fy;
+    float values = fabsf(cy) + fabsf(su + cy) + fabsf(u);
+    if constexpr (MODE == kTilt || MODE == kTiltSerial || MODE == kTiltNearest) values += fabsf(su + cy) + fabsf(u) + 2.0f * fabsf(toff);
+    return fabsf(cs) + 1.25f * 0x1p-23f * values < 1.0f;
 }
 
 // Two slices of acc += pa * wa + pb * wb in the reference's order, every product and sum rounded on
@@ -280,20 +293,20 @@ __global__ void __launch_bounds__(32 * NW, CTAS) k_bp_par_staged(const __grid_co
             const int i = s * NB + b;
             const float *g = S.geo + (gb * NB + (b < NB ? b : 0)) * GEO;
             int nmin = 0, nmax = 0;
-            bool ok = b < NB && i < P.nproj, positive = true;
+            bool ok = b < NB && i < P.nproj, pairs = true;
             if (ok) {
-                const float u = posu<MODE>(g[0], g[1], g[2], static_cast<float>((corner & 1) ? xb : xa),
-                                           static_cast<float>((corner & 2) ? yb : ya), P.toff);
+                const float fy = static_cast<float>((corner & 2) ? yb : ya);
+                const float u = posu<MODE>(g[0], g[1], g[2], static_cast<float>((corner & 1) ? xb : xa), fy, P.toff);
                 ok = fabsf(u) < 1.0e9f;
                 nmin = nmax = ok ? __float2int_rz(u) : 0;
-                positive = u >= 0.0f;
+                pairs = u >= 0.0f && rows_share<MODE>(g[1], g[2], fy, P.toff, u);
             }
 #pragma unroll
             for (int o = 1; o < 4; o <<= 1) {
                 nmin = min(nmin, __shfl_xor_sync(0xffffffffu, nmin, o));
                 nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
                 ok = __shfl_xor_sync(0xffffffffu, static_cast<int>(ok), o) && ok;
-                positive = __shfl_xor_sync(0xffffffffu, static_cast<int>(positive), o) && positive;
+                pairs = __shfl_xor_sync(0xffffffffu, static_cast<int>(pairs), o) && pairs;
             }
             int mode = kUnfit, x0 = 0;
             if (ok) {
@@ -301,7 +314,7 @@ __global__ void __launch_bounds__(32 * NW, CTAS) k_bp_par_staged(const __grid_co
                     mode = kNothing;
                 } else {
                     x0 = nmin >= 0 ? (nmin & ~3) : -(((-nmin) + 3) & ~3);
-                    if (nmax + 1 < x0 + BW) mode = positive && nmax <= P.nu - 2 && fabsf(g[1]) < 0.999f ? kClean : kStaged;
+                    if (nmax + 1 < x0 + BW) mode = pairs && nmax <= P.nu - 2 ? kClean : kStaged;
                 }
             }
             const unsigned staged = __ballot_sync(0xffffffffu, corner == 0 && mode >= kStaged);
