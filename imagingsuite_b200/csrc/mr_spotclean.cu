@@ -108,7 +108,7 @@ __global__ void k_range_init(int n, int *__restrict__ mn, int *__restrict__ mx)
 
 // Padded image (MorphSpotClean::PadEdges :264-281) after replaceInfNaN (:514-536) and
 // LimitDynamics (core/kipl/kipl/include/segmentation/thresholds.h:60-85), and the image's range as
-// keys (NaN ignored; mn null: not asked for). The edge medians that follow change rows 0 and ph - 1 only, within the range of
+// keys (NaN ignored). The edge medians that follow change rows 0 and ph - 1 only, within the range of
 // those rows' samples, which rows 9 and ph - 10 hold too, so the range is theirs as well.
 __global__ void __launch_bounds__(256) k_pad(const float *__restrict__ img, int w, int h, const float *__restrict__ finite_max, int clamp,
                       float lo, float hi, float *__restrict__ pad, int *__restrict__ mn, int *__restrict__ mx)
@@ -138,7 +138,6 @@ __global__ void __launch_bounds__(256) k_pad(const float *__restrict__ img, int 
             z = fmaxf(z, v);
         }
     }
-    if (!mn) return; // uniform
     __shared__ int ra[8], rz[8];
     const int ka = __reduce_min_sync(0xffffffffu, fkey(a)), kz = __reduce_max_sync(0xffffffffu, fkey(z));
     if ((threadIdx.x & 31) == 0) {
@@ -477,7 +476,9 @@ __global__ void k_band_into(const float *__restrict__ band, int pw, int ph, floa
 //     third.
 //
 // Every value is a maximum or minimum of pixel values: the result is the unique reconstruction, the
-// reference's bit for bit (NaN counts as the lowest height). There are no chains of dependent
+// reference's bit for bit. Its comparisons are false for a NaN, which leaves such a pixel as it is and
+// lets no path through: its height is kWall, above every other. A region whose level is not below that
+// is shut in by such pixels; there the marker stays, the image's maximum (k_replace). There are no chains of dependent
 // relaxations along paths: the work is full passes of 8 bytes per pixel while components are smaller
 // than a tile, then only over tiles that still hold a boundary.
 //
@@ -514,14 +515,13 @@ struct Flood {
     __device__ __forceinline__ u64 *best(int round) const { return round & 1 ? best1 : best0; }
 };
 
-// Height of a pixel: its key, or its negation's (the complement, flip -1); NaN stays the lowest.
-__device__ __forceinline__ int height(int key, int flip)
-{
-    const int h = key ^ flip;
-    return h == INT_MAX ? INT_MIN : h;
-}
+constexpr int kWall = 0x7F800001; // height of a NaN (key INT_MIN, see k_to_keys), above +inf's
 
-// Height at which the ocean enters pixel (x, y) of height gp; INT_MAX: not here.
+// Height of a pixel: its key, or its negation's (the complement, flip -1).
+__device__ __forceinline__ int height(int key, int flip) { return key == INT_MIN ? kWall : key ^ flip; }
+
+// Height at which the ocean enters pixel (x, y) of height gp; INT_MAX: not here. (Not below kWall at a
+// NaN, whose band value is a NaN too.)
 __device__ __forceinline__ int ocean_height(const Flood &F, int job, int img, int x, int y, int gp)
 {
     if (!F.band) return x == 0 || y == 0 || x == F.pw - 1 || y == F.ph - 1 ? gp : INT_MAX;
@@ -560,8 +560,7 @@ __device__ __forceinline__ bool strip_of(const Flood &F, int u, int task, Strip 
     return true;
 }
 
-// The padded images as keys, in place; NaN, which the reference's comparisons skip, as the lowest (its
-// float is a NaN again).
+// The padded images as keys, in place; a NaN of any bits as INT_MIN (whose float is a NaN again).
 __global__ void __launch_bounds__(256) k_to_keys(float *__restrict__ pad, size_t n)
 {
     int *key = reinterpret_cast<int *>(pad);
@@ -925,10 +924,25 @@ struct RecJobs {
 // in 32 different banks. Positions beyond the row hold the neutral value (-inf for
 // dilation, +inf for erosion), which neither propagates into the row nor changes.
 
+//
+// A NaN of the mask takes and passes on nothing, as in the reference, whose comparisons it fails: the
+// outer operation keeps it, the inner one takes the other operand.
 template <bool DILATE>
 __device__ __forceinline__ float rec_op(float g, float v, float x)
 {
-    return DILATE ? fminf(g, fmaxf(v, x)) : fmaxf(g, fminf(v, x));
+    const float inner = DILATE ? fmaxf(v, x) : fminf(v, x);
+    float r;
+    if (DILATE) asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(g), "f"(inner));
+    else asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(g), "f"(inner));
+    return r;
+}
+
+// Key of a mask or marker value; of a NaN the one that improves no neighbour and that nothing improves.
+// (The NaN that arithmetic makes, as in sign * g and rec_op, is 0x7FFFFFFF: its fkey is INT_MAX.)
+template <bool DILATE>
+__device__ __forceinline__ int rec_key(float v)
+{
+    return DILATE && v != v ? INT_MIN : fkey(v);
 }
 
 __device__ __forceinline__ void cp_async4(float *dst, const float *src)
@@ -1137,7 +1151,7 @@ __global__ void __launch_bounds__(32 * RW) k_reconstruct(const float *__restrict
             const size_t ro = static_cast<size_t>(y) * pw;
             if constexpr (LAST) {
                 int *vk = reinterpret_cast<int *>(v);
-                for (int c = t; c < pw; c += T) vk[ro + c] = fkey(V[1 + c]);
+                for (int c = t; c < pw; c += T) vk[ro + c] = rec_key<DILATE>(V[1 + c]);
             } else {
                 for (int c = t; c < pw; c += T) v[ro + c] = V[1 + c];
             }
@@ -1169,7 +1183,7 @@ __global__ void __launch_bounds__(32 * RW) k_reconstruct(const float *__restrict
     if (!keys) {
         // converged before the last round: nothing to list; store the marker as keys
         int *vk = reinterpret_cast<int *>(v);
-        for (size_t i = t; i < n; i += T) vk[i] = fkey(__int_as_float(vk[i]));
+        for (size_t i = t; i < n; i += T) vk[i] = rec_key<DILATE>(__int_as_float(vk[i]));
     }
     if (t == 0) counts[blockIdx.x] = listed; // the pushes precede the barriers of the last vote
 }
@@ -1263,7 +1277,7 @@ __global__ void __launch_bounds__(kFrontThreads) k_complete(const float *__restr
                         const int kq = __ldcg(v + qy * pw + qx);
                         kn = DILATE ? max(kn, kq) : min(kn, kq);
                     }
-                    const int kg = i < n ? fkey(sign * __ldg(g + i)) : 0;
+                    const int kg = i < n ? rec_key<DILATE>(sign * __ldg(g + i)) : 0;
                     c[u] = DILATE ? min(kg, kn) : max(kg, kn);
                     kv[u] = i < n ? __ldcg(v + i) : c[u];
                 }
@@ -1295,7 +1309,7 @@ __global__ void __launch_bounds__(kFrontThreads) k_complete(const float *__restr
                         const int qx = x + nx[k], qy = y + ny[k];
                         const bool in = qx >= 0 && qx < pw && qy >= 0 && qy < ph;
                         const int q = qy * pw + qx;
-                        const int kg = in ? fkey(sign * __ldg(g + q)) : 0;
+                        const int kg = in ? rec_key<DILATE>(sign * __ldg(g + q)) : 0;
                         kv[k] = in ? __ldcg(v + q) : 0;
                         c[k] = DILATE ? min(kg, kp) : max(kg, kp);
                         if (in && improves(c[k], kv[k])) ok |= 1u << k;
@@ -1364,7 +1378,9 @@ static mr_status launch_reconstruct(const RecJobs &jobs, int njobs, const float 
 // kipl::math::SigmoidWeights mathfunctions.hpp:92-99).
 template <bool LEVELS>
 __global__ void k_replace(const void *__restrict__ pad, const int *__restrict__ hole_lab, const int *__restrict__ hole_lev,
-                          const int *__restrict__ peak_lab, const int *__restrict__ peak_lev, size_t cap, int w, int h, int detect, float th0, float th1, float s0, float s1, float *__restrict__ img)
+                          const int *__restrict__ peak_lab, const int *__restrict__ peak_lev, size_t cap,
+                          const int *__restrict__ mn, const int *__restrict__ mx, int w, int h, int detect, float th0,
+                          float th1, float s0, float s1, float *__restrict__ img)
 {
     const int pw = w + 2 * kMargin, ph = h + 2 * kMargin;
     const size_t n = static_cast<size_t>(pw) * ph;
@@ -1375,13 +1391,20 @@ __global__ void k_replace(const void *__restrict__ pad, const int *__restrict__ 
         const size_t idx = static_cast<size_t>(y) * w + x;
         const size_t pi = b * n + static_cast<size_t>(y + kMargin) * pw + x + kMargin;
         // LEVELS: the image as keys, a reconstruction the larger of the pixel and its basin's level (peaks:
-        // of the negated image); else reconstructions stored as keys (peaks alone: of the image itself)
+        // of the negated image), or the marker where no path leads; else reconstructions stored as keys
+        // (peaks alone: of the image itself)
         float val, hv = 0.0f, pv = 0.0f;
         if (LEVELS) {
             const int key = static_cast<const int *>(pad)[pi];
             val = funkey(key);
-            if (hole_lab) hv = funkey(max(height(key, 0), hole_lev[b * cap + ~hole_lab[pi]]));
-            if (peak_lab) pv = -funkey(max(height(key, -1), peak_lev[b * cap + ~peak_lab[pi]]));
+            if (hole_lab) {
+                const int rec = max(height(key, 0), hole_lev[b * cap + ~hole_lab[pi]]);
+                hv = funkey(rec < kWall ? rec : mx[b]);
+            }
+            if (peak_lab) {
+                const int rec = max(height(key, -1), peak_lev[b * cap + ~peak_lab[pi]]);
+                pv = rec < kWall ? -funkey(rec) : funkey(mn[b]);
+            }
         } else {
             val = static_cast<const float *>(pad)[pi];
             if (hole_lab) hv = funkey(hole_lab[pi]);
@@ -1477,10 +1500,8 @@ mr_status mr_morphspotclean(float *proj_d, size_t nu, size_t nv, size_t nproj, i
         int *peak_lab = jobs == 2 ? F.lab1 : F.lab0;
         float *H = reinterpret_cast<float *>(F.lab0), *K = reinterpret_cast<float *>(peak_lab);
         if (removeinfnan) k_finite_max<<<nb, 256, 0, s>>>(img, nu * nv, fmax);
-        const bool range = !flood || detect == 1;
-        if (range) k_range_init<<<div_up(nb, 256), 256, 0, s>>>(nb, mn, mx);
-        k_pad<<<dim3(gx, nb), 256, 0, s>>>(img, w, h, removeinfnan ? fmax : nullptr, clamp, minlevel, maxlevel, P,
-                                           range ? mn : nullptr, mx);
+        k_range_init<<<div_up(nb, 256), 256, 0, s>>>(nb, mn, mx);
+        k_pad<<<dim3(gx, nb), 256, 0, s>>>(img, w, h, removeinfnan ? fmax : nullptr, clamp, minlevel, maxlevel, P, mn, mx);
         k_edge_median<<<2 * nb, 32, pw * sizeof(float), s>>>(P, pw, ph, edge);
         if (detect == 1) { // the forward scan's border band; the rest of the marker is the minimum
             const size_t smem = (8 * static_cast<size_t>(ph) + 2 * static_cast<size_t>(pw)) * sizeof(float);
@@ -1515,11 +1536,11 @@ mr_status mr_morphspotclean(float *proj_d, size_t nu, size_t nv, size_t nproj, i
         if (st != MR_OK) break;
         const int *hole_lab = detect != 1 ? F.lab0 : nullptr, *peaks = detect != 0 ? peak_lab : nullptr;
         if (flood)
-            k_replace<true><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, F.lev, peaks, F.lev + (jobs - 1) * nb * cap, cap, w, h,
-                                                         detect, th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
+            k_replace<true><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, F.lev, peaks, F.lev + (jobs - 1) * nb * cap, cap, mn,
+                                                         mx, w, h, detect, th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
         else
-            k_replace<false><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, nullptr, peaks, nullptr, 0, w, h, detect, th_h[0],
-                                                          th_h[1], sigma_h[0], sigma_h[1], img);
+            k_replace<false><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, nullptr, peaks, nullptr, 0, mn, mx, w, h, detect,
+                                                          th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
         st = check_launch("k_replace");
     }
     cudaFreeAsync(scratch, s);
