@@ -1396,6 +1396,7 @@ __global__ void k_replace(const void *__restrict__ pad, const int *__restrict__ 
         float val, hv = 0.0f, pv = 0.0f;
         if (LEVELS) {
             const int key = static_cast<const int *>(pad)[pi];
+            if (key == INT_MIN) continue; // a NaN stays, with its bits
             val = funkey(key);
             if (hole_lab) {
                 const int rec = max(height(key, 0), hole_lev[b * cap + ~hole_lab[pi]]);

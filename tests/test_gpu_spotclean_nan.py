@@ -61,3 +61,12 @@ def test_few_equal_many(cuda, detect, edge):
     few = _clean(img, detect, True, edge)
     many = _clean(np.resize(img, (MANY, 40, 52)), detect, True, edge)
     assert np.array_equal(many, np.resize(few, many.shape), equal_nan=True)
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_nan_bits_stay(cuda, many):
+    bits = np.array([0x7FC00001, 0xFFC12345, 0x7F800001, 0xFFFFFFFF, 0x7FFFFFFF], np.uint32)
+    img = np.random.default_rng(4).standard_normal((1, 20, 30)).astype(np.float32)
+    img.view(np.uint32)[0, 7, 3:28:5] = bits
+    got = _clean(np.repeat(img, MANY if many else 1, axis=0), "both", True, 5)
+    assert np.array_equal(got[-1].view(np.uint32)[7, 3:28:5], bits)
