@@ -20,7 +20,7 @@
 // is replayed over that band (k_peaks_band_smem), and the exact reconstruction follows.
 //
 // Few images are reconstructed by merging basins over the whole GPU (k_descend and following), many
-// (kFloodUnits) by sweeps and a worklist, one CTA per image:
+// (few_units) by sweeps and a worklist, one CTA per image:
 //
 // Each reconstruction runs in two kernels, one CTA per image in both. The sweep kernel
 // alternates downward and upward row sweeps for a few rounds (it stops early when a round
@@ -61,12 +61,23 @@ namespace msc {
 constexpr int kMargin = 5;
 constexpr int kSweepRounds = 3; // dense sweep rounds before the worklist completion (2-6 measured: 3 is fastest)
 constexpr int kMaxEdge = 63;
-// From this many reconstructions on, one CTA each fills the SMs and the sweeps' throughput (34 ps per
-// pixel of a reconstruction) beats the basins' (90 ps); below it a sweep CTA's latency counts, 25 to 50 ns
-// per pixel of one image: 64 images of 1000 x 700 (holes) 17 to 27 against 5 ms, 16 of 1024 x 1024 (both)
-// 34 to 39 against 3.7 ms, 4 of 2000 x 2000 (holes) 76 to 108 against 2.2 ms, 250 of 500 x 300 (both) 8.1
-// to 8.5 against 6.8 to 7.4 ms, but 700 of 1500 x 64 (both) 8 against 14 ms.
-constexpr size_t kFloodUnits = 148 * 4;
+// Few reconstructions merge basins, many take sweeps. Basins cost 90 ps per pixel over the whole GPU.
+// Sweeps have one CTA per image: up to 148 of them take as long as one (rows times a step that grows
+// slowly with the row: 10 ns per pixel on rows of 1000, 17 on 500, 34 on 200), and 34 ps per pixel beyond
+// that. So the line falls with the row length. Images whose paths wind take up to three times as long in
+// the worklist, with 8 neighbours above all. Basins against sweeps in ms, smooth images to projections of
+// a phantom with counting noise and stuck pixels:
+//   holes, 8 neighbours:  110 of 700 x 1000  6.8-8.0 against 7.4-19    200  12-14 against 8.6-24
+//                         200 of 300 x 500   2.7-3.3 against 2.8-7.9   400  5.1-6.1 against 3.3-6.6
+//   peaks, 4 neighbours:  110 of 700 x 1000  6.6-7.7 against 6.9-12    200  12-14 against 8.2-15
+//                         148 of 300 x 500   2.0-2.4 against 2.5-3.9   295  3.6-4.4 against 2.8-4.0
+// Over 40 to 590 reconstructions of eight sizes (16 x 2048 to 500 x 300) the choice is within 2 % of the
+// faster one on average and 1.7 at worst; basins for all of them: 14 to 20 % and 2.6. Above 592 (four
+// CTAs per SM) sweeps are as fast or faster on all but rows below 100 pixels.
+inline bool few_units(size_t units, size_t pw, bool conn8)
+{
+    return units < std::min<size_t>(592, 40 + (conn8 ? 190000 : 100000) / pw);
+}
 constexpr size_t kBandSmem = 200 * 1024; // shared memory of k_peaks_band_smem
 
 // ---- preparation
@@ -483,7 +494,7 @@ __global__ void k_band_into(const float *__restrict__ band, int pw, int ph, floa
 // than a tile, then only over tiles that still hold a boundary.
 //
 // Measured against row sweeps finished by a worklist, which are bound by the latency of their relaxation
-// chains: see kFloodUnits.
+// chains: see few_units.
 
 constexpr int kOcean = -1, kNone = -2;
 constexpr int kStripThreads = 256;
@@ -903,7 +914,7 @@ static mr_status launch_flood(const Flood &F, cudaStream_t s)
     return check_launch("morphspotclean reconstruction");
 }
 
-// ---- reconstruction by row sweeps and a worklist (many images; see kFloodUnits)
+// ---- reconstruction by row sweeps and a worklist (many images; see few_units)
 
 // One or two reconstructions of the same images in one launch (FillHole of the image and of its
 // negation in the 'both' mode): CTA b < nimg works on image b with sign[0] into vol[0], CTA
@@ -1457,7 +1468,7 @@ mr_status mr_morphspotclean(float *proj_d, size_t nu, size_t nv, size_t nproj, i
     // images per batch: the padded image and, per reconstruction, a result or the labels with the basins'
     // component, level, hook and two edges, or two worklists; up to a quarter of the free device memory
     const int jobs = detect == 2 ? 2 : 1;
-    const bool flood = nproj * jobs < kFloodUnits && n < size_t(1) << 30;
+    const bool flood = few_units(nproj * jobs, pw, conn8) && n < size_t(1) << 30;
     const size_t cap = flood ? most_basins(pw, ph, conn8) : static_cast<size_t>(complete_cap(n));
     const size_t band = detect == 1 ? band_size(pw, ph) : 0;
     const size_t per_unit = n * 4 + (flood ? cap * (3 * 4 + 2 * 8) + strips_of(pw, ph) + (kMostRounds + 2) * 4 : 2 * cap * 4 + 4);

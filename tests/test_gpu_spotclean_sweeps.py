@@ -64,6 +64,19 @@ def test_worklist_completion(cuda, detect, conn8, h, w):
     _check(_noisy_profile(h, w, 2, h + w), detect, conn8, (0.1, 0.1))
 
 
+# stacks beyond the number up to which basins are merged at their width and neighbourhood (230, 139 and
+# 118 reconstructions; with 'both', two per image) equal their parts below it
+@pytest.mark.parametrize("detect,conn8,w,n,part", [("holes", True, 990, 240, 80), ("both", True, 990, 117, 39),
+                                                   ("peaks", False, 990, 150, 50), ("holes", False, 1270, 120, 40)])
+def test_line_between_the_reconstructions(cuda, detect, conn8, w, n, part):
+    img = _noisy_profile(12, w, n, w + n)
+    got = _clean(img, detect, conn8, (0.1, 0.1), 5)
+    parts = torch.cat([_clean(img[a:a + part], detect, conn8, (0.1, 0.1), 5) for a in range(0, n, part)])
+    assert torch.equal(got, parts)
+    exp = O.morphspotclean(img[:3], detect, conn8, (0.1, 0.1), (0.0, 0.0), edge=5)
+    assert np.array_equal(got[:3].cpu().numpy(), exp)
+
+
 @pytest.mark.parametrize("detect", ["holes", "peaks", "both"])
 def test_checked_build(cuda, detect, monkeypatch):
     img = np.tile(_noisy_profile(40, 300, 2, 9), (MANY // 2, 1, 1))
