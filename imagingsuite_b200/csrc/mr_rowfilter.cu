@@ -157,11 +157,12 @@ struct RowPair {
         m0 = fmaxf(m0, fabsf(y0));
         m1 = fmaxf(m1, fabsf(y1));
     }
-    // largest |output| of each row into its projection's
+    // largest |output| of each row into its projection's (all lanes; blocks are whole warps)
     __device__ __forceinline__ void put_max(const RowFilterArgs &a, float m0, float m1) const
     {
         if (!a.amax) return;
-        const int k0 = __reduce_max_sync(__activemask(), __float_as_int(m0)), k1 = __reduce_max_sync(__activemask(), __float_as_int(m1));
+        const int k0 = __reduce_max_sync(0xffffffffu, __float_as_int(m0));
+        const int k1 = __reduce_max_sync(0xffffffffu, __float_as_int(m1));
         if ((threadIdx.x & 31) != 0) return;
         atomicMax(reinterpret_cast<int *>(a.amax + r0 / a.nv), k0);
         if (has1) atomicMax(reinterpret_cast<int *>(a.amax + r1 / a.nv), k1);

@@ -59,3 +59,24 @@ def test_fdk_filter_and_its_scales(cuda, nu):
     for prec in ("bf16", "fp16"):
         bits, scale = M.quantize(res["fp32"][0], prec)
         assert torch.equal(scale, res[prec][1]) and torch.equal(bits.view(torch.int16), res[prec][0].view(torch.int16))
+
+
+@pytest.mark.parametrize("nu", [12, 33, 99, 130, 301])
+def test_scales_from_a_maximum_in_any_column(cuda, nu):
+    """Each projection's largest |value| in another column, so in another lane of the kernel's warps: the
+    scales equal those of the filtered projections quantised apart."""
+    nv = 13
+    g = torch.Generator(device=cuda).manual_seed(nu)
+    p = 0.01 * torch.randn((nu, nv, nu), device=cuda, generator=g)
+    c = torch.arange(nu, device=cuda)
+    p[c, 6, c] = 10.0 * 1.37 ** (c % 17).float()
+    geo = (torch.ones(nu, device=cuda), None, None, None, np.float32(0.25), np.float32(0.5), 1, (0, 0), None)
+    res = {}
+    for prec in ("fp32", "bf16", "fp16"):
+        f = M.FDKbp_single()
+        f.Configure(M.ReconConfig(), {"ProjectionBufferSize": "16", "SliceBlock": "32", "SubVolume": "1 1", "precision": prec})
+        f.SizeU, f.SizeV = nu, nv
+        res[prec] = f.ramp_filter(p, geo)
+    for prec in ("bf16", "fp16"):
+        bits, scale = M.quantize(res["fp32"][0], prec)
+        assert torch.equal(scale, res[prec][1]) and torch.equal(bits.view(torch.int16), res[prec][0].view(torch.int16))
