@@ -263,7 +263,7 @@ struct Smem {
     float *tg;            // [2][NB][TGEO] (fast kernel)
     int4 *meta;           // [2][NB]: offset of the stage (see issue), mode; .w of a group's first entry: Group
     uint64_t *bars;       // [2]
-    uint32_t *gdesc;      // [NB][GEO]: source of each geometry element (exact kernel)
+    uint32_t *gdesc;      // [NB][GEO]: source of each geometry element (exact kernel with a table)
     __device__ Smem(unsigned char *base, int boxbytes)
     {
         stage = base;
@@ -275,48 +275,47 @@ struct Smem {
         bars = reinterpret_cast<uint64_t *>(meta + 2 * NB);
         gdesc = reinterpret_cast<uint32_t *>(bars + 2);
     }
-    static size_t bytes(int boxbytes)
+    static size_t bytes(int boxbytes, bool table = A1)
     {
         return 2 * NB * static_cast<size_t>(boxbytes) +
                (3 * NB * GEO + (A1 ? NWARPS * NB * (TK + 2) : 2 * NB * TGEO)) * sizeof(float) +
-               2 * NB * sizeof(int4) + 2 * sizeof(uint64_t) + (A1 ? NB * GEO * sizeof(uint32_t) : 0);
+               2 * NB * sizeof(int4) + 2 * sizeof(uint64_t) + (table ? NB * GEO * sizeof(uint32_t) : 0);
     }
 };
 
-// Sources of the exact kernel's geometry of a batch, fixed for the tile: element (or, with geo16,
-// run of four elements) idx of projection b = idx / (elements per projection) is array[offset + p *
-// stride], p the projection; bits 0-25 the offset, 26-27 the array (0 zip, 1 xip, 2 yip, 3 none:
-// zero), 28-31 b.
-template <int NB>
-__device__ __forceinline__ void geometry_sources(const Params &P, uint32_t *gdesc, int i0, int j0, int k0)
+// Source of an element of the exact kernel's geometry of a batch, fixed for the tile: element (or, with
+// geo16, run of four elements) idx of projection b = idx / (elements per projection) is array[offset + p *
+// stride], p the projection; bits 0-25 the offset, 26-27 the array (0 zip, 1 xip, 2 yip, 3 none: zero),
+// 28-31 b. The tile keeps a table of them (TABLE), except for boxes so large that the table's 3.5 KB would
+// leave an SM one CTA; there the producer warp forms them for each batch: 256^3 from 180 projections takes
+// 995 us with a box of 56 x 53 and the table, 1085 with 56 x 54 and without it, and 3430 by direct loads.
+template <int RUN>
+__device__ __forceinline__ uint32_t geometry_source(const Params &P, int idx, int i0, int j0, int k0)
 {
-    const int run = P.geo16 ? 4 : 1, per = GEO_EXACT / run;
-    for (int idx = threadIdx.x; idx < NB * per; idx += THREADS) {
-        const int b = idx / per, e = idx % per * run;
-        uint32_t arr = 3, off = 0;
-        if (e < GX) {
-            if (k0 + e / 3 < P.nv) arr = 0, off = static_cast<uint32_t>(k0 * 3 + e);
-        } else if (e < GY) {
-            if (i0 + (e - GX) / 3 < P.nu) arr = 1, off = static_cast<uint32_t>(i0 * 3 + e - GX);
-        } else if (e < G0) {
-            if (j0 + (e - GY) / 3 < P.nu) arr = 2, off = static_cast<uint32_t>(j0 * 3 + e - GY);
-        } else if (e < G0 + 3) {
-            arr = 0, off = static_cast<uint32_t>(e - G0);
-        }
-        gdesc[idx] = off | arr << 26 | static_cast<uint32_t>(b) << 28;
+    constexpr int PER = GEO_EXACT / RUN;
+    const int b = idx / PER, e = idx % PER * RUN;
+    uint32_t arr = 3, off = 0;
+    if (e < GX) {
+        if (k0 + e / 3 < P.nv) arr = 0, off = static_cast<uint32_t>(k0 * 3 + e);
+    } else if (e < GY) {
+        if (i0 + (e - GX) / 3 < P.nu) arr = 1, off = static_cast<uint32_t>(i0 * 3 + e - GX);
+    } else if (e < G0) {
+        if (j0 + (e - GY) / 3 < P.nu) arr = 2, off = static_cast<uint32_t>(j0 * 3 + e - GY);
+    } else if (e < G0 + 3) {
+        arr = 0, off = static_cast<uint32_t>(e - G0);
     }
+    return off | arr << 26 | static_cast<uint32_t>(b) << 28;
 }
 
 // Starts the asynchronous copy of batch s's per-projection geometry into geometry buffer gb
 // (threads first, first + threads, ...; zero where a projection, column, row or slice does not exist).
-template <bool EXACT, int NB>
-__device__ __forceinline__ void stage_geometry(const Params &P, float *geo, int s, const uint32_t *gdesc, int first, int threads)
+template <bool EXACT, int NB, bool TABLE>
+__device__ __forceinline__ void stage_geometry(const Params &P, float *geo, int s, const uint32_t *gdesc, int i0, int j0, int k0,
+                                               int first, int threads)
 {
     if constexpr (EXACT) {
         const uint32_t zstride = static_cast<uint32_t>(P.nv) * 3, xstride = static_cast<uint32_t>(P.nu) * 3;
-        const int count = P.geo16 ? NB * GEO_EXACT / 4 : NB * GEO_EXACT;
-        for (int idx = first; idx < count; idx += threads) {
-            const uint32_t d = gdesc[idx];
+        auto copy = [&](int idx, uint32_t d) {
             const uint32_t arr = (d >> 26) & 3;
             const int p = s * NB + static_cast<int>(d >> 28);
             const bool ok = arr != 3 && p < P.nproj;
@@ -324,6 +323,14 @@ __device__ __forceinline__ void stage_geometry(const Params &P, float *geo, int 
             const float *src = base + (d & 0x3FFFFFFu) + static_cast<size_t>(p) * (arr == 0 ? zstride : xstride);
             if (P.geo16) tma::copy16_zfill(geo + 4 * idx, ok ? src : P.zip, ok);
             else copy4_zfill(geo + idx, ok ? src : P.zip, ok);
+        };
+        if constexpr (TABLE) {
+            const int count = P.geo16 ? NB * GEO_EXACT / 4 : NB * GEO_EXACT;
+            for (int idx = first; idx < count; idx += threads) copy(idx, gdesc[idx]);
+        } else if (P.geo16) {
+            for (int idx = first; idx < NB * GEO_EXACT / 4; idx += threads) copy(idx, geometry_source<4>(P, idx, i0, j0, k0));
+        } else {
+            for (int idx = first; idx < NB * GEO_EXACT; idx += threads) copy(idx, geometry_source<1>(P, idx, i0, j0, k0));
         }
     } else {
         const float *maps = reinterpret_cast<const float *>(P.maps); // 24 words per projection
@@ -448,7 +455,7 @@ __device__ __forceinline__ void issue(const Params &P, const CUtensorMap *tmap, 
     }
 }
 
-template <int DT, bool EXACT, int NB>
+template <int DT, bool EXACT, int NB, bool TABLE = EXACT>
 __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __grid_constant__ CUtensorMap tmap, const Params P)
 {
     constexpr int GEO = EXACT ? GEO_EXACT : GEO_FAST;
@@ -522,11 +529,16 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
 
     // geometry of batches 0-2, footprints and copies of batches 0-1
     if constexpr (EXACT) {
-        geometry_sources<NB>(P, S.gdesc, i0, j0, k0);
+        if constexpr (TABLE) {
+            if (P.geo16)
+                for (int idx = threadIdx.x; idx < NB * GEO_EXACT / 4; idx += THREADS) S.gdesc[idx] = geometry_source<4>(P, idx, i0, j0, k0);
+            else
+                for (int idx = threadIdx.x; idx < NB * GEO_EXACT; idx += THREADS) S.gdesc[idx] = geometry_source<1>(P, idx, i0, j0, k0);
+        }
         __syncthreads();
     }
     for (int s = 0; s < 3 && s < nbatch; ++s)
-        stage_geometry<EXACT, NB>(P, S.geo + s * NB * GEO, s, S.gdesc, threadIdx.x, THREADS);
+        stage_geometry<EXACT, NB, TABLE>(P, S.geo + s * NB * GEO, s, S.gdesc, i0, j0, k0, threadIdx.x, THREADS);
     copy_wait_all();
     __syncthreads();
     constexpr int ROUNDS = NB / 4;
@@ -559,7 +571,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) k_fdk_staged(const __gri
 #pragma unroll
                 for (int r = 0; r < ROUNDS; ++r) issue<DT, EXACT, NB>(P, &tmap, S, f[r], s + 2, st, r);
             }
-            if (s + 3 < nbatch) stage_geometry<EXACT, NB>(P, S.geo + gb * NB * GEO, s + 3, S.gdesc, lane, 32);
+            if (s + 3 < nbatch) stage_geometry<EXACT, NB, TABLE>(P, S.geo + gb * NB * GEO, s + 3, S.gdesc, i0, j0, k0, lane, 32);
         }
         if (stopped) {
             // copies still in flight: batch s (its wait expired) and batch s + 1 when it was issued;
@@ -904,7 +916,8 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
     if (bw <= 0 || bh <= 0 || bw > 256 || bh > 256 || bw % xalign) return MR_ERR_UNSUPPORTED;
     PFN_cuTensorMapEncodeTiled enc = tma::encode_fn();
     if (!enc) return fail(MR_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
-    constexpr size_t kMaxSmem = (227 * 1024) / CTAS_PER_SM - 1024; // CTAS_PER_SM CTAs per SM
+    // CTAS_PER_SM CTAs on an SM's 228 KB, each with 1 KB of the system's (and, the fast kernel, a few static words)
+    const size_t kMaxSmem = (228 * 1024) / CTAS_PER_SM - 1024 - (exact ? 0 : 512);
     CUtensorMap map;
     cuuint64_t dims[3] = {nu, nv, nproj};
     cuuint64_t strides[2] = {pitch * es, pitch * nv * es};
@@ -949,9 +962,11 @@ static mr_status staged_launch(bool exact, const void *proj_d, int dtype, const 
         if (dtype != MR_F32) return MR_ERR_UNSUPPORTED;
         P.geo16 = nu % 4 == 0 && nv % 4 == 0 && kbegin % 4 == 0 &&
                   ((reinterpret_cast<uintptr_t>(xip_d) | reinterpret_cast<uintptr_t>(yip_d) | reinterpret_cast<uintptr_t>(zip_d)) % 16) == 0;
-        const size_t s8 = Smem<8, GEO_EXACT, true>::bytes(P.boxbytes), s4 = Smem<4, GEO_EXACT, true>::bytes(P.boxbytes);
+        const size_t s8 = Smem<8, GEO_EXACT, true>::bytes(P.boxbytes);
+        const size_t s4 = Smem<4, GEO_EXACT, true>::bytes(P.boxbytes), bare = Smem<4, GEO_EXACT, true>::bytes(P.boxbytes, false);
         if (s8 <= kMaxSmem) return go(k_fdk_staged<MR_F32, true, 8>, s8);
         if (s4 <= kMaxSmem) return go(k_fdk_staged<MR_F32, true, 4>, s4);
+        if (bare <= kMaxSmem) return go(k_fdk_staged<MR_F32, true, 4, false>, bare);
         return MR_ERR_UNSUPPORTED;
     }
     const size_t s8 = Smem<8, GEO_FAST, false>::bytes(P.boxbytes), s4 = Smem<4, GEO_FAST, false>::bytes(P.boxbytes);
