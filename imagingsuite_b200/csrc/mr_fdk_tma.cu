@@ -363,6 +363,9 @@ __device__ __forceinline__ Foot footprint(const Params &P, const float *geo, int
     const int p = s * NB + b;
     Foot f;
     int rmin = 0, rmax = 0, cmin = 0, cmax = 0;
+    // side of the source plane (exact kernel; bits: in front, behind; 0: no position here). The corners
+    // bound a tile's samples only when all of it lies on one side: at the plane positions have no bound.
+    int side = 1;
     bool ok = p < P.nproj;
     if (ok) {
         const int ci = (corner & 1) ? i_hi : i0, cj = (corner & 2) ? j_hi : j0;
@@ -372,7 +375,8 @@ __device__ __forceinline__ Foot footprint(const Params &P, const float *geo, int
             const float *X = g + GX + 3 * (ci - i0), *Y = g + GY + 3 * (cj - j0);
             const float Z0 = g[G0], Z2 = g[G0 + 2];
             const float a1 = __fadd_rn(g[(corner & 4) ? 3 * (kmax - 1) + 1 : 1], Y[1]);
-            const float dw = __frcp_rn(__fadd_rn(__fadd_rn(Z2, Y[2]), X[2]));
+            const float depth = __fadd_rn(__fadd_rn(Z2, Y[2]), X[2]), dw = __frcp_rn(depth);
+            side = depth > 0.0f ? 1 : depth < 0.0f ? 2 : 0;
             r = __fadd_rn(__fmul_rn(dw, __fadd_rn(a1, X[1])), 0.5f);
             c = __fadd_rn(__fmul_rn(dw, __fadd_rn(__fadd_rn(Z0, Y[0]), X[0])), 0.5f);
             ok = ok && fabsf(r) < 4.0e6f && fabsf(c) < 4.0e6f;
@@ -394,14 +398,16 @@ __device__ __forceinline__ Foot footprint(const Params &P, const float *geo, int
             }
         }
     }
+    if (!ok) side = 0;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
         rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
         rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
         cmin = min(cmin, __shfl_xor_sync(0xffffffffu, cmin, o));
         cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
-        ok = __shfl_xor_sync(0xffffffffu, static_cast<int>(ok), o) && ok;
+        side &= __shfl_xor_sync(0xffffffffu, side, o);
     }
+    ok = side != 0;
     f.mode = p < P.nproj ? 0 : 2;
     f.x0 = f.y0 = 0;
     if (p < P.nproj && ok) {

@@ -1,4 +1,5 @@
-"""FDK staging: the largest boxes that two CTAs' shared memory holds."""
+"""FDK staging: the largest boxes that two CTAs' shared memory holds, and geometries whose source plane
+passes through a tile."""
 import ctypes
 
 import numpy as np
@@ -60,4 +61,31 @@ def test_box_is_staged(cuda, nu, nv, box):
         L.check(L.lib().mr_set_wait_limit(-1))
     got, direct = _backproject(cuda, m, filt, ang, box), _backproject(cuda, m, filt, ang, (0, 0))
     assert _word() == 0
+    assert torch.equal(got, direct)
+
+
+# the source inside the volume, detector pixels of a third to all of the source's distance: tiles with
+# corners on both sides of the source plane whose footprints would fit the box
+@pytest.mark.parametrize("sod,sdd,res", [(2.0, 4.0, 2.0), (1.0, 3.0, 1.0), (1.5, 2.0, 2.0), (0.8, 4.0, 1.5)])
+def test_source_plane_inside_a_tile(cuda, sod, sdd, res):
+    nu, nv, box = 64, 64, (56, 56)
+    ang = np.array([0.0, 30.0, 90.0, 135.0, 180.0, 200.0, 270.0, 301.0], np.float32)
+    m = _module(nu, nv, sod, sdd, res, 0.1)
+    xip, yip, zip_, *_, uni = m.partials(ang)
+    assert uni
+    fits = 0  # such tiles
+    for p in range(ang.size):
+        for j0 in range(0, nu, 8):
+            for i0 in range(0, nu, 32):
+                i, j = np.array([i0, i0 + 31])[:, None], np.array([j0, j0 + 7])[None]
+                X, Y = xip[p, i], yip[p, j]
+                d = zip_[p, 0, 2] + Y[..., 2] + X[..., 2]
+                if d.min() < 0 < d.max():
+                    c = (zip_[p, 0, 0] + Y[..., 0] + X[..., 0]) / d + 0.5
+                    r = np.stack([(zip_[p, k, 1] + Y[..., 1] + X[..., 1]) / d + 0.5 for k in (0, 31)])
+                    fits += np.ptp(c) < 50 and np.ptp(r) < 50 and c.max() > -1 and c.min() < nu and r.max() > -1 and r.min() < nv
+    assert fits > 0
+    rng = np.random.default_rng(3)
+    filt = torch.from_numpy(rng.standard_normal((ang.size, nv, nu)).astype(np.float32)).to(cuda)
+    got, direct = _backproject(cuda, m, filt, ang, box), _backproject(cuda, m, filt, ang, (0, 0))
     assert torch.equal(got, direct)
