@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kAdjTX * TY, CTAS) k_mbp_adjoint_staged(const 
         }
     };
     uint32_t phase0 = 0, phase1 = 0;
-    bool failed = false;
+    bool failed = false, stopped = false; // a wait of this warp expired; of any warp
     int s = 0;
     if (any) {
         for (int k = 0; k < 3 && k < nbatch; ++k) stage_geometry(k, k);
@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(kAdjTX * TY, CTAS) k_mbp_adjoint_staged(const 
         }
         // batch s + 2's geometry is published; stage st and geometry buffer gb are free
         tma::copy_wait_all();
-        if (__syncthreads_or(failed)) break;
+        stopped = __syncthreads_or(failed);
+        if (stopped) break;
         if (s + 2 < nbatch) issue(s + 2, st, gb == 0 ? 2 : gb - 1);
         if (s + 3 < nbatch) stage_geometry(s + 3, gb);
     }
@@ -254,9 +255,11 @@ __global__ void __launch_bounds__(kAdjTX * TY, CTAS) k_mbp_adjoint_staged(const 
         if (s + 1 < nbatch) tma::mbar_wait(&bars[st ^ 1], st ? phase0 : phase1);
     }
     if (valid && (inside || !P.accumulate)) {
+        // sums that a stopped tile has not finished pass for values in a gradient that nobody checks: NaN
+        const bool lost = stopped && inside;
 #pragma unroll
         for (int c = 0; c < kAdjTZ; ++c)
-            if (c < zmax) col[c] = (c & 1) ? acc[c >> 1].y : acc[c >> 1].x;
+            if (c < zmax) col[c] = lost ? __int_as_float(0x7FC00000) : (c & 1) ? acc[c >> 1].y : acc[c >> 1].x;
     }
 }
 

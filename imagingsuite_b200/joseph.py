@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from ._lib import check
+from ._lib import check, check_device
 
 
 def _stream() -> int:
@@ -109,7 +109,11 @@ class MatchedOperator:
     (nproj, nz, n): the detector is n bins wide, as the reference backprojector takes it; nz a
     multiple of 4 (the backprojector updates slices in groups of 4). Angles in degrees, rotation
     direction as ReconConfig's eDirection (0 = clockwise). Same interface as JosephOperator, so
-    project(), cgls(), fbp() and estimate_geometry() take either operator."""
+    project(), cgls(), fbp() and estimate_geometry() take either operator.
+
+    The adjoint's kernels wait for their copies a bounded number of times. If that ever runs out, the
+    tiled form (tilt) leaves NaN in the voxels concerned, and both set the device error word, which
+    cgls() and fbp() read; after adjoint() and backward() by themselves _lib.check_device() does."""
 
     def __init__(self, n: int, nz: int, angles_deg, pivot: float | None = None, direction: int = 0, device=None):
         if nz % 4:
@@ -231,7 +235,8 @@ def cgls(op: JosephOperator, p: torch.Tensor, x0: torch.Tensor, centre: float, t
     (the two extra columns scaled to the operator's norm); the geometry increments are then
     applied (the centre step clipped to max_centre_step bins, the reach of the linearisation
     of an interpolation that is linear within one pixel) and the next block is linearised
-    anew. Returns x, centre, tilt (degrees) and the history of 1/2 |residual|^2."""
+    anew. Returns x, centre, tilt (degrees) and the history of 1/2 |residual|^2; raises MrError when a
+    kernel reported an expired wait."""
     x = x0.clone()
     history = []
     zw = (torch.arange(op.nz, dtype=torch.float32, device=x.device) - op.pivot).view(1, op.nz, 1)
@@ -291,6 +296,7 @@ def cgls(op: JosephOperator, p: torch.Tensor, x0: torch.Tensor, centre: float, t
             du = max(-lim, min(lim, du))
             centre += dc
             tilt_deg = math.degrees(math.atan(math.tan(math.radians(tilt_deg)) + du))
+    check_device()
     return x, centre, tilt_deg, history
 
 
@@ -298,7 +304,8 @@ def fbp(op: JosephOperator, p: torch.Tensor, centre: float, tilt_deg: float = 0.
         cutoff: float = 0.5) -> torch.Tensor:
     """Filtered backprojection through the pair: detector rows ramp-filtered by the
     ProjectionFilterSingle kernels (mr_projfilter_*), backprojected with A^T, and scaled by
-    the least-squares factor s minimising |A (s b) - p| (the starting volume of CGLS)."""
+    the least-squares factor s minimising |A (s b) - p| (the starting volume of CGLS). Raises MrError
+    when a kernel reported an expired wait."""
     plan = ctypes.c_void_p()
     check(L.lib().mr_projfilter_create(op.nu, filtertype.encode(), float(cutoff), 1.0, 1, 0.1, 2, ctypes.byref(plan)))
     try:
@@ -309,6 +316,7 @@ def fbp(op: JosephOperator, p: torch.Tensor, centre: float, tilt_deg: float = 0.
     b = op.adjoint(f, centre, tilt_deg)
     ab = op.forward(b, centre, tilt_deg)
     s = _dot(ab, p) / max(_dot(ab, ab), 1e-300)
+    check_device()
     return b.mul_(s)
 
 

@@ -494,7 +494,8 @@ mr_status mr_device_status(int *status);
  *   (and the matched adjoint; default 4194304; a negative value restores it), read at each launch. A wait that runs
  *   out sets the device error word (mr_device_status returns 1), skips the rest of the block's
  *   projections, waits for the block's copies still in flight (with the default limit) and
- *   returns; the context stays usable. 0 makes every such wait expire at once.
+ *   returns; the context stays usable. The matched adjoint leaves NaN in the block's voxels. 0 makes
+ *   every such wait expire at once.
  * mr_debug_fail_allocation: the scratch allocation made after `after` further successful ones
  *   fails with MR_ERR_ALLOCATION, once (a negative value disarms the hook). Process-wide.
  * mr_trace_push / mr_trace_pop: an NVTX range on the calling thread (the host modules put one
