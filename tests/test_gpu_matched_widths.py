@@ -68,3 +68,22 @@ def test_adjoint_without_scratch(cuda, n, tilt):
     finally:
         L.check(L.lib().mr_debug_fail_allocation(-1))
     assert torch.equal(got, exp)
+
+
+@pytest.mark.parametrize("n,nz", [(64, 32), (61, 12), (192, 64)])
+def test_accumulate_keeps_what_is_outside_the_circle(cuda, n, nz):
+    """A volume of nonzero values: untouched outside the circle; inside, one call continues it as two do."""
+    g = torch.Generator(device=cuda).manual_seed(1)
+    p = torch.randn((40, nz, n), device=cuda, generator=g)
+    op = J.MatchedOperator(n, nz, (np.arange(40) * 4.5).astype(np.float32))
+    preset = torch.rand((n, n, nz), device=cuda, generator=g) + 1.0
+    one, two = preset.clone(), preset.clone()
+    op.adjoint(p, n / 2 + 0.3, 0.4, out=one, accumulate=True)
+    for a, b in ((0, 17), (17, 40)):
+        J.MatchedOperator(n, nz, op.angles[a:b]).adjoint(p[a:b].contiguous(), n / 2 + 0.3, 0.4, out=two, accumulate=True)
+    m = op._mask.cpu().numpy().view(np.uint32).reshape(-1, 2)
+    x = np.arange(1, n + 1)
+    inside = torch.from_numpy((x > m[:, :1]) & (x <= m[:, 1:])).to(cuda)
+    assert torch.equal(one[~inside], preset[~inside])
+    assert torch.equal(one, two)
+    assert bool((one[inside] != preset[inside]).any(dim=1).all())
