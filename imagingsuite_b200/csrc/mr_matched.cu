@@ -540,9 +540,9 @@ __global__ void __launch_bounds__(kStripWarps * 32, 10) k_mbp_forward_strip(cons
 // Bound by instruction issue. 256^2 x 64 slices, 180 projections, with the derivative: 1231 -> 965 us (two CTAs
 // where they shorten the last wave: 991 with one), 192^2 x 16 x 60 307 -> 125 (one: 216), 64^2 x 8 x 60 42 -> 22.
 // Clusters of four and eight find too few places for CTAs that fill an SM (192^2 x 64 x 360: 994 -> 3661 with
-// eight). Up to kFwdSmemBins, two CTAs' bins fit an SM and this beats the strips: 384^2 x 20 x 120 815 against
-// 887 us, 64^2 x 8 x 60 22 against 86; at 512^2 1455 against 1401, and 1387 against 888 with 8 slices and 60
-// projections.
+// eight). A CTA of 1024 threads at 64 registers has its SM alone. Narrow detectors beat the strips: 384^2 x 20 x
+// 120 815 against 887 us, 64^2 x 8 x 60 22 against 86; at 512^2 1455 against 1401, and 1387 against 888 with 8
+// slices and 60 projections. kFwdSmemBins lies between; where exactly they cross was not measured.
 constexpr int kFwdThreads = 1024;
 constexpr size_t kFwdSmemBins = 400;
 
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mbp_forward_smem(const float
     __syncthreads();
     if (zok) {
         const float suz = startu[static_cast<size_t>(i) * nz + z];
-        const int warp = rank * (kFwdThreads / 32) + static_cast<int>(threadIdx.x >> 5), nwarps = ctas * (kFwdThreads / 32);
+        const int per = static_cast<int>(blockDim.x >> 5), warp = rank * per + static_cast<int>(threadIdx.x >> 5), nwarps = ctas * per;
         // u falls along x by sin and grows along y by cos
         if (by_rows ? s.x <= 0.0f : s.y >= 0.0f)
             forward_walk<DERIV, true>(vol, s, suz, n, nz, z, by_rows, warp, nwarps, rowmask, colspan, bins + lane, dbins + lane);
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mbp_forward_smem(const float
     cluster.sync();
     // write-out: consecutive threads take consecutive bins of one slice (coalesced stores), summed over the CTAs
     const int zs = min(32, nz - z0);
-    for (int e = rank * kFwdThreads + threadIdx.x; e < zs * n; e += ctas * kFwdThreads) {
+    for (int e = rank * blockDim.x + threadIdx.x; e < zs * n; e += ctas * blockDim.x) {
         const int zz = e / n, m = e - zz * n;
         const size_t o = (static_cast<size_t>(i) * nz + z0 + zz) * n + m;
         float a = 0.0f, d = 0.0f;
@@ -782,9 +782,14 @@ mr_status mr_mbp_forward(const float *vol_d, size_t n, size_t nz, const float *s
         return fail(MR_ERR_ARGUMENT, "mr_mbp_forward: unsupported size");
     const float2 *sc = reinterpret_cast<const float2 *>(sincos_d);
     if (n <= kFwdSmemBins) {
-        // two CTAs per (projection, 32 slices) where that shortens the last wave
-        const size_t units = nproj * div_up(nz, 32);
-        const unsigned ctas = div_up(2 * units, 148) < 2 * div_up(units, 148) ? 2 : 1;
+        // Two CTAs per (projection, 32 slices) where that shortens the last wave. Zeroing, masks and the cluster's
+        // barriers are paid once per wave, so the shorter the lines the fewer waves may be: 192^2 x 32 slices,
+        // 180 projections (2 waves) 325 us with two against 351, but 96^2 113 against 101, and 128^2 with 310
+        // projections (3 waves) 271 against 220. Detectors so narrow that the lines leave warps idle take half
+        // as many threads from two waves on, two CTAs to an SM: 48^2 x 128 x 360 152 us against 181.
+        const size_t units = nproj * div_up(nz, 32), waves = div_up(units, 148);
+        const unsigned ctas = div_up(2 * units, 148) < 2 * waves && (waves == 1 || n >= 64 * waves) ? 2 : 1;
+        const unsigned threads = waves > 1 && n <= 48 ? kFwdThreads / 2 : kFwdThreads;
         const size_t smem = fwd_smem_bytes(static_cast<int>(n), dproj_d != nullptr);
         auto launch = [&](auto kernel) -> mr_status {
             MR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
@@ -793,7 +798,7 @@ mr_status mr_mbp_forward(const float *vol_d, size_t n, size_t nz, const float *s
             attr.val.clusterDim = {ctas, 1, 1};
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(static_cast<unsigned>(nproj) * ctas, div_up(nz, 32));
-            cfg.blockDim = dim3(kFwdThreads);
+            cfg.blockDim = dim3(threads);
             cfg.dynamicSmemBytes = smem;
             cfg.stream = as_stream(stream);
             cfg.attrs = &attr;

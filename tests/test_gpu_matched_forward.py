@@ -62,3 +62,19 @@ def test_forward_two_ctas(cuda):
         exp = O.mbp_forward64(x, ang, 32.9, 0.01, 1.5)
         got, _ = _forward(x, ang, 32.9, 0.01, 1.5, mask, False)
         assert np.sqrt(np.sum((got - exp) ** 2)) <= 1e-6 * np.sqrt(np.sum(exp ** 2))
+
+
+# more pairs than the GPU has SMs: half as many threads up to 48 bins, whole ones beyond, two CTAs each where the
+# lines are long enough for the number of waves (130 bins, 160 pairs) and one where not
+@pytest.mark.parametrize("n,nz,nproj", [(3, 33, 80), (16, 4, 150), (48, 34, 100), (49, 4, 160), (130, 4, 160), (130, 34, 160)])
+def test_forward_several_waves(cuda, n, nz, nproj):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, n, nz)).astype(np.float32)
+    mask = O.circle_mask(n, n).astype(np.uint32)
+    ang = (np.arange(nproj) * 2.3).astype(np.float32)
+    exp, dexp = O.mbp_forward64(x, ang, n / 2 + 0.2, 0.01, nz / 2, derivative=True)
+    for derivative in (False, True):
+        got, d = _forward(x, ang, n / 2 + 0.2, 0.01, nz / 2, mask, derivative)
+        assert np.sqrt(np.sum((got - exp) ** 2)) <= 1e-6 * np.sqrt(np.sum(exp ** 2))
+        if derivative:
+            assert np.abs(d - dexp).max() <= 1e-3 * np.abs(dexp).max()
