@@ -676,7 +676,11 @@ extern "C" mr_status mr_bp_parallel_variant(int variant, const void *proj_d, siz
     const bool other_column = variant == MR_BP_MULTIPROJ_SERIAL && (nv & 3) != 0;
     if (!other_column && dtype == MR_F32 && nproj > 0 && nproj <= 0x7fffffff && nu >= 2 && nu <= 65536 &&
         nv <= 65536 && y_begin < y_end) {
-        if (!index_d && nslabs < nproj) return fail(MR_ERR_ARGUMENT, "mr_bp_parallel_variant: nslabs below nproj");
+        if (!index_d && nslabs < nproj) {
+            // with tilt correction the count was never asked for: the list is the slabs then
+            if (!correcttilt) return fail(MR_ERR_ARGUMENT, "mr_bp_parallel_variant: nslabs below nproj");
+            nslabs = nproj;
+        }
         mr_status st = bp_parallel_staged_launch(variant, static_cast<const float *>(proj_d), nslabs, weight_d, index_d,
                                                  sin_d, cos_d, startu_d, nproj, nu, nv, mask_d, correcttilt, tiltoffset,
                                                  tiltinc, y_begin, y_end, vol_d, as_stream(stream));

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import oracle as O
+from imagingsuite_b200 import _lib as L
 from imagingsuite_b200 import modules as M
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +96,23 @@ def test_values_that_are_not_finite(cuda, nu):
         bp.Process(proj, {"angles": _text(ang), "weights": _text(np.ones(nproj))}, prefiltered_weights=True)
         vols.append(bp.GetVolume().cpu().numpy())
     assert np.isnan(vols[1]).any() and np.array_equal(vols[0], vols[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("nu", [64, 66])
+def test_slab_count_below_the_list(cuda, nu):
+    """Without an index list fewer slabs than projections are refused, with tilt correction they never were."""
+    nv, nproj = 8, 20
+    g = torch.Generator(device=cuda).manual_seed(nu)
+    p = torch.randn((nproj, nv, nu), device=cuda, generator=g)
+    sn, cs, su = (torch.rand(nproj, device=cuda, generator=g) * s + o for s, o in ((0.7, 0.0), (0.3, 0.7), (2.0, 0.0)))
+    mask = torch.tensor([0, nu], dtype=torch.int32, device=cuda).repeat(nu)
+    vols = {}
+    for tilt, nslabs in ((1, nproj), (1, nproj - 1), (1, 0), (0, nproj - 1)):
+        vol = torch.zeros((nu, nu, nv), device=cuda)
+        st = L.lib().mr_bp_parallel_staged(p.data_ptr(), nslabs, L.MR_F32, None, None, None, sn.data_ptr(), cs.data_ptr(),
+                                           su.data_ptr(), nproj, nu, nv, mask.data_ptr(), tilt, 0.3, 0.01, vol.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream)
+        assert st == (L.MR_OK if tilt else L.MR_ERR_ARGUMENT)
+        vols[tilt, nslabs] = vol
+    assert torch.equal(vols[1, nproj], vols[1, nproj - 1]) and torch.equal(vols[1, nproj], vols[1, 0])
+    assert not bool(vols[0, nproj - 1].any())
