@@ -1466,15 +1466,22 @@ mr_status mr_morphspotclean(float *proj_d, size_t nu, size_t nv, size_t nproj, i
     const size_t n = static_cast<size_t>(pw) * ph;
     cudaStream_t s = as_stream(stream);
     // images per batch: the padded image and, per reconstruction, a result or the labels with the basins'
-    // component, level, hook and two edges, or two worklists; up to a quarter of the free device memory
+    // component, level, hook and two edges, or two worklists; up to a quarter of the free device memory.
+    // An image whose basins (26 to 40 bytes a pixel with both modes) do not fit that takes the sweeps (13).
     const int jobs = detect == 2 ? 2 : 1;
-    const bool flood = few_units(nproj * jobs, pw, conn8) && n < size_t(1) << 30;
-    const size_t cap = flood ? most_basins(pw, ph, conn8) : static_cast<size_t>(complete_cap(n));
     const size_t band = detect == 1 ? band_size(pw, ph) : 0;
-    const size_t per_unit = n * 4 + (flood ? cap * (3 * 4 + 2 * 8) + strips_of(pw, ph) + (kMostRounds + 2) * 4 : 2 * cap * 4 + 4);
-    const size_t per_img = (n + band + 3) * 4 + jobs * per_unit + 64;
     const size_t most = std::min<size_t>(nproj, size_t(65535) / jobs);
-    const size_t batch = std::max<size_t>(1, std::min<size_t>(most, scratch_budget(most * per_img) / per_img));
+    bool flood = few_units(nproj * jobs, pw, conn8) && n < size_t(1) << 30;
+    size_t cap, per_img, budget;
+    for (;;) {
+        cap = flood ? most_basins(pw, ph, conn8) : static_cast<size_t>(complete_cap(n));
+        const size_t per_unit = n * 4 + (flood ? cap * (3 * 4 + 2 * 8) + strips_of(pw, ph) + (kMostRounds + 2) * 4 : 2 * cap * 4 + 4);
+        per_img = (n + band + 3) * 4 + jobs * per_unit + 64;
+        budget = scratch_budget(most * per_img);
+        if (!flood || per_img <= budget) break;
+        flood = false;
+    }
+    const size_t batch = std::max<size_t>(1, std::min<size_t>(most, budget / per_img));
     char *scratch = nullptr;
     MR_TRY(device_alloc(&scratch, batch * per_img, s, "mr_morphspotclean: scratch"));
     const size_t units = batch * jobs;
