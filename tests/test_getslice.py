@@ -113,3 +113,15 @@ def test_matrix_roi_mask_and_slices_match_reference(cuda, ref_lib, cone):
         assert np.array_equal(gv == 0, ev == 0)  # the same masked voxels
     else:
         assert np.array_equal(gv, ev) and np.array_equal(gs, es)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("zxy", [True, False])
+@pytest.mark.parametrize("roi", CASES)
+def test_getslice_device_equals_host(cuda, zxy, roi):
+    """Device volumes give the slices of host volumes, which are pinned against the reference above."""
+    vol = _volume(zxy, 1)
+    for idx in (0, 3, 4):
+        got = _module(zxy, torch.from_numpy(vol).to(cuda), roi).GetSlice(idx)
+        assert got.is_cuda
+        assert np.array_equal(got.cpu().numpy(), _module(zxy, torch.from_numpy(vol), roi).GetSlice(idx).numpy())
