@@ -36,8 +36,8 @@ sys.path.insert(0, ROOT)
 
 METRIC = "backprojection GUPS + projections/s, FP32 vs BF16-proj at <=1e-3 rel RMS vs FP64"
 # DRAM bytes (read + write) of one k_fdk_staged<f32, exact> launch, measured with ncu on this
-# workload (detector width -> bytes): 1024^3 547.23 GB + 6.27 GB, 256^3 69.9 MB + 41.8 MB
-MEASURED_TRAFFIC = {1024: 553.50e9, 256: 111.7e6}
+# workload (detector width -> bytes): 1024^3 594.47 GB + 8.50 GB, 256^3 70.7 MB + 45.5 MB
+MEASURED_TRAFFIC = {1024: 602.97e9, 256: 116.2e6}
 
 
 def workload(small: bool, c2: bool = False):
