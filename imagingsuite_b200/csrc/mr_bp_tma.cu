@@ -123,7 +123,8 @@ __device__ __forceinline__ bool rows_share(float cs, float su, float fy, float t
 {
     const float cy = cs * fy;
     float values = fabsf(cy) + fabsf(su + cy) + fabsf(u);
-    if constexpr (MODE == kTilt || MODE == kTiltSerial || MODE == kTiltNearest) values += fabsf(su + cy) + fabsf(u) + 2.0f * fabsf(toff);
+    if constexpr (MODE == kTilt || MODE == kTiltSerial || MODE == kTiltNearest)
+        values += fabsf(su + cy) + fabsf(u) + 2.0f * fabsf(toff);
     return fabsf(cs) + 1.25f * 0x1p-23f * values < 1.0f;
 }
 
@@ -677,7 +678,7 @@ extern "C" mr_status mr_bp_parallel_variant(int variant, const void *proj_d, siz
     if (!other_column && dtype == MR_F32 && nproj > 0 && nproj <= 0x7fffffff && nu >= 2 && nu <= 65536 &&
         nv <= 65536 && y_begin < y_end) {
         if (!index_d && nslabs < nproj) {
-            // with tilt correction the count was never asked for: the list is the slabs then
+            // with tilt correction a caller need not count the slabs: they are the list's
             if (!correcttilt) return fail(MR_ERR_ARGUMENT, "mr_bp_parallel_variant: nslabs below nproj");
             nslabs = nproj;
         }

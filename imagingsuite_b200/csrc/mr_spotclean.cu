@@ -72,8 +72,9 @@ constexpr int kMaxEdge = 63;
 //   peaks, 4 neighbours:  110 of 700 x 1000  6.6-7.7 against 6.9-12    200  12-14 against 8.2-15
 //                         148 of 300 x 500   2.0-2.4 against 2.5-3.9   295  3.6-4.4 against 2.8-4.0
 // Over 40 to 590 reconstructions of eight sizes (16 x 2048 to 500 x 300) the choice is within 2 % of the
-// faster one on average and 1.7 at worst; basins for all of them: 14 to 20 % and 2.6. Above 592 (four
-// CTAs per SM) sweeps are as fast or faster on all but rows below 100 pixels.
+// faster one on average and 1.7 at worst; basins for all of them: 14 to 20 % and 2.6. With 590 the sweeps
+// are faster but on rows below 100 pixels and on winding paths in rows of 300; 592, four CTAs per SM, is
+// the most that was measured.
 inline bool few_units(size_t units, size_t pw, bool conn8)
 {
     return units < std::min<size_t>(592, 40 + (conn8 ? 190000 : 100000) / pw);
@@ -1558,8 +1559,9 @@ mr_status mr_morphspotclean(float *proj_d, size_t nu, size_t nv, size_t nproj, i
         if (st != MR_OK) break;
         const int *hole_lab = detect != 1 ? F.lab0 : nullptr, *peaks = detect != 0 ? peak_lab : nullptr;
         if (flood) // (a block per row of few images: with 128 blocks one of 2000 x 2000 took 77 us, 20 now)
-            k_replace<true><<<dim3(std::min<unsigned>(h, std::max(gx, 148u * 8 / nb)), nb), 256, 0, s>>>(P, hole_lab, F.lev, peaks, F.lev + (jobs - 1) * nb * cap, cap, mn,
-                                                         mx, w, h, detect, th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
+            k_replace<true><<<dim3(std::min<unsigned>(h, std::max(gx, 148u * 8 / nb)), nb), 256, 0, s>>>(
+                P, hole_lab, F.lev, peaks, F.lev + (jobs - 1) * nb * cap, cap, mn, mx, w, h, detect, th_h[0], th_h[1],
+                sigma_h[0], sigma_h[1], img);
         else
             k_replace<false><<<dim3(gx, nb), 256, 0, s>>>(P, hole_lab, nullptr, peaks, nullptr, 0, mn, mx, w, h, detect,
                                                           th_h[0], th_h[1], sigma_h[0], sigma_h[1], img);
